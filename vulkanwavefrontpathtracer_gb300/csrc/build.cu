@@ -1,7 +1,7 @@
 // Device build of the acceleration structures, for scenes that are large or
 // already on the GPU.  Takes the place of the host builder (bvh.cpp; the
 // reference's driver BLAS build, WaveFrontPathTracer.cpp:202-457):
-//   1. triangle boxes, the centroid box and the largest absolute coordinate
+//   1. the scene box, the centroid box and the largest absolute coordinate
 //      (for the conservative box growth) in one pass;
 //   2. 63-bit Morton keys of the triangle centroids, sorted with the
 //      library's radix sort;
@@ -10,15 +10,17 @@
 //      cluster picks the neighbour among the 8 (knob) on either side (in
 //      Morton order) whose merged box has the least surface area, mutual pairs
 //      merge, the cluster list is compacted by a prefix sum, until one
-//      cluster is left;
-//   4. the BVH2 in the traversal format (children's boxes grown by 2^-22 P
-//      as in the host builder; single-triangle leaves);
-//   5. the BVH8 by the host's SAH collapse: a bottom-up dynamic programme
-//      (one thread per leaf climbs towards the root; the second thread to
-//      arrive at a node computes it), then a top-down emission one level at
-//      a time with prefix-summed allocation, so the layout is deterministic.
-// Every loop over clusters or levels is bounded on the host; kernels check
-// their indices against the buffers they write.
+//      cluster is left.  All passes run in one cooperative launch, and the
+//      thread that merges a pair also writes the BVH2 node in the traversal
+//      format (children's boxes grown by 2^-22 P as in the host builder;
+//      single-triangle leaves) and the node's tables of the SAH collapse,
+//      whose dynamic programme is bottom-up like the clustering;
+//   4. the BVH8 by the host's SAH collapse, emitted top-down one level at a
+//      time in a second cooperative launch, eight lanes per node, with
+//      look-back allocation, so the layout is deterministic.
+// The host reads the device back once, at the end.  Every device wait is
+// bounded (kSpinLimit polls, then the timeout status); kernels check their
+// indices against the buffers they write.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -45,7 +47,6 @@ namespace {
 
 constexpr int kBB = 256;      // threads per build block
 constexpr int kPlocRMax = 64;  // largest PLOC search radius (knob build.ploc.radius)
-constexpr int kScanItems = 8;  // elements per thread of the prefix sum
 constexpr uint32_t kNone = 0xFFFFFFFFu;
 
 struct BuildStats {
@@ -53,6 +54,13 @@ struct BuildStats {
     uint32_t cmin[3], cmax[3];  // ... of the centroid box
     uint32_t pmax;              // bits of the largest |coordinate|
     uint32_t bad_index;
+    // Clustering: clusters and nodes after the last finished pass, passes,
+    // no pair merged (cannot happen), blocks that reached the pass barriers.
+    uint32_t clusters, next_id, iterations, stuck, ploc_barrier;
+    // Emission: BVH8 nodes and triangles emitted; by level parity, the tasks
+    // of the next level and the triangles so far; blocks that reached the
+    // level barriers.
+    uint32_t nodes8, tris8, tasks[2], tris[2], emit_barrier;
 };
 
 __device__ __forceinline__ uint32_t ord(float f) {
@@ -69,35 +77,38 @@ __device__ __forceinline__ float box_area(float4 lo, float4 hi) {
 }
 
 // ---------------------------------------------------------------- stage 1
+// Box of triangle g; false when one of its indices is out of range (read as
+// vertex 0, so the build can go on to the one read-back at its end).
+__device__ __forceinline__ bool tri_box(const float* __restrict__ pos, uint32_t nv, const uint32_t* __restrict__ idx,
+                                        uint32_t g, float lo[3], float hi[3]) {
+    bool ok = true;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        uint32_t v = idx[3 * (size_t)g + j];
+        if (v >= nv) {
+            ok = false;
+            v = 0;
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const float p = pos[3 * (size_t)v + k];
+            lo[k] = j == 0 ? p : fminf(lo[k], p);
+            hi[k] = j == 0 ? p : fmaxf(hi[k], p);
+        }
+    }
+    return ok;
+}
+
 __global__ void __launch_bounds__(kBB) k_tri_bounds(const float* __restrict__ pos, uint32_t nv,
                                                     const uint32_t* __restrict__ idx, uint32_t nt,
-                                                    float4* __restrict__ tlo, float4* __restrict__ thi,
                                                     BuildStats* __restrict__ st) {
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t bl[3] = {kNone, kNone, kNone}, bh[3] = {0, 0, 0};
     uint32_t cl[3] = {kNone, kNone, kNone}, ch[3] = {0, 0, 0};
     uint32_t pm = 0;
     if (g < nt) {
-        uint32_t v[3];
-        bool bad = false;
-        for (int j = 0; j < 3; ++j) {
-            v[j] = idx[3 * (size_t)g + j];
-            if (v[j] >= nv) {
-                bad = true;
-                v[j] = 0;
-            }
-        }
-        if (bad) atomicOr(&st->bad_index, 1u);
         float lo[3], hi[3];
-        for (int k = 0; k < 3; ++k) lo[k] = hi[k] = pos[3 * (size_t)v[0] + k];
-        for (int j = 1; j < 3; ++j)
-            for (int k = 0; k < 3; ++k) {
-                float p = pos[3 * (size_t)v[j] + k];
-                lo[k] = fminf(lo[k], p);
-                hi[k] = fmaxf(hi[k], p);
-            }
-        tlo[g] = make_float4(lo[0], lo[1], lo[2], 0.0f);
-        thi[g] = make_float4(hi[0], hi[1], hi[2], 0.0f);
+        if (!tri_box(pos, nv, idx, g, lo, hi)) atomicOr(&st->bad_index, 1u);
         float pmf = 0.0f;
         for (int k = 0; k < 3; ++k) {
             bl[k] = ord(lo[k]);
@@ -152,19 +163,20 @@ __device__ __forceinline__ uint64_t spread21(uint32_t x) {
     return v;
 }
 
-__global__ void __launch_bounds__(kBB) k_centroid_keys(const float4* __restrict__ tlo, const float4* __restrict__ thi,
-                                                       uint32_t nt, const BuildStats* __restrict__ st,
-                                                       uint64_t* __restrict__ keys, uint32_t* __restrict__ vals) {
+__global__ void __launch_bounds__(kBB) k_centroid_keys(const float* __restrict__ pos, uint32_t nv,
+                                                       const uint32_t* __restrict__ idx, uint32_t nt,
+                                                       const BuildStats* __restrict__ st, uint64_t* __restrict__ keys,
+                                                       uint32_t* __restrict__ vals) {
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= nt) return;
-    const float4 lo = tlo[g], hi = thi[g];
-    const float c[3] = {__fmul_rn(0.5f, __fadd_rn(lo.x, hi.x)), __fmul_rn(0.5f, __fadd_rn(lo.y, hi.y)),
-                        __fmul_rn(0.5f, __fadd_rn(lo.z, hi.z))};
+    float lo[3], hi[3];
+    tri_box(pos, nv, idx, g, lo, hi);
     uint32_t q[3];
     for (int k = 0; k < 3; ++k) {
+        const float c = __fmul_rn(0.5f, __fadd_rn(lo[k], hi[k]));
         const float a = unord(st->cmin[k]), b = unord(st->cmax[k]);
         const float ext = __fsub_rn(b, a);
-        float t = ext > 0.0f ? __fdiv_rn(__fsub_rn(c[k], a), ext) : 0.0f;
+        float t = ext > 0.0f ? __fdiv_rn(__fsub_rn(c, a), ext) : 0.0f;
         t = fminf(fmaxf(t, 0.0f), 1.0f);
         q[k] = min((uint32_t)__fmul_rn(t, 2097151.0f), 2097151u);
     }
@@ -173,14 +185,13 @@ __global__ void __launch_bounds__(kBB) k_centroid_keys(const float4* __restrict_
 }
 
 // Leaves in Morton order: node i is the triangle vals[i]; its record goes to
-// slot i of the BVH2 triangle table.
+// slot i of the BVH2 triangle table, its box to boxes[2 i], boxes[2 i + 1].
 __global__ void __launch_bounds__(kBB) k_leaves(const uint32_t* __restrict__ vals, uint32_t nt,
-                                                const float4* __restrict__ tlo, const float4* __restrict__ thi,
                                                 const float* __restrict__ pos, uint32_t nv,
                                                 const uint32_t* __restrict__ idx,
                                                 const uint32_t* __restrict__ geom_first, uint32_t ngeom,
-                                                float4* __restrict__ nlo, float4* __restrict__ nhi,
-                                                float4* __restrict__ recs, uint32_t* __restrict__ clusters) {
+                                                float4* __restrict__ boxes, float4* __restrict__ recs,
+                                                uint32_t* __restrict__ clusters) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nt) return;
     const uint32_t g = vals[i];
@@ -188,8 +199,6 @@ __global__ void __launch_bounds__(kBB) k_leaves(const uint32_t* __restrict__ val
         raise_status(kErrBounds);
         return;
     }
-    nlo[i] = tlo[g];
-    nhi[i] = thi[g];
     // Geometry: the last entry of geom_first that is <= g (upper_bound - 1).
     uint32_t a = 0, b = ngeom;
     while (a < b) {
@@ -205,6 +214,10 @@ __global__ void __launch_bounds__(kBB) k_leaves(const uint32_t* __restrict__ val
         if (v >= nv) v = 0;
         r[j] = make_float4(pos[3 * (size_t)v], pos[3 * (size_t)v + 1], pos[3 * (size_t)v + 2], 0.0f);
     }
+    boxes[2 * (size_t)i] = make_float4(fminf(fminf(r[0].x, r[1].x), r[2].x), fminf(fminf(r[0].y, r[1].y), r[2].y),
+                                       fminf(fminf(r[0].z, r[1].z), r[2].z), 0.0f);
+    boxes[2 * (size_t)i + 1] = make_float4(fmaxf(fmaxf(r[0].x, r[1].x), r[2].x), fmaxf(fmaxf(r[0].y, r[1].y), r[2].y),
+                                           fmaxf(fmaxf(r[0].z, r[1].z), r[2].z), 0.0f);
     r[0].w = __int_as_float((int32_t)prim);
     r[1].w = __int_as_float((int32_t)geom);
     r[2].w = __uint_as_float(g);
@@ -214,368 +227,316 @@ __global__ void __launch_bounds__(kBB) k_leaves(const uint32_t* __restrict__ val
     clusters[i] = i;
 }
 
-// ----------------------------------------------------------- prefix sums
-// Exclusive prefix sum of n u64 values in three launches: per-block sums,
-// one block scanning those, per-block scan plus offset.
-constexpr uint32_t kScanTile = kBB * kScanItems;
+// ----------------------------------------------- waits between the blocks
+// of a cooperative launch (all of them resident at once).
 
-__device__ __forceinline__ uint64_t block_exclusive_u64(uint64_t v, uint64_t* s_warp, uint64_t* total) {
+// Exclusive prefix over the tiles before `tile` of two counts packed as
+// hi << 28 | lo (totals below 2^27 and 2^28) by decoupled look-back, 32
+// predecessors per round trip; called by one full warp, result in all lanes.
+// A state holds epoch (7 bits, the pass or level: states are not cleared in
+// between) | flag (1 aggregate, 2 inclusive prefix) | hi | lo.
+constexpr int kStFlag = 55, kStEpoch = 57;
+constexpr uint64_t kStValue = (1ull << kStFlag) - 1;
+__device__ __forceinline__ uint64_t pack_state(uint32_t epoch, uint64_t flag, uint64_t v) {
+    return ((uint64_t)(epoch & 127u) << kStEpoch) | (flag << kStFlag) | v;
+}
+__device__ uint64_t tile_prefix64(unsigned long long* state, uint32_t tile, uint64_t v, uint32_t epoch) {
+    const uint32_t lane = threadIdx.x & 31;
+    if (lane == 0) atomicExch(&state[tile], (unsigned long long)pack_state(epoch, tile == 0 ? 2 : 1, v));
+    if (tile == 0) return 0;
+    uint64_t excl = 0;
+    uint32_t spins = 0;
+    int32_t top = (int32_t)tile - 1;
+    for (;;) {
+        const int32_t t = top - (int32_t)lane;
+        uint64_t s = pack_state(epoch, 2, 0);  // before tile 0: a prefix of 0
+        if (t >= 0) s = *((volatile unsigned long long*)&state[t]);
+        const uint32_t flag =
+            (uint32_t)(s >> kStEpoch) == (epoch & 127u) ? (uint32_t)(s >> kStFlag) & 3u : 0u;
+        const uint32_t pref = __ballot_sync(0xffffffffu, flag == 2u);
+        const uint32_t unset = __ballot_sync(0xffffffffu, flag == 0u);
+        const uint32_t p = pref ? (uint32_t)__ffs(pref) - 1u : 32u;
+        const uint32_t upto = p < 31u ? ((2u << p) - 1u) : 0xffffffffu;  // lanes 0..p
+        if (unset & upto) {
+            if (++spins > kSpinLimit) {
+                raise_status(kErrTimeout);
+                break;
+            }
+            continue;
+        }
+        const uint64_t w = lane <= p ? (s & kStValue) : 0u;
+        excl += ((uint64_t)__reduce_add_sync(0xffffffffu, (uint32_t)(w >> 28)) << 28) +
+                __reduce_add_sync(0xffffffffu, (uint32_t)w & 0xFFFFFFFu);
+        if (p < 32u) break;
+        top -= 32;
+    }
+    if (lane == 0) atomicExch(&state[tile], (unsigned long long)pack_state(epoch, 2, (excl + v) & kStValue));
+    return excl;
+}
+
+// All `blocks` blocks arrive (the counter reaches `target`, the sum of the
+// arrivals of all barriers so far); what they wrote before is visible after.
+// False after a timeout.
+__device__ bool block_barrier(uint32_t* counter, uint32_t target) {
+    __shared__ uint32_t s_ok;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        atomicAdd(counter, 1u);
+        uint32_t ok = 1, spins = 0;
+        while ((int32_t)(*((volatile uint32_t*)counter) - target) < 0) {
+            if (++spins > kSpinLimit) {
+                raise_status(kErrTimeout);
+                ok = 0;
+                break;
+            }
+        }
+        __threadfence();
+        s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
+// Exclusive scan of one word per thread over the block (two 16-bit counts
+// that do not overflow into each other); *total receives the block's sum.
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* s_warp, uint32_t* total) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint64_t x = v;
+    uint32_t x = v;
+#pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        uint64_t y = __shfl_up_sync(0xffffffffu, x, o);
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
         if (lane >= (uint32_t)o) x += y;
     }
     if (lane == 31) s_warp[warp] = x;
     __syncthreads();
-    uint64_t off = 0, sum = 0;
+    uint32_t off = 0, sum = 0;
+#pragma unroll
     for (int w = 0; w < kBB / 32; ++w) {
-        uint64_t c = s_warp[w];
+        const uint32_t c = s_warp[w];
         if (w < (int)warp) off += c;
         sum += c;
     }
-    __syncthreads();
     *total = sum;
     return off + x - v;
 }
 
-__global__ void __launch_bounds__(kBB) k_scan_reduce(const uint64_t* __restrict__ in, uint32_t n,
-                                                     uint64_t* __restrict__ block_sums) {
-    __shared__ uint64_t s_warp[kBB / 32];
-    const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    uint64_t s = 0;
-    for (int j = 0; j < kScanItems; ++j)
-        if (base + j < n) s += in[base + j];
-    uint64_t total;
-    block_exclusive_u64(s, s_warp, &total);
-    if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
-}
-
-__global__ void __launch_bounds__(kBB) k_scan_sums(uint64_t* __restrict__ block_sums, uint32_t nb,
-                                                   uint64_t* __restrict__ grand_total) {
-    __shared__ uint64_t s_warp[kBB / 32];
-    uint64_t carry = 0;
-    for (uint32_t c0 = 0; c0 < nb; c0 += kBB) {
-        const uint32_t i = c0 + threadIdx.x;
-        const uint64_t v = i < nb ? block_sums[i] : 0;
-        uint64_t total;
-        const uint64_t ex = block_exclusive_u64(v, s_warp, &total);
-        if (i < nb) block_sums[i] = carry + ex;
-        carry += total;
-    }
-    if (threadIdx.x == 0) *grand_total = carry;
-}
-
-__global__ void __launch_bounds__(kBB) k_scan_apply(const uint64_t* __restrict__ in, uint32_t n,
-                                                    const uint64_t* __restrict__ block_sums,
-                                                    uint64_t* __restrict__ out) {
-    __shared__ uint64_t s_warp[kBB / 32];
-    const uint32_t base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-    uint64_t v[kScanItems], s = 0;
-    for (int j = 0; j < kScanItems; ++j) {
-        v[j] = base + j < n ? in[base + j] : 0;
-        s += v[j];
-    }
-    uint64_t total;
-    uint64_t run = block_exclusive_u64(s, s_warp, &total) + block_sums[blockIdx.x];
-    for (int j = 0; j < kScanItems; ++j) {
-        if (base + j < n) out[base + j] = run;
-        run += v[j];
-    }
-}
-
-struct Scan {
-    uint64_t* block_sums = nullptr;  // >= ceil(n / kScanTile) entries
-    uint64_t* total = nullptr;       // one entry
+// ---------------------------------------------------------------- stage 3
+// Collapse tables of a BVH2 node (the host's plan_sah): cost[2 i], [2 i + 1]
+// are the least costs of node i's subtree with at most 1..8 BVH8 children;
+// meta[i] = {how[0..3], how[4..7], triangles, split8}: byte how[0] is -1 for
+// one leaf child, 0 for one inner child; how[s-1] (s > 1) 0 for the same as
+// s-1, a > 0 for a slots to child 0; split8 is child 0's slots when the node
+// is a BVH8 inner node.
+struct Grown {
+    float4 lo, hi;
 };
 
-cudaError_t exclusive_scan(const uint64_t* in, uint64_t* out, uint32_t n, const Scan& sc, cudaStream_t s) {
-    const uint32_t nb = (n + kScanTile - 1) / kScanTile;
-    if (nb == 0) return cudaMemsetAsync(sc.total, 0, sizeof(uint64_t), s);
-    k_scan_reduce<<<nb, kBB, 0, s>>>(in, n, sc.block_sums);
-    k_scan_sums<<<1, kBB, 0, s>>>(sc.block_sums, nb, sc.total);
-    k_scan_apply<<<nb, kBB, 0, s>>>(in, n, sc.block_sums, out);
-    count_launch();
-    count_launch();
-    count_launch();
-    return cudaGetLastError();
-}
-
-// ---------------------------------------------------------------- stage 3
-// Nearest neighbour of every cluster within `radius` positions: the least
-// merged surface area, ties to the smaller position.  For a fixed cluster
-// that order is the order of (area, smaller position, larger position) over
-// pairs, so the pair that is least in that order over all pairs is mutual
-// and every iteration merges at least one pair.
-__global__ void __launch_bounds__(kBB) k_ploc_nn(const uint32_t* __restrict__ cl, uint32_t m,
-                                                 const float4* __restrict__ nlo, const float4* __restrict__ nhi,
-                                                 uint32_t* __restrict__ nn, int radius) {
-    __shared__ float4 s_lo[kBB + 2 * kPlocRMax], s_hi[kBB + 2 * kPlocRMax];
-    const int R = radius < 1 ? 1 : (radius > kPlocRMax ? kPlocRMax : radius);
-    const int b0 = (int)(blockIdx.x * kBB);
-    for (int t = threadIdx.x; t < kBB + 2 * R; t += kBB) {
-        const int j = b0 - R + t;
-        if (j >= 0 && j < (int)m) {
-            const uint32_t id = cl[j];
-            s_lo[t] = nlo[id];
-            s_hi[t] = nhi[id];
+// BVH2 node `index` over clusters a and b (ids: below n a triangle, above an
+// inner node stored at index 2 n - 2 - id, so that the root, merged last, is
+// node 0 and children come after their parents), and its collapse tables.
+__device__ __forceinline__ void write_node2(uint32_t index, uint32_t n, const uint32_t id[2], const float4 lo[2],
+                                            const float4 hi[2], float delta, bool want8, float tri_cost,
+                                            float4* __restrict__ nodes2, float4* cost, uint4* meta) {
+    const uint32_t last = 2 * n - 2;
+    Grown g[2];
+    int32_t link[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        g[c].lo = make_float4(__fsub_rn(lo[c].x, delta), __fsub_rn(lo[c].y, delta), __fsub_rn(lo[c].z, delta), 0.0f);
+        g[c].hi = make_float4(__fadd_rn(hi[c].x, delta), __fadd_rn(hi[c].y, delta), __fadd_rn(hi[c].z, delta), 0.0f);
+        link[c] = id[c] < n ? (int32_t)~(id[c] << 3) : (int32_t)(last - id[c]);
+    }
+    float4* o = nodes2 + 4 * (size_t)index;
+    o[0] = make_float4(g[0].lo.x, g[0].hi.x, g[0].lo.y, g[0].hi.y);
+    o[1] = make_float4(g[1].lo.x, g[1].hi.x, g[1].lo.y, g[1].hi.y);
+    o[2] = make_float4(g[0].lo.z, g[0].hi.z, g[1].lo.z, g[1].hi.z);
+    o[3] = make_float4(__int_as_float(link[0]), __int_as_float(link[1]), 0.0f, 0.0f);
+    if (!want8) return;
+    float cc[2][8];
+    uint32_t tris = 0;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        if (link[c] < 0) {
+            const float a = __fmul_rn(box_area(g[c].lo, g[c].hi), tri_cost);
+#pragma unroll
+            for (int s = 0; s < 8; ++s) cc[c][s] = a;
+            tris += 1;
+        } else {
+            const float4 x = __ldcg(&cost[2 * (size_t)link[c]]), y = __ldcg(&cost[2 * (size_t)link[c] + 1]);
+            cc[c][0] = x.x; cc[c][1] = x.y; cc[c][2] = x.z; cc[c][3] = x.w;
+            cc[c][4] = y.x; cc[c][5] = y.y; cc[c][6] = y.z; cc[c][7] = y.w;
+            tris += __ldcg(&meta[link[c]]).z;
         }
     }
-    __syncthreads();
-    const int i = b0 + (int)threadIdx.x;
-    if (i >= (int)m) return;
-    const float4 alo = s_lo[threadIdx.x + R], ahi = s_hi[threadIdx.x + R];
-    unsigned long long best = ~0ull;
-    for (int d = -R; d <= R; ++d) {
-        const int j = i + d;
-        if (d == 0 || j < 0 || j >= (int)m) continue;
-        const float4 blo = s_lo[threadIdx.x + R + d], bhi = s_hi[threadIdx.x + R + d];
-        const float4 ulo = make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), 0.0f);
-        const float4 uhi = make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.0f);
-        const unsigned long long key =
-            ((unsigned long long)__float_as_uint(box_area(ulo, uhi)) << 32) | (uint32_t)j;
-        best = key < best ? key : best;
+    const float4 ulo = make_float4(fminf(g[0].lo.x, g[1].lo.x), fminf(g[0].lo.y, g[1].lo.y), fminf(g[0].lo.z, g[1].lo.z), 0.0f);
+    const float4 uhi = make_float4(fmaxf(g[0].hi.x, g[1].hi.x), fmaxf(g[0].hi.y, g[1].hi.y), fmaxf(g[0].hi.z, g[1].hi.z), 0.0f);
+    const float A = box_area(ulo, uhi);
+    const float inf = __int_as_float(0x7f800000);
+    float dist[9];
+    uint32_t arg[9];
+#pragma unroll
+    for (int j = 2; j <= 8; ++j) {
+        dist[j] = inf;
+        arg[j] = 1;
+#pragma unroll
+        for (int a = 1; a < j; ++a) {
+            const float c = __fadd_rn(cc[0][a - 1], cc[1][j - a - 1]);
+            if (c < dist[j]) {
+                dist[j] = c;
+                arg[j] = a;
+            }
+        }
     }
-    nn[i] = (uint32_t)best;
+    const float c_inner = __fadd_rn(A, dist[8]);
+    const float c_leaf = tris <= 3 ? __fmul_rn(__fmul_rn(A, (float)tris), tri_cost) : inf;
+    float out[8];
+    uint32_t how[2] = {c_leaf <= c_inner ? 0xFFu : 0u, 0u};
+    out[0] = fminf(c_leaf, c_inner);
+#pragma unroll
+    for (int s = 2; s <= 8; ++s) {
+        const bool split = dist[s] < out[s - 2];
+        out[s - 1] = split ? dist[s] : out[s - 2];
+        how[(s - 1) >> 2] |= (split ? arg[s] : 0u) << (8 * ((s - 1) & 3));
+    }
+    __stcg(&cost[2 * (size_t)index], make_float4(out[0], out[1], out[2], out[3]));
+    __stcg(&cost[2 * (size_t)index + 1], make_float4(out[4], out[5], out[6], out[7]));
+    __stcg(&meta[index], make_uint4(how[0], how[1], tris, arg[8]));
 }
 
-// flags[i] = merge << 32 | keep: a mutual pair merges into its lower
-// position; the upper one is dropped.
-__global__ void __launch_bounds__(kBB) k_ploc_flags(const uint32_t* __restrict__ nn, uint32_t m,
-                                                    uint64_t* __restrict__ flags) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    const uint32_t j = nn[i];
-    const bool mutual = j < m && nn[j] == i;
-    const bool merge = mutual && i < j;
-    const bool keep = !(mutual && i > j);
-    flags[i] = ((uint64_t)merge << 32) | (uint64_t)keep;
-}
-
-__global__ void __launch_bounds__(kBB) k_ploc_merge(const uint32_t* __restrict__ cl, const uint32_t* __restrict__ nn,
-                                                    uint32_t m, const uint64_t* __restrict__ excl, uint32_t next_id,
-                                                    uint32_t n_leaves, uint32_t cap, float4* __restrict__ nlo,
-                                                    float4* __restrict__ nhi, int2* __restrict__ kids,
-                                                    uint32_t* __restrict__ parent, uint32_t* __restrict__ cl_out) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    const uint32_t j = nn[i];
-    const bool mutual = j < m && nn[j] == i;
-    if (mutual && i > j) return;  // merged by its partner
-    const uint64_t e = excl[i];
-    const uint32_t posn = (uint32_t)e;
-    if (!(mutual && i < j)) {
-        cl_out[posn] = cl[i];
-        return;
+// The whole clustering.  A block takes tiles of kBB - 2 R cluster positions
+// and holds the boxes of the tile and of 2 R positions on either side in
+// shared memory: enough to find the nearest neighbour (least merged surface
+// area, ties to the smaller position) of every position of the tile and of
+// the R on either side, hence the mutual pairs that start or end in the
+// tile.  For a fixed cluster that order is the order of (area, smaller
+// position, larger position) over pairs, so the pair that is least in that
+// order over all pairs is mutual and every pass merges at least one pair.
+// A pair's node is made by the block of its lower position, the first
+// threads of the block taking one pair each.  The pass ends at a barrier of
+// the blocks that had a tile; blocks without one are done for good, since
+// the list only shrinks, and once one tile is left its block goes on alone.
+//
+// Bound by latency: 3M triangles take 52 passes, the 40 last of them with
+// less than one tile per SM, each a chain of a few dependent L2 round trips
+// (28 % issue active, 1.1 TB/s).  0.88 ms, against 0.97 ms for the same passes
+// as separate kernels (neighbours, flags, a three-launch prefix sum, merge)
+// with as much again in launches and a host read-back per pass, plus 0.82 ms
+// for the BVH2 nodes and the collapse tables in kernels of their own.  Four
+// blocks per SM: whole 3M build 2.68 ms with three, 2.58 with four, 2.59 with
+// five.
+__global__ void __launch_bounds__(kBB, 4) k_ploc(uint32_t* cl_a, uint32_t* cl_b, uint32_t n, int radius,
+                                                 float4* boxes, float4* __restrict__ nodes2, float4* cost,
+                                                 uint4* meta, int want8, float tri_cost, unsigned long long* state,
+                                                 BuildStats* st) {
+    constexpr int kMost = kBB + 2 * kPlocRMax;
+    __shared__ float4 s_lo[kMost], s_hi[kMost];
+    __shared__ uint32_t s_id[kMost], s_nn[kBB], s_pair[kBB], s_warp[kBB / 32];
+    __shared__ unsigned long long s_base;
+    const int R = radius < 1 ? 1 : (radius > kPlocRMax ? kPlocRMax : radius);
+    const int T = kBB - 2 * R;
+    const int tid = (int)threadIdx.x;
+    const uint32_t cap = 2 * n - 1;
+    const float delta = __fmul_rn(__uint_as_float(st->pmax), 0x1p-22f);
+    uint32_t m = n, next_id = n, iter = 0, target = 0;
+    while (m > 1) {
+        const uint32_t ntiles = (m + T - 1) / T;
+        const uint32_t nblocks = min(gridDim.x, ntiles);
+        if (blockIdx.x >= nblocks) return;
+        const uint32_t* cin = (iter & 1) ? cl_b : cl_a;
+        uint32_t* cout = (iter & 1) ? cl_a : cl_b;
+        for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+            const int b0 = (int)tile * T;
+            for (int t = tid; t < kBB + 2 * R; t += kBB) {
+                const int j = b0 - 2 * R + t;
+                if (j >= 0 && j < (int)m) {
+                    const uint32_t id = __ldcg(&cin[j]);
+                    s_id[t] = id;
+                    if (id < cap) {
+                        s_lo[t] = __ldcg(&boxes[2 * (size_t)id]);
+                        s_hi[t] = __ldcg(&boxes[2 * (size_t)id + 1]);
+                    }
+                }
+            }
+            __syncthreads();
+            const int i = b0 - R + tid;
+            uint32_t nn = kNone;
+            if (i >= 0 && i < (int)m) {
+                const float4 alo = s_lo[tid + R], ahi = s_hi[tid + R];
+                uint32_t best = kNone;
+                const int d0 = max(-R, -i), d1 = min(R, (int)m - 1 - i);
+                for (int d = d0; d <= d1; ++d) {
+                    if (d == 0) continue;
+                    const float4 blo = s_lo[tid + R + d], bhi = s_hi[tid + R + d];
+                    const float4 ulo = make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), 0.0f);
+                    const float4 uhi = make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.0f);
+                    const uint32_t key = __float_as_uint(box_area(ulo, uhi));
+                    if (key < best) {
+                        best = key;
+                        nn = (uint32_t)(i + d);
+                    }
+                }
+            }
+            s_nn[tid] = nn;
+            __syncthreads();
+            bool keep = false, merge = false;
+            if (tid >= R && tid < R + T && i < (int)m) {
+                const bool mutual = nn != kNone && s_nn[tid + ((int)nn - i)] == (uint32_t)i;
+                merge = mutual && i < (int)nn;
+                keep = !(mutual && i > (int)nn);
+            }
+            uint32_t total;
+            const uint32_t rank = block_scan(((uint32_t)merge << 16) | (uint32_t)keep, s_warp, &total);
+            const uint32_t pairs = total >> 16, kept = total & 0xFFFFu;
+            if (tid < 32) {
+                const uint64_t p = tile_prefix64(state, tile, ((uint64_t)pairs << 28) | kept, iter);
+                if (tid == 0) s_base = p;
+            }
+            if (merge) s_pair[rank >> 16] = (uint32_t)tid;
+            __syncthreads();
+            const uint32_t id0 = next_id + (uint32_t)(s_base >> 28), pos0 = (uint32_t)s_base & 0xFFFFFFFu;
+            if (keep) {
+                const uint32_t at = pos0 + (rank & 0xFFFFu);
+                if (at < m) __stcg(&cout[at], merge ? id0 + (rank >> 16) : s_id[tid + R]);
+                else raise_status(kErrBounds);
+            }
+            if (tid < (int)pairs) {
+                const int t = (int)s_pair[tid], li = t + R, lj = li + ((int)s_nn[t] - (b0 - R + t));
+                const uint32_t id = id0 + (uint32_t)tid;
+                const uint32_t kid[2] = {s_id[li], s_id[lj]};
+                if (id < cap && kid[0] < id && kid[1] < id) {
+                    const float4 lo[2] = {s_lo[li], s_lo[lj]}, hi[2] = {s_hi[li], s_hi[lj]};
+                    __stcg(&boxes[2 * (size_t)id], make_float4(fminf(lo[0].x, lo[1].x), fminf(lo[0].y, lo[1].y), fminf(lo[0].z, lo[1].z), 0.0f));
+                    __stcg(&boxes[2 * (size_t)id + 1], make_float4(fmaxf(hi[0].x, hi[1].x), fmaxf(hi[0].y, hi[1].y), fmaxf(hi[0].z, hi[1].z), 0.0f));
+                    write_node2(2 * n - 2 - id, n, kid, lo, hi, delta, want8 != 0, tri_cost, nodes2, cost, meta);
+                } else {
+                    raise_status(kErrBounds);
+                }
+            }
+            if (tile == ntiles - 1 && tid == 0) {
+                st->clusters = pos0 + kept;
+                st->next_id = id0 + pairs;
+            }
+            __syncthreads();
+        }
+        target += nblocks;
+        if (nblocks > 1 && !block_barrier(&st->ploc_barrier, target)) return;
+        const uint32_t left = __ldcg(&st->clusters);
+        next_id = __ldcg(&st->next_id);
+        ++iter;
+        if (blockIdx.x == 0 && tid == 0) {
+            st->iterations = iter;
+            if (left >= m) st->stuck = 1;
+        }
+        if (left >= m) return;
+        m = left;
+        // A lone block rewrites st->clusters in its next pass: not before
+        // every thread has read it.
+        __syncthreads();
     }
-    const uint32_t id = next_id + (uint32_t)(e >> 32);
-    const uint32_t a = cl[i], b = cl[j];
-    if (id >= cap || a >= cap || b >= cap || id < n_leaves) {
-        raise_status(kErrBounds);
-        return;
-    }
-    const float4 alo = nlo[a], ahi = nhi[a], blo = nlo[b], bhi = nhi[b];
-    nlo[id] = make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), 0.0f);
-    nhi[id] = make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.0f);
-    kids[id - n_leaves] = make_int2((int)a, (int)b);
-    parent[a] = id;
-    parent[b] = id;
-    cl_out[posn] = id;
 }
 
 // ---------------------------------------------------------------- stage 4
-// Inner node id (n_leaves .. 2 n_leaves - 2, in creation order) -> BVH2
-// index 2 n_leaves - 2 - id: the root (created last) is node 0 and children
-// come after their parents.
-__global__ void __launch_bounds__(kBB) k_write_bvh2(uint32_t n, const int2* __restrict__ kids,
-                                                    const float4* __restrict__ nlo, const float4* __restrict__ nhi,
-                                                    const BuildStats* __restrict__ st, Bvh2Node* __restrict__ out) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k + 1 >= n) return;
-    const uint32_t last = 2 * n - 2;
-    const uint32_t index = last - (n + k);
-    // Same growth as the host builder: delta = 2^-22 * P.
-    const float delta = __fmul_rn(__uint_as_float(st->pmax), 0x1p-22f);
-    Bvh2Node node;
-    const int2 ch = kids[k];
-    for (int c = 0; c < 2; ++c) {
-        const uint32_t id = (uint32_t)(c == 0 ? ch.x : ch.y);
-        const float4 lo = nlo[id], hi = nhi[id];
-        const float lx = __fsub_rn(lo.x, delta), ly = __fsub_rn(lo.y, delta), lz = __fsub_rn(lo.z, delta);
-        const float hx = __fadd_rn(hi.x, delta), hy = __fadd_rn(hi.y, delta), hz = __fadd_rn(hi.z, delta);
-        const int o = c == 0 ? 0 : 4;
-        node.f[o + 0] = lx;
-        node.f[o + 1] = hx;
-        node.f[o + 2] = ly;
-        node.f[o + 3] = hy;
-        node.f[8 + 2 * c] = lz;
-        node.f[9 + 2 * c] = hz;
-        node.link[c] = id < n ? (int32_t)~(id << 3) : (int32_t)(last - id);
-    }
-    node.link[2] = 0;
-    node.link[3] = 0;
-    out[index] = node;
-}
-
-// ---------------------------------------------------------------- stage 5
-__device__ __forceinline__ float4 child_lo(const Bvh2Node& n, int c) {
-    return c == 0 ? make_float4(n.f[0], n.f[2], n.f[8], 0.0f) : make_float4(n.f[4], n.f[6], n.f[10], 0.0f);
-}
-__device__ __forceinline__ float4 child_hi(const Bvh2Node& n, int c) {
-    return c == 0 ? make_float4(n.f[1], n.f[3], n.f[9], 0.0f) : make_float4(n.f[5], n.f[7], n.f[11], 0.0f);
-}
-
-__device__ __forceinline__ Bvh2Node load_node(const Bvh2Node* nodes, uint32_t i) {
-    const float4* p = reinterpret_cast<const float4*>(nodes + i);
-    Bvh2Node n;
-    float4* q = reinterpret_cast<float4*>(&n);
-    for (int k = 0; k < 4; ++k) q[k] = __ldg(p + k);
-    return n;
-}
-
-// Bottom-up SAH collapse tables (the host's plan_sah): cost[i*8 + s-1] is
-// the least cost of node i's subtree with at most s BVH8 children; how[i*8]
-// -1 = one leaf child, 0 = one inner child; how[i*8 + s-1] (s > 1) 0 = same
-// as s-1, a > 0 = a slots to child 0; split8[i] = child 0's slots when the
-// node is a BVH8 inner node.
-__global__ void __launch_bounds__(kBB) k_collapse_dp(uint32_t n, const Bvh2Node* __restrict__ nodes,
-                                                     const uint32_t* __restrict__ parent,
-                                                     uint32_t* __restrict__ visits, float* __restrict__ cost,
-                                                     int8_t* __restrict__ how, int8_t* __restrict__ split8,
-                                                     uint32_t* __restrict__ ntris, float tri_cost) {
-    const uint32_t leaf = blockIdx.x * blockDim.x + threadIdx.x;
-    if (leaf >= n) return;
-    const uint32_t last = 2 * n - 2;
-    uint32_t pid = parent[leaf];
-    for (uint32_t guard = 0; pid != kNone && guard < n; ++guard) {
-        if (pid < n || pid > last) {
-            raise_status(kErrBounds);
-            return;
-        }
-        const uint32_t i = last - pid;
-        __threadfence();
-        if (atomicAdd(&visits[i], 1u) == 0u) return;  // the sibling's thread computes it
-        __threadfence();
-        const Bvh2Node nd = load_node(nodes, i);
-        float cc[2][8];
-        uint32_t tc[2];
-        float4 ulo, uhi;
-        for (int c = 0; c < 2; ++c) {
-            const float4 lo = child_lo(nd, c), hi = child_hi(nd, c);
-            if (c == 0) {
-                ulo = lo;
-                uhi = hi;
-            } else {
-                ulo = make_float4(fminf(ulo.x, lo.x), fminf(ulo.y, lo.y), fminf(ulo.z, lo.z), 0.0f);
-                uhi = make_float4(fmaxf(uhi.x, hi.x), fmaxf(uhi.y, hi.y), fmaxf(uhi.z, hi.z), 0.0f);
-            }
-            const int32_t link = nd.link[c];
-            if (link < 0) {
-                const uint32_t cnt = ((~(uint32_t)link) & 7u) + 1u;
-                const float a = __fmul_rn(__fmul_rn(box_area(lo, hi), (float)cnt), tri_cost);
-                for (int s = 0; s < 8; ++s) cc[c][s] = a;
-                tc[c] = cnt;
-            } else {
-                for (int s = 0; s < 8; ++s) cc[c][s] = __ldcg(&cost[(size_t)link * 8 + s]);
-                tc[c] = __ldcg(&ntris[link]);
-            }
-        }
-        const float A = box_area(ulo, uhi);
-        float dist[9];
-        int8_t arg[9];
-        for (int j = 2; j <= 8; ++j) {
-            dist[j] = __int_as_float(0x7f800000);
-            arg[j] = 1;
-            for (int a = 1; a < j; ++a) {
-                const float c = __fadd_rn(cc[0][a - 1], cc[1][j - a - 1]);
-                if (c < dist[j]) {
-                    dist[j] = c;
-                    arg[j] = (int8_t)a;
-                }
-            }
-        }
-        const uint32_t t = tc[0] + tc[1];
-        const float c_inner = __fadd_rn(A, dist[8]);
-        const float c_leaf = t <= 3 ? __fmul_rn(__fmul_rn(A, (float)t), tri_cost) : __int_as_float(0x7f800000);
-        float prev = fminf(c_leaf, c_inner);
-        __stcg(&cost[(size_t)i * 8], prev);
-        __stcg(&how[(size_t)i * 8], (int8_t)(c_leaf <= c_inner ? -1 : 0));
-        for (int s = 2; s <= 8; ++s) {
-            int8_t h = 0;
-            if (dist[s] < prev) {
-                prev = dist[s];
-                h = arg[s];
-            }
-            __stcg(&cost[(size_t)i * 8 + s - 1], prev);
-            __stcg(&how[(size_t)i * 8 + s - 1], h);
-        }
-        __stcg(&split8[i], arg[8]);
-        __stcg(&ntris[i], t);
-        pid = parent[pid];
-    }
-}
-
-struct Child8 {
-    int32_t link;      // BVH2 link
-    uint32_t parent;   // BVH2 node holding the child's box
-    uint8_t k;         // which child of `parent`
-    uint8_t leaf;      // becomes a leaf child
-    uint8_t tris;      // triangles of a leaf child
-};
-
-// The BVH8 children of BVH2 node `node` as an inner BVH8 node (the host's
-// collect over split8): child 0's share first, each share depth-first.
-__device__ int collect8(const Bvh2Node* __restrict__ nodes, const int8_t* __restrict__ how,
-                        const int8_t* __restrict__ split8, const uint32_t* __restrict__ ntris, uint32_t node,
-                        Child8* out) {
-    struct Item {
-        uint32_t p;
-        uint8_t k, s;
-    };
-    Item st[16];
-    int sp = 0, cnt = 0;
-    const int a8 = split8[node];
-    st[sp++] = {node, 1, (uint8_t)(8 - a8)};
-    st[sp++] = {node, 0, (uint8_t)a8};
-    while (sp > 0 && cnt < 8) {
-        const Item it = st[--sp];
-        const Bvh2Node pn = load_node(nodes, it.p);
-        const int32_t link = pn.link[it.k];
-        if (link < 0) {
-            out[cnt++] = {link, it.p, it.k, 1, (uint8_t)(((~(uint32_t)link) & 7u) + 1u)};
-            continue;
-        }
-        int s = it.s;
-        while (s > 1 && how[(size_t)link * 8 + s - 1] == 0) --s;
-        if (s <= 1) {
-            const bool lf = how[(size_t)link * 8] == -1;
-            out[cnt++] = {link, it.p, it.k, (uint8_t)(lf ? 1 : 0), (uint8_t)(lf ? ntris[link] : 0)};
-            continue;
-        }
-        const int a = how[(size_t)link * 8 + s - 1];
-        if (sp + 2 > 16) break;  // cannot happen: at most 8 children
-        st[sp++] = {(uint32_t)link, 1, (uint8_t)(s - a)};
-        st[sp++] = {(uint32_t)link, 0, (uint8_t)a};
-    }
-    return cnt;
-}
-
-__global__ void __launch_bounds__(kBB) k_emit_count(const uint2* __restrict__ tasks, uint32_t ntasks,
-                                                    const Bvh2Node* __restrict__ nodes, const int8_t* __restrict__ how,
-                                                    const int8_t* __restrict__ split8,
-                                                    const uint32_t* __restrict__ ntris, uint64_t* __restrict__ counts) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ntasks) return;
-    Child8 ch[8];
-    const int nc = collect8(nodes, how, split8, ntris, tasks[t].y, ch);
-    uint32_t inner = 0, tris = 0;
-    for (int c = 0; c < nc; ++c) {
-        if (ch[c].leaf) tris += ch[c].tris;
-        else ++inner;
-    }
-    counts[t] = ((uint64_t)inner << 32) | tris;
-}
-
 // Triangles of a leaf child (a subtree of at most three triangles), depth
 // first, child 0 first, like the host's gather_tris.
 __device__ int gather3(const Bvh2Node* __restrict__ nodes, int32_t link, uint32_t* recs) {
@@ -590,158 +551,314 @@ __device__ int gather3(const Bvh2Node* __restrict__ nodes, int32_t link, uint32_
             for (uint32_t q = 0; q < c && cnt < 3; ++q) recs[cnt++] = first + q;
             continue;
         }
-        const Bvh2Node nd = load_node(nodes, (uint32_t)l);
+        const int2 kids = *reinterpret_cast<const int2*>(nodes[l].link);
         if (sp + 2 > 8) break;
-        st[sp++] = nd.link[1];
-        st[sp++] = nd.link[0];
+        st[sp++] = kids.y;
+        st[sp++] = kids.x;
     }
     return cnt;
 }
 
-__global__ void __launch_bounds__(kBB) k_emit_write(const uint2* __restrict__ tasks, uint32_t ntasks,
-                                                    const uint64_t* __restrict__ excl, uint32_t node_base,
-                                                    uint32_t tri_base0, uint32_t node_cap, uint32_t tri_cap,
-                                                    const Bvh2Node* __restrict__ nodes,
-                                                    const int8_t* __restrict__ how, const int8_t* __restrict__ split8,
-                                                    const uint32_t* __restrict__ ntris,
-                                                    const float4* __restrict__ recs2, Bvh8Node* __restrict__ out,
-                                                    float4* __restrict__ recs8,
-                                                    uint2* __restrict__ next_tasks) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ntasks) return;
-    const uint2 task = tasks[t];
-    Child8 ch[8];
-    const int nc = collect8(nodes, how, split8, ntris, task.y, ch);
-    const uint64_t e = excl[t];
-    const uint32_t inner_off = (uint32_t)(e >> 32), tri_off0 = (uint32_t)e;
-    Bvh8Node node;
-    memset(&node, 0, sizeof(node));
-    float4 clo[8], chi[8];
-    float nlo[3] = {__int_as_float(0x7f800000), __int_as_float(0x7f800000), __int_as_float(0x7f800000)};
-    float nhi[3] = {-nlo[0], -nlo[1], -nlo[2]};
-    for (int c = 0; c < nc; ++c) {
-        const Bvh2Node pn = load_node(nodes, ch[c].parent);
-        clo[c] = child_lo(pn, ch[c].k);
-        chi[c] = child_hi(pn, ch[c].k);
-        nlo[0] = fminf(nlo[0], clo[c].x);
-        nlo[1] = fminf(nlo[1], clo[c].y);
-        nlo[2] = fminf(nlo[2], clo[c].z);
-        nhi[0] = fmaxf(nhi[0], chi[c].x);
-        nhi[1] = fmaxf(nhi[1], chi[c].y);
-        nhi[2] = fmaxf(nhi[2], chi[c].z);
-    }
-    // Quantisation grid (the host's emit_children): the smallest power-of-two
-    // scale whose 255 steps from the box minimum reach the box maximum.
-    float scale[3];
-    for (int k = 0; k < 3; ++k) {
-        node.p[k] = nlo[k];
-        const float ext = __fsub_rn(nhi[k], nlo[k]);
-        int ex = -126;
-        if (ext > 0.0f) {
-            int e2;
-            frexpf(__fdiv_rn(ext, 255.0f), &e2);
-            ex = e2;
-        }
-        for (int guard = 0; guard < 300; ++guard) {
-            ex = max(-126, min(127, ex));
-            scale[k] = ldexpf(1.0f, ex);
-            const float top = __fadd_rn(node.p[k], __fmul_rn(255.0f, scale[k]));
-            if (top >= nhi[k] || ex == 127) break;
-            ++ex;
-        }
-        node.e[k] = (uint8_t)(ex + 127);
-    }
-    // Slots: greedy by descending octant score, ties to the lower (child,
-    // slot) pair, as the host's stable sort.
-    float pc[3];
-    for (int k = 0; k < 3; ++k) pc[k] = __fmul_rn(0.5f, __fadd_rn(nlo[k], nhi[k]));
-    float off[8][3];
-    for (int c = 0; c < nc; ++c) {
-        off[c][0] = __fsub_rn(__fmul_rn(0.5f, __fadd_rn(clo[c].x, chi[c].x)), pc[0]);
-        off[c][1] = __fsub_rn(__fmul_rn(0.5f, __fadd_rn(clo[c].y, chi[c].y)), pc[1]);
-        off[c][2] = __fsub_rn(__fmul_rn(0.5f, __fadd_rn(clo[c].z, chi[c].z)), pc[2]);
-    }
-    int slot_of[8], child_at[8];
-    for (int q = 0; q < 8; ++q) slot_of[q] = child_at[q] = -1;
-    for (int round = 0; round < nc; ++round) {
-        float best = 0.0f;
-        int bc = -1, bs = -1;
-        for (int c = 0; c < nc; ++c) {
-            if (slot_of[c] >= 0) continue;
-            for (int sl = 0; sl < 8; ++sl) {
-                if (child_at[sl] >= 0) continue;
-                float sc = 0.0f;
-                for (int k = 0; k < 3; ++k) sc = __fadd_rn(sc, ((sl >> k) & 1) ? -off[c][k] : off[c][k]);
-                if (bc < 0 || sc > best) {
-                    best = sc;
-                    bc = c;
-                    bs = sl;
-                }
-            }
-        }
-        if (bc < 0) break;
-        slot_of[bc] = bs;
-        child_at[bs] = bc;
-    }
-    const uint32_t child_base = node_base + inner_off;
-    const uint32_t tri_base = tri_base0 + tri_off0;
-    node.child_base = child_base;
-    node.tri_base = tri_base;
-    uint32_t inner_i = 0, tri_off = 0;
-    for (int sl = 0; sl < 8; ++sl) {
-        const int ci = child_at[sl];
-        if (ci < 0) continue;
-        const Child8& c = ch[ci];
-        const float lo3[3] = {clo[ci].x, clo[ci].y, clo[ci].z}, hi3[3] = {chi[ci].x, chi[ci].y, chi[ci].z};
-        for (int k = 0; k < 3; ++k) {
-            const float sc = scale[k];
-            const float lo = floorf(__fdiv_rn(__fsub_rn(lo3[k], node.p[k]), sc));
-            const float hi = ceilf(__fdiv_rn(__fsub_rn(hi3[k], node.p[k]), sc));
-            int ql = (int)fmaxf(0.0f, fminf(255.0f, lo));
-            int qh = (int)fmaxf(0.0f, fminf(255.0f, hi));
-            while (ql > 0 && __fadd_rn(node.p[k], __fmul_rn((float)ql, sc)) > lo3[k]) --ql;
-            while (qh < 255 && __fadd_rn(node.p[k], __fmul_rn((float)qh, sc)) < hi3[k]) ++qh;
-            uint8_t* qlo = k == 0 ? node.qlo_x : (k == 1 ? node.qlo_y : node.qlo_z);
-            uint8_t* qhi = k == 0 ? node.qhi_x : (k == 1 ? node.qhi_y : node.qhi_z);
-            qlo[sl] = (uint8_t)ql;
-            qhi[sl] = (uint8_t)qh;
-        }
-        if (c.leaf) {
-            uint32_t r[3];
-            const int cnt = gather3(nodes, c.link, r);
-            const uint32_t unary = cnt == 1 ? 1u : (cnt == 2 ? 3u : 7u);
-            node.meta[sl] = (uint8_t)((unary << 5) | tri_off);
-            for (int q = 0; q < cnt; ++q) {
-                const uint32_t dst = tri_base + tri_off + q;
-                if (dst >= tri_cap) {
-                    raise_status(kErrBounds);
-                    continue;
-                }
-                const float4 a = recs2[3 * (size_t)r[q]], b = recs2[3 * (size_t)r[q] + 1],
-                             cc = recs2[3 * (size_t)r[q] + 2];
-                recs8[3 * (size_t)dst] = a;
-                recs8[3 * (size_t)dst + 1] = b;
-                recs8[3 * (size_t)dst + 2] = cc;
-            }
-            tri_off += (uint32_t)cnt;
-        } else {
-            node.imask |= (uint8_t)(1u << sl);
-            node.meta[sl] = (uint8_t)((1u << 5) | (24u + (uint32_t)sl));
-            if (child_base + inner_i < node_cap) next_tasks[inner_off + inner_i] = make_uint2(child_base + inner_i, (uint32_t)c.link);
-            else raise_status(kErrBounds);
-            ++inner_i;
-        }
-    }
-    if (task.x < node_cap) out[task.x] = node;
-    else raise_status(kErrBounds);
+__device__ __forceinline__ uint32_t how_of(const uint4& m, int s) {  // byte how[s - 1]
+    return ((s <= 4 ? m.x : m.y) >> (8 * ((s - 1) & 3))) & 0xFFu;
 }
 
-template <typename T>
-cudaError_t dalloc(T** p, size_t count) {
-    return dev_malloc(reinterpret_cast<void**>(p), std::max<size_t>(1, count) * sizeof(T));
+// The whole emission, a level of BVH8 nodes per round: eight lanes per node,
+// 32 nodes per block and tile.
+//  - Children: a node's eight slots are the lanes of its group.  Each lane
+//    walks from the node to the child that covers its slot, going to child 0
+//    or 1 by the slots that the tables give each; lanes of one child make the
+//    same steps, and the first of them owns it (so children are in lane
+//    order, child 0's share first, as the host collects them).
+//  - Node box, quantisation grid and the greedy slot assignment (descending
+//    octant score, ties to the lower (child, slot) pair, as the host's stable
+//    sort) by shuffles in the group; then lane = slot.
+//  - A tile's inner children and triangles get their places by look-back over
+//    the level's tiles, in task order.
+// The level's children are the next level's tasks; a barrier of all blocks
+// ends a level.  One thread per node, with the children collected twice (once
+// to count) and a prefix sum and a read-back per level, took 1.24 ms for 3M
+// triangles; this takes 0.52 ms.
+constexpr int kEmitTile = kBB / 8;
+__global__ void __launch_bounds__(kBB, 4) k_emit8(uint32_t* tasks_a, uint32_t* tasks_b, uint32_t n,
+                                                  const Bvh2Node* __restrict__ nodes, const uint4* __restrict__ meta,
+                                                  const float4* __restrict__ recs2, float4* __restrict__ out,
+                                                  float4* __restrict__ recs8, unsigned long long* state,
+                                                  BuildStats* st) {
+    __shared__ uint32_t s_warp[kBB / 32];
+    __shared__ unsigned long long s_base;
+    __shared__ uint8_t s_at[kBB];
+    __shared__ __align__(16) uint8_t s_node[kEmitTile][80];
+    const uint32_t lane = threadIdx.x & 31, l = lane & 7, group = lane & 24u, slot_group = threadIdx.x >> 3;
+    const uint32_t node_cap = n - 1;
+    const float inf = __int_as_float(0x7f800000);
+    uint32_t ntasks = 1, level_base = 0, tri_base0 = 0, target = 0;
+    for (uint32_t level = 0; ntasks > 0; ++level) {
+        if (level > 64 || ntasks > node_cap || level_base + ntasks > node_cap) {  // cannot happen
+            if (blockIdx.x == 0 && threadIdx.x == 0) st->stuck = 1;
+            return;
+        }
+        const uint32_t* tin = (level & 1) ? tasks_b : tasks_a;
+        uint32_t* tout = (level & 1) ? tasks_a : tasks_b;
+        const uint32_t node_base = level_base + ntasks;  // the next level's first node
+        const uint32_t ntiles = (ntasks + kEmitTile - 1) / kEmitTile;
+        for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+            const uint32_t task = tile * kEmitTile + slot_group;
+            const bool valid = task < ntasks;
+            // This lane's child.
+            uint32_t p = 0, k = 0, pos = 0, ntri = 0;
+            int32_t link = 0;
+            bool leaf = false;
+            if (valid) {
+                p = level == 0 ? 0u : __ldcg(&tin[task]);
+                if (p >= node_cap) {
+                    raise_status(kErrBounds);
+                    p = 0;
+                }
+                int s = (int)meta[p].w;
+                if ((int)l >= s) {
+                    k = 1;
+                    pos = (uint32_t)s;
+                    s = 8 - s;
+                }
+                for (int step = 0; step < 8; ++step) {
+                    link = nodes[p].link[k];
+                    if (link < 0) {
+                        leaf = true;
+                        ntri = ((~(uint32_t)link) & 7u) + 1u;
+                        break;
+                    }
+                    const uint4 h = meta[link];
+                    while (s > 1 && how_of(h, s) == 0) --s;
+                    if (s <= 1) {
+                        leaf = how_of(h, 1) == 0xFFu;
+                        ntri = leaf ? h.z : 0u;
+                        break;
+                    }
+                    const int a = (int)how_of(h, s);
+                    p = (uint32_t)link;
+                    k = (int)(l - pos) < a ? 0u : 1u;
+                    if (k == 0) {
+                        s = a;
+                    } else {
+                        s -= a;
+                        pos += (uint32_t)a;
+                    }
+                }
+            }
+            const bool child = valid && l == pos;
+            // Places of the tile's inner children and triangles.
+            uint32_t total;
+            const uint32_t mine = child ? (leaf ? ntri : 1u << 16) : 0u;
+            const uint32_t before = block_scan(mine, s_warp, &total);
+            if (threadIdx.x < 32) {
+                const uint64_t q = tile_prefix64(state, tile, ((uint64_t)(total >> 16) << 28) | (total & 0xFFFFu), level);
+                if (threadIdx.x == 0) s_base = q;
+            }
+            // Box of the child (empty when this lane owns none).
+            float lo[3] = {inf, inf, inf}, hi[3] = {-inf, -inf, -inf};
+            if (child) {
+                const float4* f = reinterpret_cast<const float4*>(&nodes[p]);
+                const float4 xy = f[k];
+                const float2 z = reinterpret_cast<const float2*>(f + 2)[k];
+                lo[0] = xy.x; hi[0] = xy.y; lo[1] = xy.z; hi[1] = xy.w; lo[2] = z.x; hi[2] = z.y;
+            }
+            float nlo[3], nhi[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                nlo[a] = lo[a];
+                nhi[a] = hi[a];
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) {
+                    nlo[a] = fminf(nlo[a], __shfl_xor_sync(0xffffffffu, nlo[a], o));
+                    nhi[a] = fmaxf(nhi[a], __shfl_xor_sync(0xffffffffu, nhi[a], o));
+                }
+            }
+            // Quantisation grid (the host's emit_children): the smallest
+            // power-of-two scale whose 255 steps from the box minimum reach
+            // the box maximum; lane a of the group finds axis a's.
+            int ex = -126;
+            {
+                const float b0 = l == 0 ? nlo[0] : (l == 1 ? nlo[1] : nlo[2]);
+                const float b1 = l == 0 ? nhi[0] : (l == 1 ? nhi[1] : nhi[2]);
+                const float ext = __fsub_rn(b1, b0);
+                if (ext > 0.0f) {
+                    int e2;
+                    frexpf(__fdiv_rn(ext, 255.0f), &e2);
+                    ex = e2;
+                }
+                for (int guard = 0; guard < 300; ++guard) {
+                    ex = max(-126, min(127, ex));
+                    if (__fadd_rn(b0, __fmul_rn(255.0f, ldexpf(1.0f, ex))) >= b1 || ex == 127) break;
+                    ++ex;
+                }
+            }
+            int exs[3];
+            float scale[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                exs[a] = __shfl_sync(0xffffffffu, ex, (int)group + a);
+                scale[a] = ldexpf(1.0f, exs[a]);
+            }
+            // Slots.
+            float off[3];
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+                off[a] = __fsub_rn(__fmul_rn(0.5f, __fadd_rn(lo[a], hi[a])), __fmul_rn(0.5f, __fadd_rn(nlo[a], nhi[a])));
+            uint32_t open = 0xFFu, slot = 8u;
+            s_at[threadIdx.x] = 0xFF;
+            __syncwarp();
+            for (int round = 0; round < 8; ++round) {
+                const bool want = child && slot == 8u;
+                if (!__any_sync(0xffffffffu, want)) break;
+                float best = 0.0f;
+                uint32_t bs = 8u;
+#pragma unroll
+                for (uint32_t sl = 0; sl < 8; ++sl) {
+                    float sc = __fadd_rn(0.0f, (sl & 1u) ? -off[0] : off[0]);
+                    sc = __fadd_rn(sc, (sl & 2u) ? -off[1] : off[1]);
+                    sc = __fadd_rn(sc, (sl & 4u) ? -off[2] : off[2]);
+                    if (((open >> sl) & 1u) && (bs == 8u || sc > best)) {
+                        best = sc;
+                        bs = sl;
+                    }
+                }
+                const uint32_t key = want ? ord(__fadd_rn(best, 0.0f)) : 0u;
+                uint32_t top = key;
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
+                const uint32_t won = (__ballot_sync(0xffffffffu, want && key == top) >> group) & 0xFFu;
+                const uint32_t first = won ? (uint32_t)__ffs(won) - 1u : 0u;
+                const uint32_t taken = __shfl_sync(0xffffffffu, bs, (int)(group + first));
+                if (won) {
+                    open &= ~(1u << taken);
+                    if (l == first) {
+                        slot = bs;
+                        s_at[(threadIdx.x & ~7u) + bs] = (uint8_t)l;
+                    }
+                }
+            }
+            __syncwarp();
+            // From here on lane = slot.
+            const uint32_t src = s_at[threadIdx.x];
+            const bool has = src < 8u;
+            const int from = (int)(group + (src & 7u));
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                lo[a] = __shfl_sync(0xffffffffu, lo[a], from);
+                hi[a] = __shfl_sync(0xffffffffu, hi[a], from);
+            }
+            link = __shfl_sync(0xffffffffu, link, from);
+            leaf = __shfl_sync(0xffffffffu, (int)leaf, from) != 0 && has;
+            ntri = __shfl_sync(0xffffffffu, ntri, from);
+            if (!leaf) ntri = 0u;
+            const bool inner = has && !leaf;
+            uint32_t tri_off = ntri;  // inclusive scan over the slots
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, tri_off, o, 8);
+                if (l >= (uint32_t)o) tri_off += y;
+            }
+            tri_off -= ntri;
+            const uint32_t imask = (__ballot_sync(0xffffffffu, inner) >> group) & 0xFFu;
+            const uint32_t inner_i = __popc(imask & ((1u << l) - 1u));
+            __syncthreads();  // s_base
+            const uint32_t at = __shfl_sync(0xffffffffu, before, (int)group);
+            const uint32_t inner_off = (uint32_t)(s_base >> 28) + (at >> 16);
+            const uint32_t tri_base = tri_base0 + ((uint32_t)s_base & 0xFFFFFFFu) + (at & 0xFFFFu);
+            uint8_t* const img = s_node[slot_group];
+            uint8_t mt = 0;
+            if (leaf) mt = (uint8_t)(((ntri == 1 ? 1u : (ntri == 2 ? 3u : 7u)) << 5) | tri_off);
+            if (inner) mt = (uint8_t)((1u << 5) | (24u + l));
+            img[24 + l] = mt;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                int ql = 0, qh = 0;
+                if (has) {
+                    const float sc = scale[a];
+                    ql = (int)fmaxf(0.0f, fminf(255.0f, floorf(__fdiv_rn(__fsub_rn(lo[a], nlo[a]), sc))));
+                    qh = (int)fmaxf(0.0f, fminf(255.0f, ceilf(__fdiv_rn(__fsub_rn(hi[a], nlo[a]), sc))));
+                    while (ql > 0 && __fadd_rn(nlo[a], __fmul_rn((float)ql, sc)) > lo[a]) --ql;
+                    while (qh < 255 && __fadd_rn(nlo[a], __fmul_rn((float)qh, sc)) < hi[a]) ++qh;
+                }
+                img[32 + 8 * a + l] = (uint8_t)ql;
+                img[56 + 8 * a + l] = (uint8_t)qh;
+            }
+            if (l == 0) {
+                float* h = reinterpret_cast<float*>(img);
+                h[0] = nlo[0];
+                h[1] = nlo[1];
+                h[2] = nlo[2];
+                uint32_t* w = reinterpret_cast<uint32_t*>(img);
+                w[3] = (uint32_t)(exs[0] + 127) | ((uint32_t)(exs[1] + 127) << 8) | ((uint32_t)(exs[2] + 127) << 16) | (imask << 24);
+                w[4] = node_base + inner_off;
+                w[5] = tri_base;
+            }
+            __syncwarp();
+            if (valid && l < 5) out[5 * (size_t)(level_base + task) + l] = reinterpret_cast<const float4*>(img)[l];
+            if (inner) {
+                if (node_base + inner_off + inner_i < node_cap) __stcg(&tout[inner_off + inner_i], (uint32_t)link);
+                else raise_status(kErrBounds);
+            }
+            if (leaf) {
+                uint32_t r[3];
+                const int cnt = gather3(nodes, link, r);
+                for (int q = 0; q < cnt; ++q) {
+                    const uint32_t dst = tri_base + tri_off + (uint32_t)q;
+                    if (dst >= n || r[q] >= n) {
+                        raise_status(kErrBounds);
+                        continue;
+                    }
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) recs8[3 * (size_t)dst + c] = recs2[3 * (size_t)r[q] + c];
+                }
+            }
+            if (tile == ntiles - 1 && threadIdx.x == 0) {
+                const uint32_t tris = tri_base0 + ((uint32_t)s_base & 0xFFFFFFFu) + (total & 0xFFFFu);
+                st->tasks[level & 1] = (uint32_t)(s_base >> 28) + (total >> 16);
+                st->tris[level & 1] = tris;
+                st->tris8 = tris;
+                st->nodes8 = node_base;
+            }
+            __syncthreads();
+        }
+        target += gridDim.x;
+        if (!block_barrier(&st->emit_barrier, target)) return;
+        // (By parity: a slot is written again two levels on, after every
+        // block has read it and reached the next barrier.)
+        level_base = node_base;
+        ntasks = __ldcg(&st->tasks[level & 1]);
+        tri_base0 = __ldcg(&st->tris[level & 1]);
+    }
 }
 
 unsigned blocks(uint64_t n) { return (unsigned)((n + kBB - 1) / kBB); }
+
+// Cooperative launch of as many blocks as are resident at once, at most `want`.
+template <typename... Args>
+cudaError_t launch_resident(void (*kernel)(Args...), uint64_t want, cudaStream_t s, Args... args) {
+    int dev = 0, sms = 0, per_sm = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kBB, 0);
+    if (e != cudaSuccess) return e;
+    const uint64_t most = std::max<uint64_t>(1, (uint64_t)sms * (uint64_t)per_sm);
+    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min(most, want));
+    void* argv[] = {(void*)&args...};
+    e = cudaLaunchCooperativeKernel((const void*)kernel, dim3(grid), dim3(kBB), argv, 0, s);
+    count_launch();
+    return e;
+}
+
+// Offsets into the build's one temporary allocation.
+struct Arena {
+    size_t bytes = 0;
+    size_t take(size_t b) {
+        const size_t at = bytes;
+        bytes += (b + 255) & ~(size_t)255;
+        return at;
+    }
+};
 
 }  // namespace
 
@@ -752,190 +869,102 @@ cudaError_t build_scene_device(const float* positions_dev, uint32_t num_vertices
     if (n < 2 || !out || num_geoms == 0) return cudaErrorInvalidValue;
     *out = DeviceBuild{};
     cudaError_t e = cudaSuccess;
-    // Temporaries, freed at the end.
-    float4 *tlo = nullptr, *thi = nullptr, *nlo = nullptr, *nhi = nullptr;
-    uint64_t *keys = nullptr, *flags = nullptr, *excl = nullptr, *bsums = nullptr, *total = nullptr;
-    uint32_t *vals = nullptr, *cl = nullptr, *cl2 = nullptr, *nn = nullptr, *parent = nullptr;
-    int2* kids = nullptr;
-    BuildStats* st = nullptr;
-    unsigned char* sort_scratch = nullptr;
-    float* cost = nullptr;
-    int8_t *how = nullptr, *split8 = nullptr;
-    uint32_t *ntris = nullptr, *visits = nullptr;
-    uint2 *tasks = nullptr, *tasks2 = nullptr;
-    Bvh8Node* nodes8_tmp = nullptr;
+    const size_t ninner = (size_t)n - 1, nall = 2 * (size_t)n - 1;
+    const size_t sort_bytes = sort_scratch_bytes(n, 63);
+    const int radius = g_ploc_radius;
+    // Temporaries in one allocation (an allocation and its release cost
+    // 0.05-0.1 ms each; 29 of them were a third of a 3M-triangle build).  The
+    // BVH8 nodes are emitted over the sort's and the clustering's buffers,
+    // which are dead by then, and copied to their exact size.
+    Arena ar;
+    const size_t o_keys = ar.take(8 * (size_t)n), o_vals = ar.take(4 * (size_t)n), o_sort = ar.take(sort_bytes);
+    const size_t o_boxes = ar.take(32 * nall);
+    if (want8) ar.bytes = std::max(ar.bytes, (ninner * sizeof(Bvh8Node) + 255) & ~(size_t)255);
+    const size_t o_a = ar.take(4 * (size_t)n), o_b = ar.take(4 * (size_t)n);  // clusters, then emission tasks
+    const size_t o_cost = ar.take(want8 ? 32 * ninner : 0), o_meta = ar.take(want8 ? 16 * ninner : 0);
+    const size_t ploc_tiles = ((size_t)n + (kBB - 2 * kPlocRMax) - 1) / (kBB - 2 * kPlocRMax);
+    const size_t emit_tiles = want8 ? (ninner + kEmitTile - 1) / kEmitTile : 0;
+    const size_t o_zero = ar.take(8 * (ploc_tiles + emit_tiles));
+    const size_t o_st = ar.take(sizeof(BuildStats));
+    unsigned char* tmp = nullptr;
     Bvh2Node* nodes2 = nullptr;
     float4* recs2 = nullptr;
     float4* recs8 = nullptr;
     Bvh8Node* nodes8 = nullptr;
-    const size_t ninner = (size_t)n - 1, nall = 2 * (size_t)n - 1;
-    const size_t sort_bytes = sort_scratch_bytes(n, 63);
-    const uint32_t nb = (n + kScanTile - 1) / kScanTile;
-    Scan scan;
-    uint64_t host_total = 0;
-    uint32_t m = n, next_id = n, iterations = 0;
+    uint32_t status = 0;
+    BuildStats got;
 
 #define WFPT_TRY(x)                      \
     do {                                 \
         if ((e = (x)) != cudaSuccess) goto done; \
     } while (0)
 
-    WFPT_TRY(dalloc(&tlo, n));
-    WFPT_TRY(dalloc(&thi, n));
-    WFPT_TRY(dalloc(&nlo, nall));
-    WFPT_TRY(dalloc(&nhi, nall));
-    WFPT_TRY(dalloc(&keys, n));
-    WFPT_TRY(dalloc(&vals, n));
-    WFPT_TRY(dalloc(&flags, n));
-    WFPT_TRY(dalloc(&excl, n));
-    WFPT_TRY(dalloc(&bsums, nb + 1));
-    WFPT_TRY(dalloc(&total, 1));
-    WFPT_TRY(dalloc(&cl, n));
-    WFPT_TRY(dalloc(&cl2, n));
-    WFPT_TRY(dalloc(&nn, n));
-    WFPT_TRY(dalloc(&parent, nall));
-    WFPT_TRY(dalloc(&kids, ninner));
-    WFPT_TRY(dalloc(&st, 1));
-    WFPT_TRY(dalloc(&sort_scratch, sort_bytes));
-    WFPT_TRY(dalloc(&nodes2, ninner));
-    WFPT_TRY(dalloc(&recs2, 3 * (size_t)n));
-    scan.block_sums = bsums;
-    scan.total = total;
-
-    {  // stage 1: bounds
+    WFPT_TRY(dev_malloc(reinterpret_cast<void**>(&tmp), ar.bytes));
+    WFPT_TRY(dev_malloc(reinterpret_cast<void**>(&nodes2), ninner * sizeof(Bvh2Node)));
+    WFPT_TRY(dev_malloc(reinterpret_cast<void**>(&recs2), (size_t)n * sizeof(TriRec)));
+    if (want8) WFPT_TRY(dev_malloc(reinterpret_cast<void**>(&recs8), (size_t)n * sizeof(TriRec)));
+    {
+        uint64_t* keys = reinterpret_cast<uint64_t*>(tmp + o_keys);
+        uint32_t* vals = reinterpret_cast<uint32_t*>(tmp + o_vals);
+        float4* boxes = reinterpret_cast<float4*>(tmp + o_boxes);
+        uint32_t* ids_a = reinterpret_cast<uint32_t*>(tmp + o_a);
+        uint32_t* ids_b = reinterpret_cast<uint32_t*>(tmp + o_b);
+        float4* cost = reinterpret_cast<float4*>(tmp + o_cost);
+        uint4* meta = reinterpret_cast<uint4*>(tmp + o_meta);
+        unsigned long long* ploc_state = reinterpret_cast<unsigned long long*>(tmp + o_zero);
+        unsigned long long* emit_state = ploc_state + ploc_tiles;
+        BuildStats* st = reinterpret_cast<BuildStats*>(tmp + o_st);
+        // stage 1: bounds
         BuildStats init;
-        for (int k = 0; k < 3; ++k) {
-            init.bmin[k] = init.cmin[k] = kNone;
-            init.bmax[k] = init.cmax[k] = 0;
-        }
-        init.pmax = 0;
-        init.bad_index = 0;
+        std::memset(&init, 0, sizeof(init));
+        for (int k = 0; k < 3; ++k) init.bmin[k] = init.cmin[k] = kNone;
         WFPT_TRY(cudaMemcpyAsync(st, &init, sizeof(init), cudaMemcpyHostToDevice, s));
-        k_tri_bounds<<<blocks(n), kBB, 0, s>>>(positions_dev, num_vertices, indices_dev, n, tlo, thi, st);
-        count_launch();
+        WFPT_TRY(cudaMemsetAsync(ploc_state, 0, 8 * (ploc_tiles + emit_tiles), s));
+        k_tri_bounds<<<blocks(n), kBB, 0, s>>>(positions_dev, num_vertices, indices_dev, n, st);
+        // stage 2: keys, sort, leaves
+        k_centroid_keys<<<blocks(n), kBB, 0, s>>>(positions_dev, num_vertices, indices_dev, n, st, keys, vals);
         WFPT_TRY(cudaGetLastError());
-        BuildStats got;
+        WFPT_TRY(launch_sort_pairs(keys, vals, n, nullptr, 63, tmp + o_sort, sort_bytes, s));
+        k_leaves<<<blocks(n), kBB, 0, s>>>(vals, n, positions_dev, num_vertices, indices_dev, geom_first_dev,
+                                           num_geoms, boxes, recs2, ids_a);
+        count_launch(3);
+        WFPT_TRY(cudaGetLastError());
+        // stage 3: clusters, BVH2, collapse tables
+        const float tri_cost = (float)get_bvh8_tri_cost_pct() * 0.01f;
+        const uint64_t tile = (uint64_t)(kBB - 2 * radius);
+        WFPT_TRY(launch_resident(k_ploc, ((uint64_t)n + tile - 1) / tile, s, ids_a, ids_b, n, radius, boxes,
+                                 reinterpret_cast<float4*>(nodes2), cost, meta, want8 ? 1 : 0, tri_cost, ploc_state,
+                                 st));
+        // stage 4: BVH8
+        if (want8)
+            WFPT_TRY(launch_resident(k_emit8, (uint64_t)emit_tiles, s, ids_a, ids_b, n, (const Bvh2Node*)nodes2,
+                                     (const uint4*)meta, (const float4*)recs2, reinterpret_cast<float4*>(tmp), recs8,
+                                     emit_state, st));
         WFPT_TRY(cudaMemcpyAsync(&got, st, sizeof(got), cudaMemcpyDeviceToHost, s));
         WFPT_TRY(cudaStreamSynchronize(s));
-        if (got.bad_index) {
-            e = cudaErrorInvalidValue;
-            goto done;
-        }
-        for (int k = 0; k < 3; ++k) {
-            const uint32_t lo = (got.bmin[k] & 0x80000000u) ? (got.bmin[k] & 0x7FFFFFFFu) : ~got.bmin[k];
-            const uint32_t hi = (got.bmax[k] & 0x80000000u) ? (got.bmax[k] & 0x7FFFFFFFu) : ~got.bmax[k];
-            std::memcpy(&out->bounds_min[k], &lo, 4);
-            std::memcpy(&out->bounds_max[k], &hi, 4);
-        }
     }
-    // stage 2: keys, sort, leaves
-    k_centroid_keys<<<blocks(n), kBB, 0, s>>>(tlo, thi, n, st, keys, vals);
-    count_launch();
-    WFPT_TRY(cudaGetLastError());
-    WFPT_TRY(launch_sort_pairs(keys, vals, n, nullptr, 63, sort_scratch, sort_bytes, s));
-    k_leaves<<<blocks(n), kBB, 0, s>>>(vals, n, tlo, thi, positions_dev, num_vertices, indices_dev, geom_first_dev,
-                                       num_geoms, nlo, nhi, recs2, cl);
-    count_launch();
-    WFPT_TRY(cudaGetLastError());
-    WFPT_TRY(cudaMemsetAsync(parent, 0xFF, nall * sizeof(uint32_t), s));
-    // stage 3: PLOC until one cluster is left (each pass merges at least one
-    // pair, so n passes bound the loop).
-    while (m > 1) {
-        if (++iterations > n) {
-            e = cudaErrorUnknown;
-            goto done;
-        }
-        k_ploc_nn<<<blocks(m), kBB, 0, s>>>(cl, m, nlo, nhi, nn, g_ploc_radius);
-        k_ploc_flags<<<blocks(m), kBB, 0, s>>>(nn, m, flags);
-        count_launch();
-        count_launch();
-        WFPT_TRY(cudaGetLastError());
-        WFPT_TRY(exclusive_scan(flags, excl, m, scan, s));
-        k_ploc_merge<<<blocks(m), kBB, 0, s>>>(cl, nn, m, excl, next_id, n, (uint32_t)nall, nlo, nhi, kids, parent,
-                                               cl2);
-        count_launch();
-        WFPT_TRY(cudaGetLastError());
-        WFPT_TRY(cudaMemcpyAsync(&host_total, total, sizeof(host_total), cudaMemcpyDeviceToHost, s));
-        WFPT_TRY(cudaStreamSynchronize(s));
-        const uint32_t merges = (uint32_t)(host_total >> 32), kept = (uint32_t)host_total;
-        if (merges == 0 || kept >= m) {
-            e = cudaErrorUnknown;  // no progress: cannot happen (see k_ploc_nn)
-            goto done;
-        }
-        next_id += merges;
-        m = kept;
-        std::swap(cl, cl2);
+    if (got.bad_index) {
+        e = cudaErrorInvalidValue;
+        goto done;
     }
-    if (next_id != nall) {
+    WFPT_TRY(status_build(&status));
+    if (status || got.stuck || got.clusters != 1 || got.next_id != nall || (want8 && got.tris8 != n) ||
+        (want8 && (got.nodes8 == 0 || got.nodes8 > ninner))) {
         e = cudaErrorUnknown;
         goto done;
     }
-    out->ploc_iterations = iterations;
-    // stage 4: BVH2 in the traversal format
-    k_write_bvh2<<<blocks(ninner), kBB, 0, s>>>(n, kids, nlo, nhi, st, nodes2);
-    count_launch();
-    WFPT_TRY(cudaGetLastError());
-    // stage 5: BVH8
-    if (want8) {
-        WFPT_TRY(dalloc(&cost, 8 * ninner));
-        WFPT_TRY(dalloc(&how, 8 * ninner));
-        WFPT_TRY(dalloc(&split8, ninner));
-        WFPT_TRY(dalloc(&ntris, ninner));
-        WFPT_TRY(dalloc(&visits, ninner));
-        WFPT_TRY(dalloc(&tasks, ninner));
-        WFPT_TRY(dalloc(&tasks2, ninner));
-        WFPT_TRY(dalloc(&nodes8_tmp, ninner));
-        WFPT_TRY(dalloc(&recs8, 3 * (size_t)n));
-        WFPT_TRY(cudaMemsetAsync(visits, 0, ninner * sizeof(uint32_t), s));
-        k_collapse_dp<<<blocks(n), kBB, 0, s>>>(n, nodes2, parent, visits, cost, how, split8, ntris,
-                                                (float)get_bvh8_tri_cost_pct() * 0.01f);
-        count_launch();
-        WFPT_TRY(cudaGetLastError());
-        uint2 root = make_uint2(0u, 0u);
-        WFPT_TRY(cudaMemcpyAsync(tasks, &root, sizeof(root), cudaMemcpyHostToDevice, s));
-        uint32_t ntasks = 1, node_count = 1, tri_count = 0;
-        for (int level = 0; ntasks > 0; ++level) {
-            if (level > 64 || ntasks > ninner) {
-                e = cudaErrorUnknown;
-                goto done;
-            }
-            k_emit_count<<<blocks(ntasks), kBB, 0, s>>>(tasks, ntasks, nodes2, how, split8, ntris, flags);
-            count_launch();
-            WFPT_TRY(cudaGetLastError());
-            WFPT_TRY(exclusive_scan(flags, excl, ntasks, scan, s));
-            k_emit_write<<<blocks(ntasks), kBB, 0, s>>>(tasks, ntasks, excl, node_count, tri_count,
-                                                        (uint32_t)ninner, n, nodes2, how, split8, ntris, recs2,
-                                                        nodes8_tmp, recs8, tasks2);
-            count_launch();
-            WFPT_TRY(cudaGetLastError());
-            WFPT_TRY(cudaMemcpyAsync(&host_total, total, sizeof(host_total), cudaMemcpyDeviceToHost, s));
-            WFPT_TRY(cudaStreamSynchronize(s));
-            const uint32_t inner = (uint32_t)(host_total >> 32), tris = (uint32_t)host_total;
-            node_count += inner;
-            tri_count += tris;
-            ntasks = inner;
-            std::swap(tasks, tasks2);
-            if (node_count > ninner || tri_count > n) {
-                e = cudaErrorUnknown;
-                goto done;
-            }
-        }
-        if (tri_count != n) {
-            e = cudaErrorUnknown;
-            goto done;
-        }
-        WFPT_TRY(dalloc(&nodes8, node_count));
-        WFPT_TRY(cudaMemcpyAsync(nodes8, nodes8_tmp, node_count * sizeof(Bvh8Node), cudaMemcpyDeviceToDevice, s));
-        out->bvh8_count = node_count;
+    out->ploc_iterations = got.iterations;
+    for (int k = 0; k < 3; ++k) {
+        const uint32_t lo = (got.bmin[k] & 0x80000000u) ? (got.bmin[k] & 0x7FFFFFFFu) : ~got.bmin[k];
+        const uint32_t hi = (got.bmax[k] & 0x80000000u) ? (got.bmax[k] & 0x7FFFFFFFu) : ~got.bmax[k];
+        std::memcpy(&out->bounds_min[k], &lo, 4);
+        std::memcpy(&out->bounds_max[k], &hi, 4);
     }
-    WFPT_TRY(cudaStreamSynchronize(s));
-    {
-        uint32_t flags_h = 0;
-        WFPT_TRY(status_build(&flags_h));
-        if (flags_h) {
-            e = cudaErrorUnknown;
-            goto done;
-        }
+    if (want8) {
+        WFPT_TRY(dev_malloc(reinterpret_cast<void**>(&nodes8), got.nodes8 * sizeof(Bvh8Node)));
+        WFPT_TRY(cudaMemcpyAsync(nodes8, tmp, got.nodes8 * sizeof(Bvh8Node), cudaMemcpyDeviceToDevice, s));
+        WFPT_TRY(cudaStreamSynchronize(s));
+        out->bvh8_count = got.nodes8;
     }
     out->bvh2_nodes = nodes2;
     out->bvh2_tris = recs2;
@@ -948,11 +977,7 @@ cudaError_t build_scene_device(const float* positions_dev, uint32_t num_vertices
     recs8 = nullptr;
 #undef WFPT_TRY
 done:
-    for (void* p : {(void*)tlo, (void*)thi, (void*)nlo, (void*)nhi, (void*)keys, (void*)flags, (void*)excl,
-                    (void*)bsums, (void*)total, (void*)vals, (void*)cl, (void*)cl2, (void*)nn, (void*)parent,
-                    (void*)kids, (void*)st, (void*)sort_scratch, (void*)cost, (void*)how, (void*)split8,
-                    (void*)ntris, (void*)visits, (void*)tasks, (void*)tasks2, (void*)nodes8_tmp, (void*)nodes2,
-                    (void*)recs2, (void*)recs8, (void*)nodes8})
+    for (void* p : {(void*)tmp, (void*)nodes2, (void*)recs2, (void*)recs8, (void*)nodes8})
         if (p) cudaFree(p);
     return e;
 }
