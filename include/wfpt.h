@@ -120,7 +120,7 @@ uint64_t wfpt_kernel_launch_count(void);
 /* Process-wide tuning knobs (no counterpart in the reference; set by the
  * autotuner).  Keys:
  *   "trace.bvh8.refill"    refill a persistent warp when this many lanes
- *                          are idle (1..32, default 8)
+ *                          are idle (1..32, default 6)
  *   "trace.bvh8.postpone"  per-lane triangle tests (coop 0): postpone a
  *                          node's triangle tests while fewer than this many
  *                          lanes have triangles (0..32, 0 = off)
@@ -130,14 +130,16 @@ uint64_t wfpt_kernel_launch_count(void);
  *                          identical; an any-hit ray may report a different
  *                          (equally valid) occluder
  *   "trace.bvh8.batch"     cooperative tests of closest-hit rays: run them
- *                          once this many are pending across the warp's
+ *                          once half this many are pending across the warp's
  *                          node steps (1..32, default 24; 1 = after every
  *                          loop iteration)
- *   "trace.bvh8.steps"     cooperative tests of closest-hit rays: node steps
- *                          a lane takes per loop iteration while its steps
- *                          hand it no triangles (1..8, default 2)
+ *   "trace.bvh8.steps"     cooperative tests of closest-hit rays: a loop
+ *                          iteration takes up to twice this many node steps
+ *                          per lane, each lane until a second node has
+ *                          handed it triangles (1..8, default 2)
  *   "trace.bvh8.any_batch" the same for any-hit rays (default 1)
- *   "trace.bvh8.any_steps" the same for any-hit rays (default 3)
+ *   "trace.bvh8.any_steps" the same for any-hit rays, two node steps more
+ *                          (default 3: up to eight)
  *   "sort.tiles"           radix sort tile size: 0 = by problem size
  *                          (default), 1 = small tiles, 2 = large tiles,
  *                          3 = extra-large tiles (32-bit keys; 64-bit keys

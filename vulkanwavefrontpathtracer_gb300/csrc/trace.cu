@@ -545,6 +545,13 @@ __device__ __forceinline__ unsigned long long hit_key(float t, uint32_t key) {
     return ((unsigned long long)b << 32) | key;
 }
 
+// Any-hit order: pairs of the first group that a loop iteration handed the
+// lane before those of the second, then the closest-hit order (triangle
+// indices are below 2^27).
+__device__ __forceinline__ unsigned long long any_key(float t, uint32_t key, bool second) {
+    return ((unsigned long long)second << 60) | ((hit_key(t, 0u) >> 32) << 28) | key;
+}
+
 __device__ __forceinline__ float hit_key_t(unsigned long long k) {
     uint32_t b = (uint32_t)(k >> 32);
     b = (b & 0x80000000u) ? (b ^ 0x80000000u) : ~b;
@@ -561,20 +568,39 @@ constexpr int kRing = 1024;        // per-warp ring of pending triangle tests (p
 // the test whose key is the owner's best after its round stores the hit's
 // primitive, geometry, barycentrics and t beside it, so a finished lane
 // writes its RayResult from shared memory (no reload of the winning
-// triangle at write-out: 2 % faster any hit).  Tests are batched across node steps: the ring is tested once `batch` or
-// more pairs are pending (in whole passes of 32 when 32 or more are), and
-// entirely once the lanes waiting on their own tests plus the idle lanes
-// would fill a refill, or no lane has nodes left.  A loop iteration takes up
-// to `steps` node steps per lane, stopping at the first node that hands the
-// lane triangles, so the per-iteration work (refill check, votes, scan,
-// test decision) is shared by several node steps.  A lane's ray finishes
-// only when its traversal is exhausted (any hit: when it has a hit) and all
-// of its own tests have run, so a ring entry never outlives its ray.  The
-// deferred tests leave tcur larger for a few node steps (culling stays
-// conservative: tcur only shrinks), which costs about 1 % more node steps
-// and saves most of the partly empty test passes (batch 1: test every
-// step).  A lane appends at most one node's 24 triangles per iteration, so
-// at most 31 + 32 * 24 pairs are pending after an append.
+// triangle at write-out: 2 % faster any hit).  Tests are batched across node
+// steps: the ring is tested once `batch` or more pairs are pending (in whole
+// passes of 32 when 32 or more are), and entirely once the lanes waiting on
+// their own tests plus the idle lanes would fill a refill, or no lane has
+// nodes left.  A loop iteration takes up to `steps` node steps per lane, so
+// the per-iteration work (refill check, votes, scan, test decision) is shared
+// by several node steps.  A lane's ray finishes only when its traversal is
+// exhausted (any hit: when it has a hit) and all of its own tests have run,
+// so a ring entry never outlives its ray.  The deferred tests leave tcur
+// larger for a few node steps (culling stays conservative: tcur only
+// shrinks), which costs about 1 % more node steps and saves most of the
+// partly empty test passes (batch 1: test every step).
+//
+// The node steps of an iteration are where lanes sit idle, and they are half
+// of the time: a lane that stopped at its first triangles waited for the rest
+// of the iteration, so more than two (any hit: three) steps did not pay.  A
+// lane now goes on with its triangles in hand until a second node hands it
+// some (or the first handed it more than kMoreTris), and four steps do:
+// closest hit 1070 -> 1003 us (courtyard, 2.07M sorted bounce-1 rays), 502 ->
+// 467 us (city, 1.6M), 122 -> 104 us (57K rays of the 65K soup); any hit
+// 1286 -> 1221, 393 -> 361 and 119 -> 109 us.  A closest-hit iteration asks
+// once, before its third step, whether any lane goes on (a vote per step cost
+// 0.3 %, none 0.6 %).  An any-hit iteration ends as soon as fewer than
+// kFewLanes lanes go on while there are rays to refill with: its rays are
+// short, and an early end brings the refill forward (city 392 -> 361 us
+// against steps taken to the end; a share of the tracing lanes instead of a
+// number 396-421, 16 or 22 lanes 362-363, 18 lanes and six steps 375).
+// A lane appends at most kMoreTris + 24 triangles per iteration, so at most
+// 31 + 32 * 31 pairs are pending after an append: they fit the ring.
+constexpr uint32_t kMoreTris = 7;
+constexpr uint32_t kFewLanes = 20;
+static_assert(31 + 32 * (kMoreTris + 24) <= kRing, "the ring holds every pending pair");
+
 template <bool CLOSEST, bool COUNT>
 __global__ void __launch_bounds__(kBlock, 4) k_trace_bvh8_coop(
     const float4* __restrict__ nodes, const float4* __restrict__ tris, const float4* __restrict__ rays,
@@ -585,6 +611,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_trace_bvh8_coop(
     __shared__ unsigned long long s_best[kBlock];
     __shared__ uint4 s_hit[kBlock];  // winning hit: primId, geomId, packed barycentrics, t
     __shared__ uint32_t s_task[kBlock / 32][kRing];
+    __shared__ float s_tmax[CLOSEST ? 1 : kBlock];       // any hit: the ray's tmax
+    __shared__ uint32_t s_second[CLOSEST ? 1 : kBlock];  // any hit: where the lane's second group starts in the ring
     const uint32_t count = load_count(n, n_dev);
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t lt_mask = (1u << lane) - 1u;
@@ -611,7 +639,7 @@ __global__ void __launch_bounds__(kBlock, 4) k_trace_bvh8_coop(
         if (want_mask != 0u && (__popc(want_mask) >= refill || busy_mask == 0u)) {
             if (state == kDone) {
                 const unsigned long long best = s_best[threadIdx.x];
-                if ((uint32_t)best == 0xFFFFFFFFu) {
+                if (CLOSEST ? (uint32_t)best == 0xFFFFFFFFu : best == ~0ull) {
                     write_miss(results, ri);
                 } else {
                     const uint4 hh = s_hit[threadIdx.x];
@@ -636,7 +664,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_trace_bvh8_coop(
                         state = kTracing;
                         r = setup_ray(r0, r1);
                         s_ray[threadIdx.x] = ray_shared(r);
-                        s_best[threadIdx.x] = hit_key(r1.w, 0xFFFFFFFFu);
+                        s_best[threadIdx.x] = CLOSEST ? hit_key(r1.w, 0xFFFFFFFFu) : ~0ull;
+                        if (!CLOSEST) s_tmax[threadIdx.x] = r1.w;
                         tcur = r1.w;
                         sp = 0;
                         ng = make_uint2(0u, 0x80000000u);
@@ -650,12 +679,14 @@ __global__ void __launch_bounds__(kBlock, 4) k_trace_bvh8_coop(
         if (__ballot_sync(0xffffffffu, state != kIdle || !exhausted) == 0u) break;
         if (COUNT && lane == 0) ++c_iters;
 
-        // Up to `steps` node steps; a lane stops stepping at the first node
-        // that hands it triangles (at most one group of 24 per iteration).
-        uint32_t tri_base = 0, tg = 0;
+        // Up to `steps` node steps, with up to two groups of triangles.
+        uint32_t tri_base = 0, tg = 0, tri_base2 = 0, tg2 = 0;
+        const uint32_t few = CLOSEST ? 0u : (__any_sync(0xffffffffu, exhausted) ? 1u : kFewLanes);
         for (uint32_t st = 0; st < steps; ++st) {
-            const bool go = state == kTracing && ng.y > 0x00FFFFFFu && tg == 0u;
-            if (st != 0u && !__any_sync(0xffffffffu, go)) break;
+            const bool go = state == kTracing && ng.y > 0x00FFFFFFu && tg2 == 0u && __popc(tg) <= kMoreTris;
+            if (CLOSEST ? (st == 2u && !__any_sync(0xffffffffu, go))
+                        : (st >= 1u && (uint32_t)__popc(__ballot_sync(0xffffffffu, go)) < few))
+                break;
             if (go) {
                 uint32_t bit = 31u - __clz(ng.y);
                 ng.y &= ~(1u << bit);
@@ -668,17 +699,23 @@ __global__ void __launch_bounds__(kBlock, 4) k_trace_bvh8_coop(
                         raise_status(kErrBounds);
                     }
                 }
-                uint32_t child_base, imask;
+                uint32_t child_base, imask, tb;
                 if (COUNT) ++c_nodes;
-                uint32_t hitmask = intersect_node8(nodes + 5 * (size_t)node, r, tcur, child_base, tri_base, imask);
+                uint32_t hitmask = intersect_node8(nodes + 5 * (size_t)node, r, tcur, child_base, tb, imask);
                 ng = make_uint2(child_base, (hitmask & 0xFF000000u) | imask);
-                tg = hitmask & 0x00FFFFFFu;
+                if (tg == 0u) {
+                    tg = hitmask & 0x00FFFFFFu;
+                    tri_base = tb;
+                } else {
+                    tg2 = hitmask & 0x00FFFFFFu;
+                    tri_base2 = tb;
+                }
             }
             if (state == kTracing && ng.y <= 0x00FFFFFFu && sp > 0) ng = stack[--sp];
         }
 
         // Append this step's pairs: exclusive scan of the per-lane counts.
-        const uint32_t cnt = __popc(tg);
+        const uint32_t cnt = __popc(tg) + __popc(tg2);
         uint32_t incl = cnt;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
@@ -689,10 +726,16 @@ __global__ void __launch_bounds__(kBlock, 4) k_trace_bvh8_coop(
         if (cnt != 0u) {
             uint32_t pos = appended + incl - cnt;
             const uint32_t owner = lane << kRecBits;
+            if (!CLOSEST) s_second[threadIdx.x] = pos + __popc(tg);
             while (tg != 0u) {
                 uint32_t tb = __ffs(tg) - 1u;
                 tg &= tg - 1u;
                 task[pos++ & (kRing - 1)] = owner | (tri_base + tb);
+                if (tg == 0u) {
+                    tg = tg2;
+                    tri_base = tri_base2;
+                    tg2 = 0u;
+                }
             }
             my_end = pos;
             if (COUNT) c_tris += cnt;
@@ -730,10 +773,11 @@ __global__ void __launch_bounds__(kBlock, 4) k_trace_bvh8_coop(
                     Uvw q = tri_uvw(rs, a4, b4, c4);
                     if (q.edge_ok && q.det != 0.0f) {
                         float t = __fdiv_rn(q.T, q.det);
-                        if (t >= rs.tmin) {
+                        if (t >= rs.tmin && (CLOSEST || t <= s_tmax[o])) {
                             // A stale read can only be larger than the current
                             // best, so skipping on it is safe.
-                            hk = hit_key(t, __float_as_uint(c4.w));
+                            hk = CLOSEST ? hit_key(t, __float_as_uint(c4.w))
+                                         : any_key(t, __float_as_uint(c4.w), (int32_t)(tested + j - s_second[o]) >= 0);
                             if (hk < s_best[o]) {
                                 atomicMin(&s_best[o], hk);
                                 cand = true;
@@ -755,9 +799,9 @@ __global__ void __launch_bounds__(kBlock, 4) k_trace_bvh8_coop(
 
         if (state == kTracing) {
             const unsigned long long best = s_best[threadIdx.x];
-            tcur = hit_key_t(best);
+            if (CLOSEST) tcur = hit_key_t(best);
             bool stop = waiting;
-            if (!CLOSEST && (uint32_t)best != 0xFFFFFFFFu) {
+            if (!CLOSEST && best != ~0ull) {
                 stop = true;  // any hit: no more node steps
                 ng.y = 0u;
                 sp = 0;
@@ -787,20 +831,32 @@ static std::atomic<uint32_t> g_slot{0};
 // for the cooperative one.
 static int g_blocks_per_sm[4] = {0, 0, 0, 0};
 static int g_num_sms = 0;
-static uint32_t g_refill = 8;
+static uint32_t g_refill = 6;  // 4 to 8 within 1 % on bounce-1 rays, 6 the best sum
 
 void set_trace_refill(uint32_t refill) { g_refill = refill < 1 ? 1 : (refill > 32 ? 32 : refill); }
 static uint32_t g_postpone = 0;
 void set_trace_postpone(uint32_t lanes) { g_postpone = lanes > 32 ? 32 : lanes; }
 // Cooperative-test batch and node steps per loop iteration, [0] for any-hit
-// rays, [1] for closest-hit rays.  Any-hit rays test their triangles after
-// every iteration of three node steps (a ray stops at its first hit, so
-// deferring tests only adds node steps), closest-hit rays batch 24 pairs
-// over iterations of two steps: measured on the courtyard's bounce-1 rays
-// (1.4 % / 0.6 % faster than the shared batch 16, steps 2) and its frames
-// (25.28 against 25.38 ms).
+// rays, [1] for closest-hit rays.  The kernel takes twice the steps, since a
+// lane goes on past its first triangles (any hit two more: its iterations
+// end early by themselves), and tests once half the batch is pending.  So
+// any-hit rays test after every iteration of up to eight node steps (a ray
+// stops at its first hit: deferring tests only adds node steps, 1-3 % slower
+// from batch 8 on), closest-hit rays at 12 pairs over iterations of four
+// (3, 5, 6 and 8 steps: 1.5, 0.5, 1 and 5 % slower on the courtyard's sorted
+// bounce-1 rays; 16 pairs equal there, 1 % slower on the city's and 4 % on a
+// 57K-ray wavefront).
 static uint32_t g_batch[2] = {1, 24};
 static uint32_t g_steps[2] = {3, 2};
+static uint32_t kernel_batch(bool closest) { return (g_batch[closest ? 1 : 0] + 1) / 2; }
+// lanes: rays that the grid holds at once.  A wavefront that fits has no
+// refills, so its any-hit iterations don't end early: four steps (57K soup
+// rays: 109 us, 114 with eight).
+static uint32_t kernel_steps(bool closest, uint32_t n, uint32_t lanes) {
+    if (closest) return 2 * g_steps[1];
+    const uint32_t steps = 2 * g_steps[0] + 2;
+    return n <= lanes && steps > 4 ? 4 : steps;
+}
 void set_trace_steps(uint32_t steps, bool closest) {
     g_steps[closest ? 1 : 0] = steps < 1 ? 1 : (steps > 8 ? 8 : steps);
 }
@@ -870,13 +926,14 @@ cudaError_t launch_trace(const SceneDevice& sc, int kind, const wfpt_ray* rays, 
         const bool coop = g_coop && sc.bvh8_num_tris < (1u << kRecBits);
         unsigned pgrid = (unsigned)(g_num_sms * g_blocks_per_sm[(coop ? 2 : 0) + (closest ? 1 : 0)]);
         if (pgrid == 0) pgrid = 1;
+        const uint32_t lanes = pgrid * kBlock;
         if (grid < pgrid) pgrid = grid;
         uint32_t* work = own_work ? own_work : sc.work + 16 * (g_slot.fetch_add(1) % kWorkSlots);
         if (coop) {
             auto k8 = closest ? (g_count ? k_trace_bvh8_coop<true, true> : k_trace_bvh8_coop<true, false>)
                               : (g_count ? k_trace_bvh8_coop<false, true> : k_trace_bvh8_coop<false, false>);
             k8<<<pgrid, kBlock, 0, s>>>(sc.bvh8_nodes, sc.bvh8_tris, rr, out, ray_index, n, n_dev, work, g_refill,
-                                        g_batch[closest ? 1 : 0], g_steps[closest ? 1 : 0]);
+                                        kernel_batch(closest != 0), kernel_steps(closest != 0, n, lanes));
         } else {
             auto k8 = closest ? (g_count ? k_trace_bvh8<true, true> : k_trace_bvh8<true, false>)
                               : (g_count ? k_trace_bvh8<false, true> : k_trace_bvh8<false, false>);
