@@ -192,8 +192,31 @@ __device__ __forceinline__ void box2(const RayT& r, float lox, float hix, float 
     hit = tn <= tf * kBoxSlack;
 }
 
-template <bool CLOSEST, bool COUNT>
-__global__ void __launch_bounds__(kBlock) k_trace_bvh2(const float4* __restrict__ nodes,
+// 32 bytes in one load (256-bit loads, sm_100 and later).
+__device__ __forceinline__ void load32(const float4* p, float4& a, float4& b) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+        : "l"(p));
+}
+
+// One thread per ray.  Incoherent rays keep 6 to 9 lanes of a warp busy, and
+// the kernel waits on its node loads: 66 dependent 64-byte nodes a ray through
+// an L1 that is 60 % busy.  So a node is two 256-bit loads instead of four
+// 128-bit ones (L1 requests, and with them its busy cycles, fall by a third:
+// 2-4 % faster), and wavefronts that fill the GPU run as blocks of two warps
+// with registers capped at 51 (20 blocks per SM): a block's registers wait
+// for its longest ray, so small blocks keep more warps in flight than
+// 256-thread ones.  Closest hit 1773 -> 1648 us (courtyard, 2.07M bounce-1
+// rays), 456 -> 423 us (city, 1.6M), camera rays 671 -> 632 and 257 -> 239 us,
+// any hit 1679 -> 1569 and 413 -> 387 us; 64 threads without the cap 3-4 %
+// slower, with 24 blocks 5-10 %.  Wavefronts below half of the 194,560
+// resident rays of that shape gain nothing from it and want the registers
+// (57K rays: 161 us in 256-thread blocks, 176 us in small ones; 120K: 186 and
+// 173).
+constexpr int kBvh2SmallBlock = 64, kBvh2SmallPerSm = 20;
+constexpr uint32_t kBvh2SmallMin = 152 * kBvh2SmallPerSm * kBvh2SmallBlock / 2;
+template <bool CLOSEST, bool COUNT, int BLOCK, int PER_SM>
+__global__ void __launch_bounds__(BLOCK, PER_SM) k_trace_bvh2(const float4* __restrict__ nodes,
                                                        const float4* __restrict__ tris,
                                                        const float4* __restrict__ rays, int4* __restrict__ results,
                                                        const uint32_t* __restrict__ ray_index, uint32_t n,
@@ -219,10 +242,10 @@ __global__ void __launch_bounds__(kBlock) k_trace_bvh2(const float4* __restrict_
         // Inner nodes.
         while (node >= 0) {
             if (COUNT) ++c_nodes;
-            float4 a = __ldg(&nodes[4 * node + 0]);
-            float4 b = __ldg(&nodes[4 * node + 1]);
-            float4 c = __ldg(&nodes[4 * node + 2]);
-            int4 l = __ldg(reinterpret_cast<const int4*>(&nodes[4 * node + 3]));
+            float4 a, b, c, lf;
+            load32(nodes + 4 * (size_t)node, a, b);
+            load32(nodes + 4 * (size_t)node + 2, c, lf);
+            const int2 l = make_int2(__float_as_int(lf.x), __float_as_int(lf.y));
             float t0, t1;
             bool h0, h1;
             box2(r, a.x, a.y, a.z, a.w, c.x, c.y, h.t, t0, h0);
@@ -941,9 +964,16 @@ cudaError_t launch_trace(const SceneDevice& sc, int kind, const wfpt_ray* rays, 
                                         g_postpone);
         }
     } else {
-        auto k2 = closest ? (g_count ? k_trace_bvh2<true, true> : k_trace_bvh2<true, false>)
-                          : (g_count ? k_trace_bvh2<false, true> : k_trace_bvh2<false, false>);
-        k2<<<grid, kBlock, 0, s>>>(sc.bvh2_nodes, sc.bvh2_tris, rr, out, ray_index, n, n_dev);
+        if (n >= kBvh2SmallMin) {
+            constexpr int B = kBvh2SmallBlock, P = kBvh2SmallPerSm;
+            auto k2 = closest ? (g_count ? k_trace_bvh2<true, true, B, P> : k_trace_bvh2<true, false, B, P>)
+                              : (g_count ? k_trace_bvh2<false, true, B, P> : k_trace_bvh2<false, false, B, P>);
+            k2<<<(n + B - 1) / B, B, 0, s>>>(sc.bvh2_nodes, sc.bvh2_tris, rr, out, ray_index, n, n_dev);
+        } else {
+            auto k2 = closest ? (g_count ? k_trace_bvh2<true, true, kBlock, 1> : k_trace_bvh2<true, false, kBlock, 1>)
+                              : (g_count ? k_trace_bvh2<false, true, kBlock, 1> : k_trace_bvh2<false, false, kBlock, 1>);
+            k2<<<grid, kBlock, 0, s>>>(sc.bvh2_nodes, sc.bvh2_tris, rr, out, ray_index, n, n_dev);
+        }
     }
     count_launch();
     return cudaGetLastError();
