@@ -15,6 +15,7 @@
 // (JCGT 2013), evaluated without FMA contraction, and the same closest-hit
 // rule (smallest t, ties to the smaller global triangle index), so both
 // forms return identical hits.
+#include <algorithm>
 #include <atomic>
 
 #include "common.cuh"
@@ -199,31 +200,11 @@ __device__ __forceinline__ void load32(const float4* p, float4& a, float4& b) {
         : "l"(p));
 }
 
-// One thread per ray.  Incoherent rays keep 6 to 9 lanes of a warp busy, and
-// the kernel waits on its node loads: 66 dependent 64-byte nodes a ray through
-// an L1 that is 60 % busy.  So a node is two 256-bit loads instead of four
-// 128-bit ones (L1 requests, and with them its busy cycles, fall by a third:
-// 2-4 % faster), and wavefronts that fill the GPU run as blocks of two warps
-// with registers capped at 51 (20 blocks per SM): a block's registers wait
-// for its longest ray, so small blocks keep more warps in flight than
-// 256-thread ones.  Closest hit 1773 -> 1648 us (courtyard, 2.07M bounce-1
-// rays), 456 -> 423 us (city, 1.6M), camera rays 671 -> 632 and 257 -> 239 us,
-// any hit 1679 -> 1569 and 413 -> 387 us; 64 threads without the cap 3-4 %
-// slower, with 24 blocks 5-10 %.  Wavefronts below half of the 194,560
-// resident rays of that shape gain nothing from it and want the registers
-// (57K rays: 161 us in 256-thread blocks, 176 us in small ones; 120K: 186 and
-// 173).
-constexpr int kBvh2SmallBlock = 64, kBvh2SmallPerSm = 20;
-constexpr uint32_t kBvh2SmallMin = 152 * kBvh2SmallPerSm * kBvh2SmallBlock / 2;
-template <bool CLOSEST, bool COUNT, int BLOCK, int PER_SM>
-__global__ void __launch_bounds__(BLOCK, PER_SM) k_trace_bvh2(const float4* __restrict__ nodes,
-                                                       const float4* __restrict__ tris,
-                                                       const float4* __restrict__ rays, int4* __restrict__ results,
-                                                       const uint32_t* __restrict__ ray_index, uint32_t n,
-                                                       const uint32_t* __restrict__ n_dev) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= load_count(n, n_dev)) return;
-    uint32_t ri = ray_index ? ray_index[i] : i;
+// One ray, traced by one thread.
+template <bool CLOSEST, bool COUNT>
+__device__ __forceinline__ void trace_bvh2_ray(const float4* __restrict__ nodes, const float4* __restrict__ tris,
+                                               const float4* __restrict__ rays, int4* __restrict__ results,
+                                               uint32_t ri) {
     float4 r0 = rays[2 * ri + 0];
     float4 r1 = rays[2 * ri + 1];
     if (!(r1.w >= r0.w)) {  // tmax < tmin (or NaN): empty interval
@@ -299,6 +280,78 @@ __global__ void __launch_bounds__(BLOCK, PER_SM) k_trace_bvh2(const float4* __re
     }
     write_hit(results, ri, r, tris, h, found);
     if (COUNT) add_counts(c_nodes, c_tris, 1u, 0u);
+}
+
+
+// One thread per ray.  Incoherent rays keep 6 to 9 lanes of a warp busy, and
+// the kernel waits on its node loads: 66 dependent 64-byte nodes a ray through
+// an L1 that is 60 % busy.  So a node is two 256-bit loads instead of four
+// 128-bit ones (L1 requests, and with them its busy cycles, fall by a third:
+// 2-4 % faster), and wavefronts that fill the GPU run as blocks of two warps
+// with registers capped at 51 (20 blocks per SM): a block's registers wait
+// for its longest ray, so small blocks keep more warps in flight than
+// 256-thread ones.  Closest hit 1773 -> 1648 us (courtyard, 2.07M bounce-1
+// rays), 456 -> 423 us (city, 1.6M), camera rays 671 -> 632 and 257 -> 239 us,
+// any hit 1679 -> 1569 and 413 -> 387 us; 64 threads without the cap 3-4 %
+// slower, with 24 blocks 5-10 %.  Wavefronts below half of the 194,560
+// resident rays of that shape gain nothing from it and want the registers
+// (57K rays: 161 us in 256-thread blocks, 176 us in small ones; 120K: 186 and
+// 173).
+constexpr int kBvh2SmallBlock = 64, kBvh2SmallPerSm = 20;
+constexpr uint32_t kBvh2SmallMin = 152 * kBvh2SmallPerSm * kBvh2SmallBlock / 2;
+template <bool CLOSEST, bool COUNT, int BLOCK, int PER_SM>
+__global__ void __launch_bounds__(BLOCK, PER_SM) k_trace_bvh2(const float4* __restrict__ nodes,
+                                                              const float4* __restrict__ tris,
+                                                              const float4* __restrict__ rays,
+                                                              int4* __restrict__ results,
+                                                              const uint32_t* __restrict__ ray_index, uint32_t n,
+                                                              const uint32_t* __restrict__ n_dev) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= load_count(n, n_dev)) return;
+    trace_bvh2_ray<CLOSEST, COUNT>(nodes, tris, rays, results, ray_index ? ray_index[i] : i);
+}
+
+// The same with resident warps that take 32 rays at a time, the first by
+// warp number, the next from work[0]; work[1] counts finished warps, and the
+// last resets both.  For wavefronts whose size only the device knows: a
+// bounce's count is often far below its capacity n, and the launch above pays
+// for every empty block (68 us at n = 8.3M, 133 us for its shadow rays; this
+// one 8 us).  And for very large ones: 6.4M city bounce-1 rays 1464 -> 1388 us
+// closest, 1333 -> 1265 us any hit, 8.3M camera rays 714 -> 702 us.  At full
+// counts in between it is 2-5 % faster on incoherent rays (courtyard closest
+// 1648 -> 1613 us) but 3-20 % slower on camera rays (2.07M: 632 -> 651 us, 262K:
+// 159 -> 192 us), whose sizes the host knows; asking for the next 32 rays
+// before tracing the current ones (which binds them to a warp that may be
+// slow) made those worse still (706 and 239 us).
+constexpr int kBvh2PerSm = 5;
+constexpr unsigned kBvh2Grid = 152 * kBvh2PerSm;
+constexpr uint32_t kBvh2PersistentMin = 1u << 22;  // with a host-side count
+template <bool CLOSEST, bool COUNT>
+__global__ void __launch_bounds__(kBlock, kBvh2PerSm) k_trace_bvh2_persistent(
+    const float4* __restrict__ nodes, const float4* __restrict__ tris, const float4* __restrict__ rays,
+    int4* __restrict__ results, const uint32_t* __restrict__ ray_index, uint32_t n,
+    const uint32_t* __restrict__ n_dev, uint32_t* __restrict__ work) {
+    const uint32_t count = load_count(n, n_dev);
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t warps = gridDim.x * (kBlock / 32);
+    const uint32_t chunks = (count + 31u) / 32u;
+    uint32_t chunk = (blockIdx.x * kBlock + threadIdx.x) >> 5;
+    while (chunk < chunks) {
+        const uint32_t i = chunk * 32u + lane;
+        if (i < count) trace_bvh2_ray<CLOSEST, COUNT>(nodes, tris, rays, results, ray_index ? ray_index[i] : i);
+        uint32_t next = 0;
+        __syncwarp();
+        if (lane == 0) next = atomicAdd(&work[0], 1u);
+        chunk = warps + __shfl_sync(0xffffffffu, next, 0);
+    }
+    if (lane == 0) {
+        __threadfence();
+        if (atomicAdd(&work[1], 1u) == warps - 1u) {
+            work[0] = 0u;
+            work[1] = 0u;
+            __threadfence();
+        }
+    }
 }
 
 // --------------------------------------------------------- BVH8 (chosen)
@@ -964,7 +1017,13 @@ cudaError_t launch_trace(const SceneDevice& sc, int kind, const wfpt_ray* rays, 
                                         g_postpone);
         }
     } else {
-        if (n >= kBvh2SmallMin) {
+        if (n >= (n_dev != nullptr ? kBvh2SmallMin : kBvh2PersistentMin)) {
+            uint32_t* work = own_work ? own_work : sc.work + 16 * (g_slot.fetch_add(1) % kWorkSlots);
+            auto k2 = closest ? (g_count ? k_trace_bvh2_persistent<true, true> : k_trace_bvh2_persistent<true, false>)
+                              : (g_count ? k_trace_bvh2_persistent<false, true> : k_trace_bvh2_persistent<false, false>);
+            k2<<<std::min(grid, kBvh2Grid), kBlock, 0, s>>>(sc.bvh2_nodes, sc.bvh2_tris, rr, out, ray_index, n, n_dev,
+                                                            work);
+        } else if (n >= kBvh2SmallMin) {
             constexpr int B = kBvh2SmallBlock, P = kBvh2SmallPerSm;
             auto k2 = closest ? (g_count ? k_trace_bvh2<true, true, B, P> : k_trace_bvh2<true, false, B, P>)
                               : (g_count ? k_trace_bvh2<false, true, B, P> : k_trace_bvh2<false, false, B, P>);
