@@ -116,6 +116,7 @@ struct wfpt_renderer {
     const wfpt_geometry* geoms = nullptr;
     float smin[3] = {0, 0, 0}, smax[3] = {0, 0, 0}, light[3] = {5, -2, 1}, bg[3] = {0, 0, 1};
     int frame_index = 1;
+    bool gpu_shared = false;  // one of a batch's requests that run side by side
 
     int width = 0, height = 0;
     int alloc_samples = 0;
@@ -464,7 +465,7 @@ struct wfpt_renderer {
         cudaError_t e;
         auto plain = [&]() {
             return wfpt::launch_trace(sc, kind, rb.rays_cur(), rb.results.as<wfpt_hit>(), nullptr, n, n_dev,
-                                      closest ? 1 : 0, s, wk);
+                                      closest ? 1 : 0, s, wk, gpu_shared);
         };
         if (!sort) return timed(s, total, C_NONE, -1, plain);
         if (timing_on && log >= 0 && (e = timed(s, T_NONE, C_TRACE, log, plain)) != cudaSuccess) return e;
@@ -489,7 +490,8 @@ struct wfpt_renderer {
         }
         return timed(s, total, C_TRACE_SORT, log, [&]() {
             return wfpt::launch_trace(sc, kind, rb.rays_cur(), rb.results.as<wfpt_hit>(),
-                                      reorder ? nullptr : rb.idx.as<uint32_t>(), n, n_dev, closest ? 1 : 0, s, wk);
+                                      reorder ? nullptr : rb.idx.as<uint32_t>(), n, n_dev, closest ? 1 : 0, s, wk,
+                                      gpu_shared);
         });
     }
 
@@ -610,7 +612,7 @@ struct wfpt_renderer {
                  if (r != cudaSuccess) return r;
                  return wfpt::launch_trace(*wfpt::scene_device(scene), primary_kind(), primary.rays_cur(),
                                            primary.results.as<wfpt_hit>(), nullptr, n, nullptr, 1, s,
-                                           work.as<uint32_t>());
+                                           work.as<uint32_t>(), gpu_shared);
              })) != cudaSuccess)
             return e;
         const float one = 1.0f;
@@ -1038,6 +1040,7 @@ wfpt_status wfpt_batch_create(const wfpt_request* requests, uint32_t count, int 
         const wfpt_request& q = b->reqs[i];
         r->cfg = q.config;
         r->cfg.use_graph = 0;
+        r->gpu_shared = count > 1 && streams > 1;
         r->scene = q.scene;
         r->geoms = q.geometries;
         wfpt::scene_bounds(q.scene, r->smin, r->smax);

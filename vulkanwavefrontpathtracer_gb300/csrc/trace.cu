@@ -675,10 +675,20 @@ constexpr int kRing = 1024;        // per-warp ring of pending triangle tests (p
 // 31 + 32 * 31 pairs are pending after an append: they fit the ring.
 constexpr uint32_t kMoreTris = 7;
 constexpr uint32_t kFewLanes = 20;
+constexpr uint32_t kCoopLargeMin = 4 * 152 * 4 * kBlock;  // wavefronts of the four-block form
 static_assert(31 + 32 * (kMoreTris + 24) <= kRing, "the ring holds every pending pair");
 
-template <bool CLOSEST, bool COUNT>
-__global__ void __launch_bounds__(kBlock, 4) k_trace_bvh8_coop(
+// PER_SM: four blocks per SM (64 registers) keep the GPU busy on large
+// wavefronts; a small one is bound by the latency of its longest rays, and
+// three blocks per SM (80 registers) make each step shorter: 57K soup rays
+// 104 -> 100 us closest, 120K courtyard rays 150 -> 135, 262K 215 -> 203; any
+// hit 105 -> 91 us at 131K rays, 209 -> 206 at 524K.  Even at about 620K rays
+// (four times the rays resident at once), 2-4 % slower at 1M, 5 % at 2M; two
+// blocks per SM are equal to three below 120K rays and slower above.  Small
+// wavefronts that share the GPU (batched requests on several branches) keep
+// the four-block form: a 12-request batch 23.6 ms, 24.0 with three.
+template <bool CLOSEST, bool COUNT, int PER_SM>
+__global__ void __launch_bounds__(kBlock, PER_SM) k_trace_bvh8_coop(
     const float4* __restrict__ nodes, const float4* __restrict__ tris, const float4* __restrict__ rays,
     int4* __restrict__ results, const uint32_t* __restrict__ ray_index, uint32_t n,
     const uint32_t* __restrict__ n_dev, uint32_t* __restrict__ work,
@@ -904,8 +914,8 @@ __global__ void __launch_bounds__(kBlock, 4) k_trace_bvh8_coop(
 // traces on different streams do not share a counter.
 static std::atomic<uint32_t> g_slot{0};
 // Resident blocks per SM: [closest] for the per-lane kernel, [2 + closest]
-// for the cooperative one.
-static int g_blocks_per_sm[4] = {0, 0, 0, 0};
+// for the cooperative one, [4 + closest] for its small-wavefront form.
+static int g_blocks_per_sm[6] = {0, 0, 0, 0, 0, 0};
 static int g_num_sms = 0;
 static uint32_t g_refill = 6;  // 4 to 8 within 1 % on bounce-1 rays, 6 the best sum
 
@@ -960,12 +970,10 @@ cudaError_t trace_prepare() {
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_blocks_per_sm[0], k_trace_bvh8<false, false>, kBlock, 0);
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_blocks_per_sm[1], k_trace_bvh8<true, false>, kBlock, 0);
-    if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_blocks_per_sm[2], k_trace_bvh8_coop<false, false>, kBlock,
-                                                          0);
-    if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_blocks_per_sm[3], k_trace_bvh8_coop<true, false>, kBlock,
-                                                          0);
+    const void* coop[4] = {(const void*)k_trace_bvh8_coop<false, false, 4>, (const void*)k_trace_bvh8_coop<true, false, 4>,
+                           (const void*)k_trace_bvh8_coop<false, false, 3>, (const void*)k_trace_bvh8_coop<true, false, 3>};
+    for (int k = 0; k < 4 && e == cudaSuccess; ++k)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_blocks_per_sm[2 + k], coop[k], kBlock, 0);
     if (e == cudaSuccess) g_num_sms = sms;
     return e;
 }
@@ -985,7 +993,7 @@ uint32_t get_trace_postpone() { return g_postpone; }
 
 cudaError_t launch_trace(const SceneDevice& sc, int kind, const wfpt_ray* rays, wfpt_hit* results,
                          const uint32_t* ray_index, uint32_t n, const uint32_t* n_dev, int closest,
-                         cudaStream_t s, uint32_t* own_work) {
+                         cudaStream_t s, uint32_t* own_work, bool shared) {
     if (n == 0) return cudaSuccess;
     // A scene built without this BVH kind has no buffers for it.
     if (kind == WFPT_BVH8_Q8 ? (!sc.bvh8_nodes || !sc.bvh8_tris) : (!sc.bvh2_nodes || !sc.bvh2_tris))
@@ -1000,14 +1008,19 @@ cudaError_t launch_trace(const SceneDevice& sc, int kind, const wfpt_ray* rays, 
         }
         // The cooperative kernel packs a triangle record into 27 bits.
         const bool coop = g_coop && sc.bvh8_num_tris < (1u << kRecBits);
-        unsigned pgrid = (unsigned)(g_num_sms * g_blocks_per_sm[(coop ? 2 : 0) + (closest ? 1 : 0)]);
+        const bool small = coop && n < kCoopLargeMin && !shared;
+        unsigned pgrid = (unsigned)(g_num_sms * g_blocks_per_sm[(coop ? (small ? 4 : 2) : 0) + (closest ? 1 : 0)]);
         if (pgrid == 0) pgrid = 1;
         const uint32_t lanes = pgrid * kBlock;
         if (grid < pgrid) pgrid = grid;
         uint32_t* work = own_work ? own_work : sc.work + 16 * (g_slot.fetch_add(1) % kWorkSlots);
         if (coop) {
-            auto k8 = closest ? (g_count ? k_trace_bvh8_coop<true, true> : k_trace_bvh8_coop<true, false>)
-                              : (g_count ? k_trace_bvh8_coop<false, true> : k_trace_bvh8_coop<false, false>);
+            auto k8 = closest ? (g_count ? k_trace_bvh8_coop<true, true, 4> : k_trace_bvh8_coop<true, false, 4>)
+                              : (g_count ? k_trace_bvh8_coop<false, true, 4> : k_trace_bvh8_coop<false, false, 4>);
+            if (small) {
+                k8 = closest ? (g_count ? k_trace_bvh8_coop<true, true, 3> : k_trace_bvh8_coop<true, false, 3>)
+                             : (g_count ? k_trace_bvh8_coop<false, true, 3> : k_trace_bvh8_coop<false, false, 3>);
+            }
             k8<<<pgrid, kBlock, 0, s>>>(sc.bvh8_nodes, sc.bvh8_tris, rr, out, ray_index, n, n_dev, work, g_refill,
                                         kernel_batch(closest != 0), kernel_steps(closest != 0, n, lanes));
         } else {

@@ -36,9 +36,11 @@ cudaError_t trace_prepare();
 // work (nullable): the persistent BVH8 kernel's two self-resetting work
 // counters (zeroed once by the owner); launches that use the same counters
 // must be ordered one after another.  Null takes the next of the scene's
-// counter slots.
+// counter slots.  shared: other wavefronts run on the GPU beside this one
+// (batched requests), so a small one is launched for throughput like a large
+// one.
 cudaError_t launch_trace(const SceneDevice& sc, int kind, const wfpt_ray* rays, wfpt_hit* results,
                          const uint32_t* ray_index, uint32_t n, const uint32_t* n_dev, int closest,
-                         cudaStream_t s, uint32_t* work = nullptr);
+                         cudaStream_t s, uint32_t* work = nullptr, bool shared = false);
 
 }  // namespace wfpt
