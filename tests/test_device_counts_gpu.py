@@ -1,7 +1,7 @@
-"""Stage kernels whose count is on the device run at most 152 x 16 blocks that
-go on until the count is done: the same outputs as a launch of exactly that
-many rays, at counts around one grid's rays (622,592), empty and full, and
-nothing touched past the count.  The persistent BVH2 traversal of very large
+"""Stage kernels whose count is on the device and whose capacity is beyond
+152 x 64 blocks run 152 x 16 blocks that go on until the count is done: the
+same outputs as a launch of exactly that many rays, at counts around one
+grid's rays (622,592), empty and full, and nothing touched past the count.  The persistent BVH2 traversal of very large
 wavefronts (2^22 rays) the same."""
 import numpy as np
 import pytest
@@ -11,7 +11,7 @@ from conftest import random_rays
 pytestmark = pytest.mark.gpu
 
 GRID = 152 * 16 * 256
-CAP = 2 * GRID + 77
+CAP = 4 * GRID + 77
 
 
 @pytest.fixture(scope="module")

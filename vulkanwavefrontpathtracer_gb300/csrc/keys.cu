@@ -64,16 +64,22 @@ template <bool STREAM>
 __global__ void k_reorder(const uint32_t* __restrict__ idx, const uint4* __restrict__ in_rays,
                           uint4* __restrict__ out_rays, const int32_t* __restrict__ in_s2i,
                           int32_t* __restrict__ out_s2i, int32_t* __restrict__ out_i2s, uint32_t n,
-                          const uint32_t* __restrict__ n_dev) {
+                          const uint32_t* __restrict__ n_dev, bool wide) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= load_count(n, n_dev)) return;
     const uint64_t pol = STREAM ? l2_evict_first_policy() : 0u;
     uint32_t old = STREAM ? __ldcs(idx + i) : idx[i];
     int32_t index = in_s2i[old];
-    uint4 a = load_record<STREAM>(in_rays + 2 * (size_t)old + 0, pol);
-    uint4 b = load_record<STREAM>(in_rays + 2 * (size_t)old + 1, pol);
-    store_record<STREAM>(out_rays + 2 * (size_t)i + 0, a, pol);
-    store_record<STREAM>(out_rays + 2 * (size_t)i + 1, b, pol);
+    if (!STREAM && wide) {
+        float4 a, b;
+        load32(reinterpret_cast<const float4*>(in_rays) + 2 * (size_t)old, a, b);
+        store_ray(reinterpret_cast<float4*>(out_rays), i, a, b, true);
+    } else {
+        uint4 a = load_record<STREAM>(in_rays + 2 * (size_t)old + 0, pol);
+        uint4 b = load_record<STREAM>(in_rays + 2 * (size_t)old + 1, pol);
+        store_record<STREAM>(out_rays + 2 * (size_t)i + 0, a, pol);
+        store_record<STREAM>(out_rays + 2 * (size_t)i + 1, b, pol);
+    }
     if (STREAM) {
         __stcs(out_s2i + i, index);
     } else {
@@ -284,7 +290,7 @@ cudaError_t launch_reorder(const uint32_t* idx, const wfpt_ray* in_rays, wfpt_ra
     unsigned grid = (n + kBlock - 1) / kBlock;
     auto k = n >= kStreamRecords ? k_reorder<true> : k_reorder<false>;
     k<<<grid, kBlock, 0, s>>>(idx, reinterpret_cast<const uint4*>(in_rays), reinterpret_cast<uint4*>(out_rays), in_s2i,
-                              out_s2i, out_i2s, n, n_dev);
+                              out_s2i, out_i2s, n, n_dev, wide_rays(in_rays) && wide_rays(out_rays));
     count_launch();
     return cudaGetLastError();
 }

@@ -79,7 +79,7 @@ struct Mat4 {
 __global__ void k_raygen_primary(Mat4 s2w, const int32_t* __restrict__ index_to_pixel,
                                  float4* __restrict__ rays, float ox, float oy, float oz,
                                  int sample_index, int width, int height, float max_dist,
-                                 const FrameParams* __restrict__ fp, int pass, int spp) {
+                                 const FrameParams* __restrict__ fp, int pass, int spp, bool wide) {
     uint32_t task = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t num_pixels = (uint32_t)width * (uint32_t)height;
     if (task >= num_pixels) return;
@@ -114,8 +114,7 @@ __global__ void k_raygen_primary(Mat4 s2w, const int32_t* __restrict__ index_to_
     f3 world = mk(__fdiv_rn(w4[0], w4[3]), __fdiv_rn(w4[1], w4[3]), __fdiv_rn(w4[2], w4[3]));
     f3 o = mk(ox, oy, oz);
     f3 d = normalize(sub(world, o));
-    rays[2 * task + 0] = make_float4(ox, oy, oz, 0.0f);
-    rays[2 * task + 1] = make_float4(d.x, d.y, d.z, max_dist);
+    store_ray(rays, task, make_float4(ox, oy, oz, 0.0f), make_float4(d.x, d.y, d.z, max_dist), wide);
 }
 
 // -------------------------------------------------------------- shadow
@@ -147,20 +146,30 @@ __device__ __forceinline__ void sobol2d(uint32_t i, float& x, float& y) {
     y = __fdiv_rn(__uint2float_rn(r2), 4294967296.0f);
 }
 
+// The next element of a thread: a grid's width on in the kernels whose grid
+// is capped (LOOP, see grid_for), none where it has a thread per element (the
+// compiler then drops the loop, which cost the reconstructions 5 %).
+template <bool LOOP>
+__device__ __forceinline__ uint32_t next_task(uint32_t task) {
+    return LOOP ? task + gridDim.x * blockDim.x : 0xFFFFFFFFu;
+}
+
 // raygenShadow.comp:82-136.  Output rays of input task t occupy
 // [S*t, S*t+S) of the batch-local output buffer.
+template <bool LOOP>
 __global__ void k_raygen_shadow(const uint32_t* __restrict__ seeds,
                                 const float4* __restrict__ in_rays,
                                 const int4* __restrict__ in_results, float4* __restrict__ out_rays,
                                 int32_t* __restrict__ out_s2i, int32_t* __restrict__ out_i2s,
                                 float lx, float ly, float lz, float radius, int batch_begin,
-                                int batch_size, const uint32_t* __restrict__ n_in_dev, int S) {
+                                int batch_size, const uint32_t* __restrict__ n_in_dev, int S, bool wide) {
     int size = batch_size;
     if (n_in_dev != nullptr) {
         int avail = (int)*n_in_dev - batch_begin;
         if (avail < size) size = avail;
     }
-    for (uint32_t task = blockIdx.x * blockDim.x + threadIdx.x; (int64_t)task < size; task += gridDim.x * blockDim.x) {
+    for (uint32_t task = blockIdx.x * blockDim.x + threadIdx.x; (int64_t)task < size;
+         task = next_task<LOOP>(task)) {
         uint32_t seed = seeds[task];
         float4 r0 = in_rays[2 * (batch_begin + task) + 0];
         float4 r1 = in_rays[2 * (batch_begin + task) + 1];
@@ -195,8 +204,8 @@ __global__ void k_raygen_shadow(const uint32_t* __restrict__ seeds,
             f3 dir = sub(target, origin);
             f3 nd = tri == -1 ? mk(1.0f, 0.0f, 0.0f) : normalize(dir);
             float tmax = tri == -1 ? -1.0f : length(dir);
-            out_rays[2 * ray_index + 0] = make_float4(origin.x, origin.y, origin.z, EPS);
-            out_rays[2 * ray_index + 1] = make_float4(nd.x, nd.y, nd.z, tmax);
+            store_ray(out_rays, ray_index, make_float4(origin.x, origin.y, origin.z, EPS),
+                      make_float4(nd.x, nd.y, nd.z, tmax), wide);
             out_s2i[ray_index] = ray_index;
             out_i2s[ray_index] = ray_index;
             ++ray_index;
@@ -322,7 +331,7 @@ __global__ void k_raygen_path(uint32_t* __restrict__ seeds, const wfpt_geometry*
                               uint32_t* __restrict__ out_count, uint32_t n,
                               const uint32_t* __restrict__ n_dev, float albedo,
                               uint32_t* __restrict__ scratch, void* __restrict__ keys,
-                              uint32_t* __restrict__ key_idx, Box6 box) {
+                              uint32_t* __restrict__ key_idx, Box6 box, bool wide) {
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_warp[kBlock / 32];
     uint32_t count = load_count(n, n_dev);
@@ -388,8 +397,7 @@ __global__ void k_raygen_path(uint32_t* __restrict__ seeds, const wfpt_geometry*
         }
         if (active) {
             uint32_t dst = base + warp_off + lane_rank;
-            out_rays[2 * dst + 0] = o0;
-            out_rays[2 * dst + 1] = o1;
+            store_ray(out_rays, dst, o0, o1, wide);
             out_i2p[dst] = pixel;
             if (MK >= 0) {
                 write_morton_key<(MK < 0 ? 0 : MK)>(keys, dst, o0, o1, box);
@@ -415,6 +423,7 @@ __global__ void k_raygen_path(uint32_t* __restrict__ seeds, const wfpt_geometry*
 // are taken as zero instead of being read (the renderer's per-pass colour
 // buffer, cleared before every pass in the reference: each of its pixels
 // has one ray per pass), with the same addition to zero.
+template <bool LOOP>
 __global__ void k_reconstruct_smooth(const float4* __restrict__ rays, const int4* __restrict__ results,
                                      const int32_t* __restrict__ i2p, float4* __restrict__ pixels,
                                      const float4* __restrict__ decreases,
@@ -424,7 +433,7 @@ __global__ void k_reconstruct_smooth(const float4* __restrict__ rays, const int4
                                      uint32_t* __restrict__ hit_count, int fresh) {
     const uint32_t count = load_count(n, n_dev);
     uint32_t hits = 0;
-    for (uint32_t task = blockIdx.x * blockDim.x + threadIdx.x; task < count; task += gridDim.x * blockDim.x) {
+    for (uint32_t task = blockIdx.x * blockDim.x + threadIdx.x; task < count; task = next_task<LOOP>(task)) {
         int pixel = i2p[task];
         const float4 pc = fresh ? make_float4(0.0f, 0.0f, 0.0f, 0.0f) : pixels[pixel];
         f3 color = mk(pc.x, pc.y, pc.z);
@@ -465,6 +474,7 @@ __global__ void k_reconstruct_smooth(const float4* __restrict__ rays, const int4
 
 // ---------------------------------------------------- reconstructShadow
 // reconstructShadow.comp:39-59.
+template <bool LOOP>
 __global__ void k_reconstruct_shadow(const int4* __restrict__ results, const int32_t* __restrict__ i2p,
                                      const int32_t* __restrict__ i2s,
                                      const float4* __restrict__ in_pixels, float4* __restrict__ out_pixels,
@@ -475,7 +485,8 @@ __global__ void k_reconstruct_shadow(const int4* __restrict__ results, const int
         int avail = (int)*n_in_dev - batch_begin;
         if (avail < size) size = avail;
     }
-    for (uint32_t task = blockIdx.x * blockDim.x + threadIdx.x; (int64_t)task < size; task += gridDim.x * blockDim.x) {
+    for (uint32_t task = blockIdx.x * blockDim.x + threadIdx.x; (int64_t)task < size;
+         task = next_task<LOOP>(task)) {
         int pixel = i2p[batch_begin + task];
         float4 ip = in_pixels[pixel];
         float shadow = 0.0f;
@@ -618,9 +629,10 @@ static inline unsigned grid_for(uint64_t n) { return (unsigned)((n + kBlock - 1)
 // (two waves of blocks keep every SM full); with the BVH2 traversal's
 // persistent form a 4K city frame went from 20.4 to 18.5 ms.
 constexpr unsigned kStageGrid = 152 * 16;
+constexpr unsigned kStageCapped = 152 * 64;  // capacities of fewer blocks (2.5M rays) keep a block each
+static inline bool capped(uint64_t n, const uint32_t* n_dev) { return n_dev != nullptr && grid_for(n) > kStageCapped; }
 static inline unsigned grid_for(uint64_t n, const uint32_t* n_dev) {
-    const unsigned g = grid_for(n);
-    return n_dev != nullptr && g > kStageGrid ? kStageGrid : g;
+    return capped(n, n_dev) ? kStageGrid : grid_for(n);
 }
 
 cudaError_t launch_init_seeds(uint32_t* seeds, uint32_t n, int frame, cudaStream_t s, const FrameParams* fp) {
@@ -639,7 +651,8 @@ cudaError_t launch_raygen_primary(const float* m, const int32_t* i2p, wfpt_ray* 
     for (int i = 0; i < 16; ++i) mm.m[i] = m ? m[i] : 0.0f;
     float oo[3] = {o ? o[0] : 0.0f, o ? o[1] : 0.0f, o ? o[2] : 0.0f};
     k_raygen_primary<<<grid_for(n), kBlock, 0, s>>>(mm, i2p, reinterpret_cast<float4*>(rays), oo[0], oo[1],
-                                                    oo[2], sample_index, w, h, max_dist, fp, pass, spp);
+                                                    oo[2], sample_index, w, h, max_dist, fp, pass, spp,
+                                                    wide_rays(rays));
     count_launch();
     return cudaGetLastError();
 }
@@ -649,10 +662,11 @@ cudaError_t launch_raygen_shadow(const uint32_t* seeds, const wfpt_ray* in_rays,
                                  float radius, int bb, int bs, const uint32_t* n_in_dev, int S,
                                  cudaStream_t s) {
     if (bs <= 0) return cudaSuccess;
-    k_raygen_shadow<<<grid_for((uint64_t)bs, n_in_dev), kBlock, 0, s>>>(
+    auto k = capped((uint64_t)bs, n_in_dev) ? k_raygen_shadow<true> : k_raygen_shadow<false>;
+    k<<<grid_for((uint64_t)bs, n_in_dev), kBlock, 0, s>>>(
         seeds, reinterpret_cast<const float4*>(in_rays), reinterpret_cast<const int4*>(in_res),
         reinterpret_cast<float4*>(out_rays), s2i, i2s, light[0], light[1], light[2], radius, bb, bs,
-        n_in_dev, S);
+        n_in_dev, S, wide_rays(out_rays));
     count_launch();
     return cudaGetLastError();
 }
@@ -682,7 +696,7 @@ cudaError_t launch_raygen_path(uint32_t* seeds, const wfpt_geometry* geoms, cons
                               reinterpret_cast<float4*>(out_rays), in_i2p, out_i2p,
                               reinterpret_cast<const int4*>(in_res), reinterpret_cast<float4*>(decreases),
                               out_count, n, n_dev, albedo, reinterpret_cast<uint32_t*>(scratch),
-                              mo ? mo->keys : nullptr, mo ? mo->indices : nullptr, box);
+                              mo ? mo->keys : nullptr, mo ? mo->indices : nullptr, box, wide_rays(out_rays));
     count_launch();
     return cudaGetLastError();
 }
@@ -717,7 +731,7 @@ cudaError_t raygen_path_selftest_timeout(cudaStream_t s) {
     if (e == cudaSuccess) {
         k_raygen_path<-1><<<1, kBlock, 0, s>>>(seeds, nullptr, in_rays, out_rays, in_i2p, out_i2p, results,
                                                decreases, count, N, nullptr, 0.8f, scratch, nullptr, nullptr,
-                                               Box6{});
+                                               Box6{}, wide_rays(out_rays));
         count_launch();
         e = cudaGetLastError();
     }
@@ -821,7 +835,7 @@ cudaError_t launch_raygen_path_static(uint32_t* seeds, const wfpt_geometry* geom
     k_raygen_path<-1><<<grid, kBlock, 0, s>>>(
         seeds, geoms, reinterpret_cast<const float4*>(in_rays), reinterpret_cast<float4*>(out_rays), in_i2p,
         out_i2p, reinterpret_cast<const int4*>(in_res), reinterpret_cast<float4*>(decreases), out_count, n,
-        n_dev, albedo, scratch, nullptr, nullptr, Box6{});
+        n_dev, albedo, scratch, nullptr, nullptr, Box6{}, wide_rays(out_rays));
     count_launch();
     return cudaGetLastError();
 }
@@ -832,7 +846,8 @@ cudaError_t launch_reconstruct_smooth(const wfpt_ray* rays, const wfpt_hit* res,
                                       const uint32_t* n_dev, int spp, cudaStream_t s, uint32_t* hit_count,
                                       bool fresh) {
     if (n == 0) return cudaSuccess;
-    k_reconstruct_smooth<<<grid_for(n, n_dev), kBlock, 0, s>>>(
+    auto k = capped(n, n_dev) ? k_reconstruct_smooth<true> : k_reconstruct_smooth<false>;
+    k<<<grid_for(n, n_dev), kBlock, 0, s>>>(
         reinterpret_cast<const float4*>(rays), reinterpret_cast<const int4*>(res), i2p,
         reinterpret_cast<float4*>(pixels), reinterpret_cast<const float4*>(decreases), geoms, light[0],
         light[1], light[2], bg[0], bg[1], bg[2], n, n_dev, spp, hit_count, fresh ? 1 : 0);
@@ -844,7 +859,8 @@ cudaError_t launch_reconstruct_shadow(const wfpt_hit* res, const int32_t* i2p, c
                                       const float* in_pixels, float* out_pixels, int bb, int bs,
                                       const uint32_t* n_in_dev, int S, int replace, cudaStream_t s) {
     if (bs <= 0) return cudaSuccess;
-    k_reconstruct_shadow<<<grid_for((uint64_t)bs, n_in_dev), kBlock, 0, s>>>(
+    auto k = capped((uint64_t)bs, n_in_dev) ? k_reconstruct_shadow<true> : k_reconstruct_shadow<false>;
+    k<<<grid_for((uint64_t)bs, n_in_dev), kBlock, 0, s>>>(
         reinterpret_cast<const int4*>(res), i2p, i2s, reinterpret_cast<const float4*>(in_pixels),
         reinterpret_cast<float4*>(out_pixels), bb, bs, n_in_dev, S, replace);
     count_launch();

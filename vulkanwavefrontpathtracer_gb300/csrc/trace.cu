@@ -193,13 +193,6 @@ __device__ __forceinline__ void box2(const RayT& r, float lox, float hix, float 
     hit = tn <= tf * kBoxSlack;
 }
 
-// 32 bytes in one load (256-bit loads, sm_100 and later).
-__device__ __forceinline__ void load32(const float4* p, float4& a, float4& b) {
-    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
-        : "l"(p));
-}
-
 // One ray, traced by one thread.
 template <bool CLOSEST, bool COUNT>
 __device__ __forceinline__ void trace_bvh2_ray(const float4* __restrict__ nodes, const float4* __restrict__ tris,
