@@ -52,6 +52,7 @@ struct RayT {
     int kx, ky, kz;
     float sx, sy, sz;
     uint32_t oct;  // bit k = sign bit of d[k]
+    uint32_t perm0, perm1;  // byte c & 3: 1 << (c ^ oct) for the BVH8 slots c = 0..3 and 4..7
 };
 
 __device__ __forceinline__ float comp(const f3& v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); }
@@ -89,6 +90,9 @@ __device__ __forceinline__ RayT setup_ray(const float4& r0, const float4& r1) {
     // the BVH8 near/far plane choice must agree with the sign of inv.
     r.oct = (__float_as_uint(d.x) >> 31) | ((__float_as_uint(d.y) >> 31) << 1) |
             ((__float_as_uint(d.z) >> 31) << 2);
+    const uint32_t low = __byte_perm(0x08040201u, 0u, 0x3210u ^ ((r.oct & 3u) * 0x1111u));
+    r.perm0 = low << (r.oct & 4u);
+    r.perm1 = low << (4u - (r.oct & 4u));
     return r;
 }
 
@@ -358,11 +362,38 @@ __device__ __forceinline__ float q2f(uint32_t w, int b) {
     return __uint_as_float(__byte_perm(w, 0x47000000u, 0x7604u | ((uint32_t)b << 4)));
 }
 
-// Intersects the eight children of a BVH8 node.  Returns the hit mask:
-// bits 24..31 inner children (octant-permuted slot order, highest first),
-// bits 0..23 triangles relative to *tri_base; *child_base and *imask out.
+// Two FP32 fused multiply-adds in one instruction (sm_100 and later), each
+// rounded as one alone: a child's near and far plane of an axis.
+__device__ __forceinline__ uint64_t pair2(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ void unpair2(uint64_t v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+
+// Intersects the eight children of a BVH8 node.  Returns its inner hits in
+// bits 24..31 (octant-permuted slot order, highest first) and its leaf hits in
+// `leaf` (bit 8 (c & 3) + (c & 4) for slot c), which leaf_count and
+// leaf_tris below turn into triangles of the node's second 16 bytes.
+// A node step is half of the traversal's time, and bound by issue slots (78 %
+// used) and the half-rate ALU pipe (63 %: byte permutes, min/max, selects,
+// logic).  So a hit child costs one predicated OR here: shifting its unary
+// count to its bit index (two permutes, a shift and an OR per child, and the
+// decoding of the meta bytes) is left to the few nodes with leaf hits, once
+// per loop iteration, and the inner hits are permuted all at once by two
+// 4-way byte dot products: closest hit 1005 -> 949 us (courtyard, 2.07M sorted
+// bounce-1 rays), any hit 1221 -> 1141 us.  With the ALU relieved, the paired
+// multiply-adds pay too (24 issue slots a node): 949 -> 920 and 1141 -> 1108
+// us.  City: 468 -> 444 and 361 -> 339 us.
 __device__ __forceinline__ uint32_t intersect_node8(const float4* __restrict__ nd, const RayT& r, float tcur,
-                                                    uint32_t& child_base, uint32_t& tri_base, uint32_t& imask) {
+                                                    uint32_t& child_base, uint32_t& imask, uint32_t& leaf) {
     float4 n0 = __ldg(nd + 0);
     float4 n1 = __ldg(nd + 1);
     float4 n2 = __ldg(nd + 2);
@@ -375,7 +406,6 @@ __device__ __forceinline__ uint32_t intersect_node8(const float4* __restrict__ n
     float scz = __uint_as_float(((ew >> 16) & 0xFFu) << 23);
     imask = ew >> 24;
     child_base = __float_as_uint(n1.x);
-    tri_base = __float_as_uint(n1.y);
     // Slab distance = q * (scale*inv) + (p - o) * inv, evaluated as
     // (2^15 + q) * a + (b - 2^15 a).  The folded offset is rounded twice
     // (about 2^-24 * (|b| + 2^15 |a|) each); near planes move earlier and far
@@ -403,37 +433,48 @@ __device__ __forceinline__ uint32_t intersect_node8(const float4* __restrict__ n
     uint32_t fy[2] = {sy ? __float_as_uint(n2.z) : __float_as_uint(n4.x), sy ? __float_as_uint(n2.w) : __float_as_uint(n4.y)};
     uint32_t nz[2] = {sz ? __float_as_uint(n4.z) : __float_as_uint(n3.x), sz ? __float_as_uint(n4.w) : __float_as_uint(n3.y)};
     uint32_t fz[2] = {sz ? __float_as_uint(n3.x) : __float_as_uint(n4.z), sz ? __float_as_uint(n3.y) : __float_as_uint(n4.w)};
-    // Meta bytes, four at a time: inner children (bits 4 and 3 set) get
-    // their hit bit permuted by the octant; child_bits is the unary count.
-    uint32_t bit_index[2], child_bits[2];
-    const uint32_t oct4 = oct * 0x01010101u;
-#pragma unroll
-    for (int w = 0; w < 2; ++w) {
-        uint32_t m4 = __float_as_uint(w ? n1.w : n1.z);
-        uint32_t inner4 = (m4 & (m4 << 1)) & 0x10101010u;
-        uint32_t perm = oct4 & ((inner4 >> 4) * 7u);
-        bit_index[w] = (m4 ^ perm) & 0x1F1F1F1Fu;
-        child_bits[w] = (m4 >> 5) & 0x07070707u;
-    }
-    // Box tests; a hit child contributes its unary count at its bit index
-    // (empty slots have child_bits 0 and contribute nothing).  Building the
-    // mask inside the unrolled loop, instead of looping over the hit bits
-    // afterwards, removes a divergent loop of about 13 instructions per hit
-    // child (8 % faster closest-hit traversal).
-    uint32_t hitmask = 0;
+    // Pairs {near, far}; children's planes are multiplied and added in pairs.
+    const uint64_t A[3] = {pair2(ax, ax), pair2(ay, ay), pair2(az, az)};
+    const uint64_t B[3] = {pair2(bxn, bxf), pair2(byn, byf), pair2(bzn, bzf)};
+    // Box tests: bit 4 of byte c set for a hit child c.
+    uint32_t hit[2] = {0u, 0u};
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
         const int w = c >> 2, b = c & 3;
-        float tnx = __fmaf_rn(q2f(nx[w], b), ax, bxn), tfx = __fmaf_rn(q2f(fx[w], b), ax, bxf);
-        float tny = __fmaf_rn(q2f(ny[w], b), ay, byn), tfy = __fmaf_rn(q2f(fy[w], b), ay, byf);
-        float tnz = __fmaf_rn(q2f(nz[w], b), az, bzn), tfz = __fmaf_rn(q2f(fz[w], b), az, bzf);
+        float tnx, tny, tnz, tfx, tfy, tfz;
+        unpair2(fma2(pair2(q2f(nx[w], b), q2f(fx[w], b)), A[0], B[0]), tnx, tfx);
+        unpair2(fma2(pair2(q2f(ny[w], b), q2f(fy[w], b)), A[1], B[1]), tny, tfy);
+        unpair2(fma2(pair2(q2f(nz[w], b), q2f(fz[w], b)), A[2], B[2]), tnz, tfz);
         float tn = fmaxf(max3f(tnx, tny, tnz), r.tmin);
         float tf = fminf(min3f(tfx, tfy, tfz), tcur);
-        const uint32_t contrib = __byte_perm(child_bits[w], 0u, 0x4440u | (uint32_t)b)
-                                 << __byte_perm(bit_index[w], 0u, 0x4440u | (uint32_t)b);
-        if (tn <= tf * kBoxSlack) hitmask |= contrib;
+        if (tn <= tf * kBoxSlack) hit[w] |= 0x10u << (8 * b);
     }
-    return hitmask;
+    // Meta bytes: an inner child has bits 5, 4 and 3 set (001 | 24 + slot), a
+    // leaf its unary triangle count in bits 5..7 (bit 5 always set) over an
+    // offset of at most 23, an empty slot 0.  The inner hits go to their
+    // permuted places by the dot product of the 16-valued hit bytes with the
+    // ray's bytes 1 << (slot ^ octant).
+    const uint32_t m0 = __float_as_uint(n1.z), m1 = __float_as_uint(n1.w);
+    const uint32_t in0 = hit[0] & m0 & (m0 << 1), in1 = hit[1] & m1 & (m1 << 1);
+    leaf = ((hit[0] & ~in0 & (m0 >> 1)) >> 4) | (hit[1] & ~in1 & (m1 >> 1));
+    return __dp4a(in0, r.perm0, __dp4a(in1, r.perm1, 0u)) << 20;
+}
+
+// Triangles of a node's leaf hits (`leaf` of intersect_node8), m0 and m1 its
+// meta words.
+__device__ __forceinline__ uint32_t leaf_count(uint32_t leaf, uint32_t m0, uint32_t m1) {
+    return __popc(m0 & ((leaf & 0x01010101u) * 0xE0u)) + __popc(m1 & (((leaf >> 4) & 0x01010101u) * 0xE0u));
+}
+// The same as bits 0..23 relative to the node's first triangle.
+__device__ __forceinline__ uint32_t leaf_tris(uint32_t leaf, uint32_t m0, uint32_t m1) {
+    uint32_t tris = 0;
+    while (leaf != 0u) {
+        const uint32_t bit = (uint32_t)__ffs(leaf) - 1u;
+        leaf &= leaf - 1u;
+        const uint32_t m = ((bit & 4u) ? m1 : m0) >> (bit & 24u);
+        tris |= ((m >> 5) & 7u) << (m & 31u);
+    }
+    return tris;
 }
 
 // Persistent-warp traversal.  work[0] = next ray to hand out, work[1] =
@@ -519,11 +560,16 @@ __global__ void __launch_bounds__(kBlock, 4) k_trace_bvh8(const float4* __restri
                     raise_status(kErrBounds);
                 }
             }
-            uint32_t child_base, imask;
+            uint32_t child_base, imask, leaf;
             if (COUNT) ++c_nodes;
-            uint32_t hitmask = intersect_node8(nodes + 5 * (size_t)node, r, h.t, child_base, tri_base, imask);
-            ng = make_uint2(child_base, (hitmask & 0xFF000000u) | imask);
-            tg = hitmask & 0x00FFFFFFu;
+            const float4* nd = nodes + 5 * (size_t)node;
+            const uint32_t inner = intersect_node8(nd, r, h.t, child_base, imask, leaf);
+            ng = make_uint2(child_base, inner | imask);
+            if (leaf != 0u) {
+                const float4 n1 = __ldg(nd + 1);
+                tri_base = __float_as_uint(n1.y);
+                tg = leaf_tris(leaf, __float_as_uint(n1.z), __float_as_uint(n1.w));
+            }
         } else {
             tri_base = ng.x;
             tg = ng.y;
@@ -654,7 +700,7 @@ constexpr int kRing = 1024;        // per-warp ring of pending triangle tests (p
 // of the time: a lane that stopped at its first triangles waited for the rest
 // of the iteration, so more than two (any hit: three) steps did not pay.  A
 // lane now goes on with its triangles in hand until a second node hands it
-// some (or the first handed it more than kMoreTris), and four steps do:
+// some (or the first handed it more than kMoreLeaves leaves), and four steps do:
 // closest hit 1070 -> 1003 us (courtyard, 2.07M sorted bounce-1 rays), 502 ->
 // 467 us (city, 1.6M), 122 -> 104 us (57K rays of the 65K soup); any hit
 // 1286 -> 1221, 393 -> 361 and 119 -> 109 us.  A closest-hit iteration asks
@@ -664,12 +710,12 @@ constexpr int kRing = 1024;        // per-warp ring of pending triangle tests (p
 // short, and an early end brings the refill forward (city 392 -> 361 us
 // against steps taken to the end; a share of the tracing lanes instead of a
 // number 396-421, 16 or 22 lanes 362-363, 18 lanes and six steps 375).
-// A lane appends at most kMoreTris + 24 triangles per iteration, so at most
-// 31 + 32 * 31 pairs are pending after an append: they fit the ring.
-constexpr uint32_t kMoreTris = 7;
+// A lane appends at most 3 kMoreLeaves + 24 triangles per iteration, so at most
+// 31 + 32 * 30 pairs are pending after an append: they fit the ring.
+constexpr uint32_t kMoreLeaves = 2;
 constexpr uint32_t kFewLanes = 20;
 constexpr uint32_t kCoopLargeMin = 4 * 152 * 4 * kBlock;  // wavefronts of the four-block form
-static_assert(31 + 32 * (kMoreTris + 24) <= kRing, "the ring holds every pending pair");
+static_assert(31 + 32 * (3 * kMoreLeaves + 24) <= kRing, "the ring holds every pending pair");
 
 // PER_SM: four blocks per SM (64 registers) keep the GPU busy on large
 // wavefronts; a small one is bound by the latency of its longest rays, and
@@ -758,11 +804,11 @@ __global__ void __launch_bounds__(kBlock, PER_SM) k_trace_bvh8_coop(
         if (__ballot_sync(0xffffffffu, state != kIdle || !exhausted) == 0u) break;
         if (COUNT && lane == 0) ++c_iters;
 
-        // Up to `steps` node steps, with up to two groups of triangles.
-        uint32_t tri_base = 0, tg = 0, tri_base2 = 0, tg2 = 0;
+        // Up to `steps` node steps, with up to two nodes' leaf hits in hand.
+        uint32_t leaf = 0, leaf2 = 0, from = 0, from2 = 0;
         const uint32_t few = CLOSEST ? 0u : (__any_sync(0xffffffffu, exhausted) ? 1u : kFewLanes);
         for (uint32_t st = 0; st < steps; ++st) {
-            const bool go = state == kTracing && ng.y > 0x00FFFFFFu && tg2 == 0u && __popc(tg) <= kMoreTris;
+            const bool go = state == kTracing && ng.y > 0x00FFFFFFu && leaf2 == 0u && __popc(leaf) <= kMoreLeaves;
             if (CLOSEST ? (st == 2u && !__any_sync(0xffffffffu, go))
                         : (st >= 1u && (uint32_t)__popc(__ballot_sync(0xffffffffu, go)) < few))
                 break;
@@ -778,23 +824,29 @@ __global__ void __launch_bounds__(kBlock, PER_SM) k_trace_bvh8_coop(
                         raise_status(kErrBounds);
                     }
                 }
-                uint32_t child_base, imask, tb;
+                uint32_t child_base, imask, lf;
                 if (COUNT) ++c_nodes;
-                uint32_t hitmask = intersect_node8(nodes + 5 * (size_t)node, r, tcur, child_base, tb, imask);
-                ng = make_uint2(child_base, (hitmask & 0xFF000000u) | imask);
-                if (tg == 0u) {
-                    tg = hitmask & 0x00FFFFFFu;
-                    tri_base = tb;
+                const uint32_t inner = intersect_node8(nodes + 5 * (size_t)node, r, tcur, child_base, imask, lf);
+                ng = make_uint2(child_base, inner | imask);
+                if (leaf == 0u) {
+                    leaf = lf;
+                    from = node;
                 } else {
-                    tg2 = hitmask & 0x00FFFFFFu;
-                    tri_base2 = tb;
+                    leaf2 = lf;
+                    from2 = node;
                 }
             }
             if (state == kTracing && ng.y <= 0x00FFFFFFu && sp > 0) ng = stack[--sp];
         }
 
-        // Append this step's pairs: exclusive scan of the per-lane counts.
-        const uint32_t cnt = __popc(tg) + __popc(tg2);
+        // Append the pairs: exclusive scan of the per-lane counts.  The nodes'
+        // meta words and first triangles are read again here, mostly from
+        // L1, by the lanes with leaf hits.
+        uint4 meta = make_uint4(0u, 0u, 0u, 0u), meta2 = meta;
+        if (leaf != 0u) meta = __ldg(reinterpret_cast<const uint4*>(nodes + 5 * (size_t)from + 1));
+        if (leaf2 != 0u) meta2 = __ldg(reinterpret_cast<const uint4*>(nodes + 5 * (size_t)from2 + 1));
+        const uint32_t cnt1 = leaf_count(leaf, meta.z, meta.w);
+        const uint32_t cnt = cnt1 + leaf_count(leaf2, meta2.z, meta2.w);
         uint32_t incl = cnt;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
@@ -805,15 +857,19 @@ __global__ void __launch_bounds__(kBlock, PER_SM) k_trace_bvh8_coop(
         if (cnt != 0u) {
             uint32_t pos = appended + incl - cnt;
             const uint32_t owner = lane << kRecBits;
-            if (!CLOSEST) s_second[threadIdx.x] = pos + __popc(tg);
-            while (tg != 0u) {
-                uint32_t tb = __ffs(tg) - 1u;
-                tg &= tg - 1u;
-                task[pos++ & (kRing - 1)] = owner | (tri_base + tb);
-                if (tg == 0u) {
-                    tg = tg2;
-                    tri_base = tri_base2;
-                    tg2 = 0u;
+            if (!CLOSEST) s_second[threadIdx.x] = pos + cnt1;
+            while (leaf != 0u) {
+                const uint32_t bit = (uint32_t)__ffs(leaf) - 1u;
+                leaf &= leaf - 1u;
+                const uint32_t m = ((bit & 4u) ? meta.w : meta.z) >> (bit & 24u);
+                const uint32_t w = owner | (meta.y + (m & 31u));
+                task[pos++ & (kRing - 1)] = w;
+                if (m & 0x40u) task[pos++ & (kRing - 1)] = w + 1u;
+                if (m & 0x80u) task[pos++ & (kRing - 1)] = w + 2u;
+                if (leaf == 0u) {
+                    leaf = leaf2;
+                    meta = meta2;
+                    leaf2 = 0u;
                 }
             }
             my_end = pos;
