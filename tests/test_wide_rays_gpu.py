@@ -53,6 +53,17 @@ def test_every_ray_writer(wf, dev, n):
         write(a)
         write(b)
         assert torch.equal(a, b), write.__name__
+    # rays and vertices read from buffers 16 bytes past a multiple of 32
+    odd = buffers(dev, n)[1]
+    odd.copy_(src)
+    seeds, o, ref = [ident.clone(), ident.clone()], torch.empty_like(src), torch.empty_like(src)
+    verts = torch.zeros(geom.vertices.numel() + 4, dtype=torch.float32, device=dev)[4:]
+    verts.copy_(geom.vertices.view(-1))
+    table = torch.tensor([[verts.data_ptr(), geom.indices.data_ptr()]], dtype=torch.int64, device=dev)
+    for sd, tab, r, out in ((seeds[0], geom.table, src, ref), (seeds[1], table, odd, o)):
+        out.fill_(0)
+        api.raygen_path(sd, tab, r, out, ident, z(n), hits, torch.ones((n, 4), device=dev), z(1))
+    assert torch.equal(o, ref) and torch.equal(seeds[0], seeds[1])
     misread = buffers(dev, n)[1]
     misread.copy_(src)
     o = torch.empty_like(src)

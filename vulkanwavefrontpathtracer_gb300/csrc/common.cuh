@@ -62,6 +62,18 @@ __device__ __forceinline__ void load32(const float4* p, float4& a, float4& b) {
         : "l"(p));
 }
 
+// A 32-byte ray record in one load where its buffer starts on a multiple of 32
+// bytes (wide).
+__device__ __forceinline__ void load_ray(const float4* rays, size_t i, float4& a, float4& b, bool wide) {
+    const float4* p = rays + 2 * i;
+    if (wide) {
+        load32(p, a, b);
+    } else {
+        a = p[0];
+        b = p[1];
+    }
+}
+
 // Writes a 32-byte ray record.  One 256-bit store (sm_100 and later) when the
 // buffer allows it (wide: it starts on a multiple of 32 bytes): two 128-bit
 // ones each write half of every 32-byte sector, and a warp's stores reach L2

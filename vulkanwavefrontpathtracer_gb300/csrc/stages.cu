@@ -216,6 +216,9 @@ __global__ void k_raygen_shadow(const uint32_t* __restrict__ seeds,
 // ------------------------------------------------------- unpackTriangle
 // geometrytypes.glsl:18-47: interpolated, normalised vertex normal from the
 // 96-byte vkglTF::Vertex records (normal = (d0.w, d1.x, d1.y)).
+// WIDE: a vertex's first 32 bytes (96-byte records) in one load where the
+// array allows it (12 registers more than its caller reconstructSmooth has).
+template <bool WIDE>
 __device__ __forceinline__ f3 unpack_normal(const wfpt_geometry* __restrict__ geoms, int geom,
                                             int prim, uint32_t packed_bary) {
     wfpt_geometry g = geoms[geom];
@@ -227,11 +230,11 @@ __device__ __forceinline__ f3 unpack_normal(const wfpt_geometry* __restrict__ ge
     float cs[3] = {c0, bu, bv};
     f3 n = mk(0.0f, 0.0f, 0.0f);
     uint32_t tri = (uint32_t)prim * 3u;
+    const bool wide = WIDE && (g.vertex_addr & 31u) == 0;
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
-        uint32_t off = idx[tri + i] * 6u;
-        float4 d0 = verts[off + 0];
-        float4 d1 = verts[off + 1];
+        float4 d0, d1;
+        load_ray(verts, (size_t)(idx[tri + i] * 3u), d0, d1, wide);
         f3 ni = mul(mk(d0.w, d1.x, d1.y), cs[i]);
         n = (i == 0) ? ni : add(n, ni);
     }
@@ -323,8 +326,13 @@ __device__ uint32_t tile_prefix(uint32_t* tile_state, uint32_t tile, uint32_t co
 // the Morton key of kind MK of every output ray and its index (keys[dst],
 // key_idx[dst] = dst), which the Morton kernel would otherwise compute
 // from the written rays.
+// Bound by the latency of its chain of gathers (hit, geometry, indices,
+// vertices, then the look-back): eight blocks per SM (32 registers, a few
+// spilled) and 256-bit loads of the ray and the vertices, 97 -> 87 us at 2.07M
+// courtyard rays, 342 -> 302 at 8.3M; at 46 registers and five blocks 93 and
+// 320.
 template <int MK>
-__global__ void k_raygen_path(uint32_t* __restrict__ seeds, const wfpt_geometry* __restrict__ geoms,
+__global__ void __launch_bounds__(kBlock, 8) k_raygen_path(uint32_t* __restrict__ seeds, const wfpt_geometry* __restrict__ geoms,
                               const float4* __restrict__ in_rays, float4* __restrict__ out_rays,
                               const int32_t* __restrict__ in_i2p, int32_t* __restrict__ out_i2p,
                               const int4* __restrict__ in_results, float4* __restrict__ decreases,
@@ -355,10 +363,10 @@ __global__ void k_raygen_path(uint32_t* __restrict__ seeds, const wfpt_geometry*
             uint32_t seed = seeds[task];
             int4 res = in_results[task];
             if (res.x >= 0) {
-                float4 r0 = in_rays[2 * task + 0];
-                float4 r1 = in_rays[2 * task + 1];
+                float4 r0, r1;
+                load_ray(in_rays, task, r0, r1, wide);
                 f3 dir = mk(r1.x, r1.y, r1.z);
-                f3 nrm = unpack_normal(geoms, res.y, res.x, (uint32_t)res.w);
+                f3 nrm = unpack_normal<true>(geoms, res.y, res.x, (uint32_t)res.w);
                 f3 ff = faceforward(nrm, dir, nrm);
                 float ra = randf(seed);
                 float rb = randf(seed);
@@ -448,7 +456,7 @@ __global__ void k_reconstruct_smooth(const float4* __restrict__ rays, const int4
             float4 r0 = rays[2 * task + 0];
             float4 r1 = rays[2 * task + 1];
             f3 dir = mk(r1.x, r1.y, r1.z);
-            f3 nrm = unpack_normal(geoms, res.y, res.x, (uint32_t)res.w);
+            f3 nrm = unpack_normal<false>(geoms, res.y, res.x, (uint32_t)res.w);
             float t = __int_as_float(res.z);
             f3 hit = add(mk(r0.x, r0.y, r0.z), mul(dir, t));
             f3 L = normalize(sub(mk(lx, ly, lz), hit));
@@ -696,7 +704,8 @@ cudaError_t launch_raygen_path(uint32_t* seeds, const wfpt_geometry* geoms, cons
                               reinterpret_cast<float4*>(out_rays), in_i2p, out_i2p,
                               reinterpret_cast<const int4*>(in_res), reinterpret_cast<float4*>(decreases),
                               out_count, n, n_dev, albedo, reinterpret_cast<uint32_t*>(scratch),
-                              mo ? mo->keys : nullptr, mo ? mo->indices : nullptr, box, wide_rays(out_rays));
+                              mo ? mo->keys : nullptr, mo ? mo->indices : nullptr, box,
+                              wide_rays(in_rays) && wide_rays(out_rays));
     count_launch();
     return cudaGetLastError();
 }
@@ -835,7 +844,8 @@ cudaError_t launch_raygen_path_static(uint32_t* seeds, const wfpt_geometry* geom
     k_raygen_path<-1><<<grid, kBlock, 0, s>>>(
         seeds, geoms, reinterpret_cast<const float4*>(in_rays), reinterpret_cast<float4*>(out_rays), in_i2p,
         out_i2p, reinterpret_cast<const int4*>(in_res), reinterpret_cast<float4*>(decreases), out_count, n,
-        n_dev, albedo, scratch, nullptr, nullptr, Box6{}, wide_rays(out_rays));
+        n_dev, albedo, scratch, nullptr, nullptr, Box6{},
+        wide_rays(in_rays) && wide_rays(out_rays));
     count_launch();
     return cudaGetLastError();
 }
