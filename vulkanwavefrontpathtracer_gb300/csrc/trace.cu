@@ -319,7 +319,9 @@ __global__ void __launch_bounds__(BLOCK, PER_SM) k_trace_bvh2(const float4* __re
 // 1648 -> 1613 us) but 3-20 % slower on camera rays (2.07M: 632 -> 651 us, 262K:
 // 159 -> 192 us), whose sizes the host knows; asking for the next 32 rays
 // before tracing the current ones (which binds them to a warp that may be
-// slow) made those worse still (706 and 239 us).
+// slow) made those worse still (706 and 239 us).  Only for callers that bring
+// their own counters: the scene's are handed out in turn, and two replays of
+// one captured launch at a time would share a pair.
 constexpr int kBvh2PerSm = 5;
 constexpr unsigned kBvh2Grid = 152 * kBvh2PerSm;
 constexpr uint32_t kBvh2PersistentMin = 1u << 22;  // with a host-side count
@@ -1079,12 +1081,11 @@ cudaError_t launch_trace(const SceneDevice& sc, int kind, const wfpt_ray* rays, 
                                         g_postpone);
         }
     } else {
-        if (n >= (n_dev != nullptr ? kBvh2SmallMin : kBvh2PersistentMin)) {
-            uint32_t* work = own_work ? own_work : sc.work + 16 * (g_slot.fetch_add(1) % kWorkSlots);
+        if (own_work != nullptr && n >= (n_dev != nullptr ? kBvh2SmallMin : kBvh2PersistentMin)) {
             auto k2 = closest ? (g_count ? k_trace_bvh2_persistent<true, true> : k_trace_bvh2_persistent<true, false>)
                               : (g_count ? k_trace_bvh2_persistent<false, true> : k_trace_bvh2_persistent<false, false>);
             k2<<<std::min(grid, kBvh2Grid), kBlock, 0, s>>>(sc.bvh2_nodes, sc.bvh2_tris, rr, out, ray_index, n, n_dev,
-                                                            work);
+                                                            own_work);
         } else if (n >= kBvh2SmallMin) {
             constexpr int B = kBvh2SmallBlock, P = kBvh2SmallPerSm;
             auto k2 = closest ? (g_count ? k_trace_bvh2<true, true, B, P> : k_trace_bvh2<true, false, B, P>)
