@@ -48,6 +48,26 @@ constexpr uint32_t kLbValue = (1u << 30) - 1u;
 // warps' instructions as much as by the L2 round trip.
 constexpr int kLbChunk = 8;
 
+// Tiles of small sorts (393,216 pairs and less): 256 threads of 4 keys up to
+// 131,072 pairs, of 8 keys beyond.  Such a sort is a chain of latencies: a
+// pass of 65,536 pairs takes 4.3 us with 16 tiles or with 64, of which its
+// loads, rankings and stores are a fraction.  Smaller tiles shorten the part
+// that a tile does alone, and what can be asked for early is: the values are
+// loaded with the keys instead of when they are staged, the first tile's
+// digit counts too.  65,536 pairs, 63-bit keys 59.5 -> 45.0 us, 32-bit 31.1 ->
+// 24.5 us (the rate of its six launches); 8,192: 54.1 -> 35.3 us; 262,144:
+// 76 -> 63 us, with 4 keys 70; 400,000: 88 -> 79 us, 4 keys 88; 524,288: 94, 8
+// keys 109: look-backs over 250 tiles cost more than they save.  One resident
+// kernel for all passes (grid barriers instead of launches) 50.5 us at 65,536.
+constexpr int kTinyThreads = 256, kKptTiny = 4, kKptTinyLarge = 8;
+constexpr uint32_t kTinyMax = 1u << 17, kTinyLargeMax = 3u << 17;
+constexpr int kTinyCtasPerSm = 4;
+// These tiles are two to four times as many as the look-back tables of a pass
+// hold, so all passes use the space of all tables as one, and an entry carries
+// its pass (counts below 2^26): one of an earlier pass counts as unpublished.
+constexpr int kLbTagShift = 26;
+constexpr uint32_t kLbTagMask = 15u << kLbTagShift;
+
 // Keys per thread of the tile variants (tile = 512 * KPT keys).  The
 // extra-large variant serves sorts of more than two waves of large tiles:
 // 20 keys per thread for 32-bit keys (10 % faster than 16 on 2^26 keys).
@@ -144,16 +164,16 @@ static cudaError_t launch_dependent(Kernel kernel, unsigned grid, unsigned block
 // Histogram of every pass's digit over the first `count` keys: PASSES is a
 // template parameter so that the digit extraction unrolls into constant
 // byte selects; each thread issues the loads of 8 keys before their
-// shared-memory atomics.
-template <typename K, int PASSES>
+// shared-memory atomics.  AFTER_CLEAR: launched dependent on k_sort_clear.
+template <typename K, int PASSES, bool AFTER_CLEAR>
 __global__ void __launch_bounds__(kHistBlock) k_sort_hist(const K* __restrict__ keys, uint32_t n,
                                                            const uint32_t* __restrict__ n_dev, uint32_t top_mask,
                                                            uint32_t* __restrict__ hist) {
-    constexpr int U = 8;
+    constexpr int U = AFTER_CLEAR ? 4 : 8;
     __shared__ uint32_t s_h[PASSES * kRadix];
     // Every CTA of this grid has started: the first pass may launch its
     // CTAs into the slots this grid frees (they wait for its completion).
-    allow_dependent_launch();
+    if (!AFTER_CLEAR) allow_dependent_launch();
     for (int i = threadIdx.x; i < PASSES * kRadix; i += kHistBlock) s_h[i] = 0;
     __syncthreads();
     const uint32_t count = load_count(n, n_dev);
@@ -178,6 +198,10 @@ __global__ void __launch_bounds__(kHistBlock) k_sort_hist(const K* __restrict__ 
         }
     }
     __syncthreads();
+    if (AFTER_CLEAR) {
+        wait_for_previous_grid();
+        allow_dependent_launch();
+    }
     for (int i = threadIdx.x; i < PASSES * kRadix; i += kHistBlock) {
         uint32_t c = s_h[i];
         if (c) atomicAdd(&hist[i], c);
@@ -280,12 +304,46 @@ static void launch_hist(const K* keys, uint32_t n, const uint32_t* n_dev, int pa
     switch (passes) {
 #define WFPT_HIST(P)                                                                                   \
     case P:                                                                                            \
-        k_sort_hist<K, P><<<grid, kHistBlock, 0, s>>>(keys, n, n_dev, top, hist);                      \
+        k_sort_hist<K, P, false><<<grid, kHistBlock, 0, s>>>(keys, n, n_dev, top, hist);               \
         break;
         WFPT_HIST(1) WFPT_HIST(2) WFPT_HIST(3) WFPT_HIST(4) WFPT_HIST(5) WFPT_HIST(6) WFPT_HIST(7) WFPT_HIST(8)
 #undef WFPT_HIST
         default: break;
     }
+}
+
+// Zeroes the tickets, histograms and look-back entries of a small sort.  A
+// kernel rather than a memset, so that the histograms are counted while it
+// runs: k_sort_hist waits for it only before adding to the global ones (and
+// lets the first pass draw its tickets only then).  65,536 pairs 1 us faster,
+// 8,192 3 us.
+__global__ void __launch_bounds__(kHistBlock) k_sort_clear(uint32_t* __restrict__ p, uint32_t n) {
+    allow_dependent_launch();
+    for (uint32_t i = blockIdx.x * kHistBlock + threadIdx.x; i < n; i += gridDim.x * kHistBlock) p[i] = 0u;
+}
+
+// The clear and the histograms of a sort of tiny tiles.
+template <typename K>
+static cudaError_t launch_clear_hist(const K* keys, uint32_t n, const uint32_t* n_dev, int passes, int key_bits,
+                                     void* clear, size_t clear_bytes, uint32_t* hist, cudaStream_t s) {
+    const uint32_t top = pass_mask(key_bits, passes - 1), words = (uint32_t)(clear_bytes / 4);
+    k_sort_clear<<<std::min((words + kHistBlock - 1) / kHistBlock, 152u * 8), kHistBlock, 0, s>>>(
+        reinterpret_cast<uint32_t*>(clear), words);
+    count_launch();
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    const unsigned grid = (n + kHistBlock * 4 - 1) / (kHistBlock * 4);
+    switch (passes) {
+#define WFPT_HIST(P)                                                                                   \
+    case P:                                                                                            \
+        e = launch_dependent(k_sort_hist<K, P, true>, grid, kHistBlock, 0, s, keys, n, n_dev, top, hist); \
+        break;
+        WFPT_HIST(1) WFPT_HIST(2) WFPT_HIST(3) WFPT_HIST(4) WFPT_HIST(5) WFPT_HIST(6) WFPT_HIST(7) WFPT_HIST(8)
+#undef WFPT_HIST
+        default: break;
+    }
+    count_launch();
+    return e;
 }
 
 // Bulk prefetch into L2 of `count` keys and values (cp.async.bulk.prefetch:
@@ -301,18 +359,20 @@ __device__ __forceinline__ void prefetch_l2(const K* keys, const uint32_t* vals,
 
 // One tile of a digit pass (below).  FULL: the tile holds TILE keys, so
 // the per-key bounds checks of the last, partial tile drop out.
-template <typename K, int KPT, int DB, bool FULL>
+template <typename K, int KPT, int DB, int THREADS, bool FULL>
 __device__ __forceinline__ void onesweep_tile(const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
                                               K* __restrict__ keys_out, uint32_t* __restrict__ vals_out,
                                               uint32_t count, uint32_t tile, int shift, uint32_t dmask,
                                               const uint32_t* __restrict__ hist, uint32_t* __restrict__ lookback,
-                                              int nibble, unsigned char* smem, uint32_t* s_scan) {
-    constexpr uint32_t TILE = kSortThreads * KPT;
-    constexpr int kRadix = 1 << DB;
+                                              int nibble, uint32_t tag, unsigned char* smem, uint32_t* s_scan) {
+    constexpr uint32_t TILE = THREADS * KPT;
+    constexpr int WARPS = THREADS / 32;
+    constexpr bool TAGGED = THREADS == kTinyThreads;
+        constexpr int kRadix = 1 << DB;
     K* s_keys = reinterpret_cast<K*>(smem);
     uint32_t* s_vals = reinterpret_cast<uint32_t*>(s_keys + TILE);
     uint32_t* s_hist = s_vals + TILE;  // [warp][digit]
-    uint32_t* s_base = s_hist + kSortWarps * kRadix;
+    uint32_t* s_base = s_hist + WARPS * kRadix;
     uint32_t* s_loc = s_base + kRadix;
 
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -325,6 +385,15 @@ __device__ __forceinline__ void onesweep_tile(const K* __restrict__ keys_in, con
     for (int k = 0; k < KPT; ++k) {
         uint32_t i = base + k * 32;
         key[k] = (FULL || i < count) ? keys_in[i] : (K)0;
+    }
+    uint32_t val[TAGGED ? KPT : 1], first_cnt = 0;
+    if (TAGGED) {
+#pragma unroll
+        for (int k = 0; k < (TAGGED ? KPT : 0); ++k) {
+            uint32_t i = base + k * 32;
+            val[k] = (FULL || i < count) ? vals_in[i] : 0u;
+        }
+        if (tile == 0) first_cnt = hist[threadIdx.x & (kRadix - 1)];
     }
     uint32_t* my_hist = s_hist + warp * kRadix;
     // Warp-level stable ranking: keys are visited in input order (k, lane).
@@ -351,14 +420,14 @@ __device__ __forceinline__ void onesweep_tile(const K* __restrict__ keys_in, con
     uint32_t run = 0;
     if (owner) {
 #pragma unroll 8
-        for (int w = 0; w < kSortWarps; ++w) {
+        for (int w = 0; w < WARPS; ++w) {
             uint32_t c = s_hist[w * kRadix + d];
             s_hist[w * kRadix + d] = run;
             run += c;
         }
     }
     uint32_t tile_total;
-    const uint32_t loc = block_exclusive_scan<kSortWarps>(owner ? run : 0u, s_scan, &tile_total);
+    const uint32_t loc = block_exclusive_scan<WARPS>(owner ? run : 0u, s_scan, &tile_total);
     // Publish this tile's counts (tile 0: its inclusive prefix, from the
     // global histogram) before staging, so that successors can proceed.
     uint32_t excl = 0;
@@ -366,18 +435,18 @@ __device__ __forceinline__ void onesweep_tile(const K* __restrict__ keys_in, con
         uint32_t total, cnt_d = 0;
         if (owner) {
             if (DB == 8) {
-                cnt_d = hist[d];
+                cnt_d = TAGGED ? first_cnt : hist[d];
             } else {
 #pragma unroll
                 for (uint32_t j = 0; j < 16; ++j) cnt_d += hist[nibble ? ((d << 4) | j) : ((j << 4) | d)];
             }
         }
-        excl = block_exclusive_scan<kSortWarps>(cnt_d, s_scan, &total);
+        excl = block_exclusive_scan<WARPS>(cnt_d, s_scan, &total);
     }
     uint32_t* lb = lookback + (size_t)tile * kRadix + d;
     if (owner) {
         s_loc[d] = loc;
-        atomicExch(lb, tile == 0 ? (kLbPrefix | (excl + run)) : (kLbAggregate | run));
+        atomicExch(lb, tag | (tile == 0 ? (kLbPrefix | (excl + run)) : (kLbAggregate | run)));
     }
     __syncthreads();
 
@@ -390,7 +459,7 @@ __device__ __forceinline__ void onesweep_tile(const K* __restrict__ keys_in, con
             uint32_t dk = digit_of(key[k], shift, dmask);
             uint32_t pos = s_loc[dk] + my_hist[dk] + rank[k];
             s_keys[pos] = key[k];
-            s_vals[pos] = vals_in[i];
+            s_vals[pos] = TAGGED ? val[TAGGED ? k : 0] : vals_in[i];
         }
     }
 
@@ -406,7 +475,12 @@ __device__ __forceinline__ void onesweep_tile(const K* __restrict__ keys_in, con
 #pragma unroll
             for (int q = 0; q < kLbChunk; ++q)
                 st[q] = (j - q >= 0) ? *((volatile uint32_t*)(lookback + (size_t)(j - q) * kRadix + d))
-                                     : uint32_t(kLbPrefix);
+                                     : (tag | kLbPrefix);
+            // An entry of an earlier pass counts as not published.
+            if (TAGGED) {
+#pragma unroll
+                for (int q = 0; q < kLbChunk; ++q) st[q] = ((st[q] ^ tag) & kLbTagMask) != 0u ? 0u : st[q] ^ tag;
+            }
             // Fast path: every entry a published aggregate (flag bit 30 set
             // in all of them; a prefix has bit 31 alone, an unpublished entry
             // neither).  Their raw sum minus the flags is the sum of the
@@ -445,14 +519,14 @@ __device__ __forceinline__ void onesweep_tile(const K* __restrict__ keys_in, con
                 __nanosleep(32);
             }
         }
-        atomicExch(lb, kLbPrefix | (excl + run));
+        atomicExch(lb, tag | kLbPrefix | (excl + run));
     }
     if (owner) s_base[d] = excl - loc;
     __syncthreads();
 
     const uint32_t tile_count = FULL ? TILE : min(TILE, count - tile * TILE);
 #pragma unroll 2
-    for (uint32_t j = threadIdx.x; j < tile_count; j += kSortThreads) {
+    for (uint32_t j = threadIdx.x; j < tile_count; j += THREADS) {
         K kk = s_keys[j];
         uint32_t g = s_base[digit_of(kk, shift, dmask)] + j;
         if (g < count) {  // only fails after a look-back timeout
@@ -475,8 +549,10 @@ __device__ __forceinline__ void onesweep_tile(const K* __restrict__ keys_in, con
 // for the keys and values of tile t + lead (half the resident CTAs ahead:
 // the tile that starts about half a tile's lifetime later), so that a
 // tile's loads find their data in L2 instead of waiting on DRAM.
-template <typename K, int KPT, int DB>
-__global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm) k_onesweep(const K* __restrict__ keys_in,
+template <typename K, int KPT, int DB, int THREADS>
+__global__ void __launch_bounds__(THREADS, THREADS == kTinyThreads ? kTinyCtasPerSm
+                                                                  : kSortCtasPerSm) k_onesweep(
+                                                              const K* __restrict__ keys_in,
                                                               const uint32_t* __restrict__ vals_in,
                                                               K* __restrict__ keys_out,
                                                               uint32_t* __restrict__ vals_out, uint32_t n,
@@ -484,19 +560,20 @@ __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm) k_onesweep(const
                                                               uint32_t dmask, const uint32_t* __restrict__ hist,
                                                               uint32_t* __restrict__ lookback,
                                                               uint32_t* __restrict__ ticket, int nibble,
-                                                              uint32_t lead) {
-    constexpr uint32_t TILE = kSortThreads * KPT;
+                                                              uint32_t lead, uint32_t tag) {
+    constexpr uint32_t TILE = THREADS * KPT;
+    constexpr int WARPS = THREADS / 32;
     constexpr int kRadix = 1 << DB;
     extern __shared__ __align__(16) unsigned char smem[];
     uint32_t* s_hist = reinterpret_cast<uint32_t*>(smem + (size_t)TILE * (sizeof(K) + 4));
     __shared__ uint32_t s_tile;
-    __shared__ uint32_t s_scan[kSortWarps];
+    __shared__ uint32_t s_scan[WARPS];
 
     // Prologue that reads nothing the previous kernel writes (the tickets
     // and look-back states of this pass were cleared before the sort began).
     uint32_t t = 0;
     if (threadIdx.x == 0) t = atomicAdd(ticket, 1u);
-    for (int i = threadIdx.x; i < kSortWarps * kRadix; i += kSortThreads) s_hist[i] = 0;
+    for (int i = threadIdx.x; i < WARPS * kRadix; i += THREADS) s_hist[i] = 0;
     allow_dependent_launch();
     wait_for_previous_grid();
     const uint32_t count = load_count(n, n_dev);
@@ -511,11 +588,11 @@ __global__ void __launch_bounds__(kSortThreads, kSortCtasPerSm) k_onesweep(const
     const uint32_t tile = s_tile;
     if (tile >= ntiles) return;
     if ((size_t)(tile + 1) * TILE <= count)
-        onesweep_tile<K, KPT, DB, true>(keys_in, vals_in, keys_out, vals_out, count, tile, shift, dmask, hist,
-                                        lookback, nibble, smem, s_scan);
+        onesweep_tile<K, KPT, DB, THREADS, true>(keys_in, vals_in, keys_out, vals_out, count, tile, shift, dmask,
+                                                 hist, lookback, nibble, tag, smem, s_scan);
     else
-        onesweep_tile<K, KPT, DB, false>(keys_in, vals_in, keys_out, vals_out, count, tile, shift, dmask, hist,
-                                         lookback, nibble, smem, s_scan);
+        onesweep_tile<K, KPT, DB, THREADS, false>(keys_in, vals_in, keys_out, vals_out, count, tile, shift, dmask,
+                                                  hist, lookback, nibble, tag, smem, s_scan);
 }
 
 // After an odd number of passes: move the first `count` pairs back into the
@@ -532,14 +609,14 @@ __global__ void k_copy_back(const K* __restrict__ ks, const uint32_t* __restrict
 
 static inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-template <typename K, int KPT, int DB>
+template <typename K, int KPT, int DB, int THREADS = kSortThreads>
 static size_t onesweep_smem() {
-    return (size_t)kSortThreads * KPT * (sizeof(K) + 4) + (size_t)(kSortWarps + 2) * (1u << DB) * 4;
+    return (size_t)THREADS * KPT * (sizeof(K) + 4) + (size_t)(THREADS / 32 + 2) * (1u << DB) * 4;
 }
 
 template <typename K, int KPT, int DB>
 static cudaError_t opt_in_smem() {
-    return cudaFuncSetAttribute(k_onesweep<K, KPT, DB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    return cudaFuncSetAttribute(k_onesweep<K, KPT, DB, kSortThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)onesweep_smem<K, KPT, DB>());
 }
 
@@ -572,7 +649,8 @@ cudaError_t sort_prepare() {
 }
 
 // Tile variant: 0 = automatic, 1 = small, 2 = large, 3 = extra-large tiles
-// (64-bit keys: the large ones).  Automatic takes the small tiles while they
+// (64-bit keys: the large ones).  Automatic takes tiny tiles (tiny_kpt) for
+// small sorts, then the small tiles while they
 // fit in one wave (two tiles per SM), the large ones while those fit in two
 // waves (a frame-sized sort), and the extra-large ones beyond.
 static int g_sort_tiles = 0;
@@ -621,14 +699,27 @@ size_t sort_scratch_bytes(uint32_t max_n, int key_bits) {
     return sort_layout(max_n, key_bits).total;
 }
 
+// Keys per thread of a small sort's tiles; 0: the sort is not small, or its
+// look-back entries do not fit (fewer than four passes for 4 keys, two for 8).
+static int tiny_kpt(uint32_t n, const SortLayout& L) {
+    if (g_sort_tiles != 0 || g_digit_bits != 8 || n > kTinyLargeMax) return 0;
+    for (int kpt : {kKptTiny, kKptTinyLarge}) {
+        const size_t tile = (size_t)kTinyThreads * kpt;
+        if (kpt == kKptTiny && n > kTinyMax) continue;
+        if (((size_t)n + tile - 1) / tile <= (size_t)L.passes * L.tiles) return kpt;
+    }
+    return 0;
+}
+
 // The layout is sized for 8-bit digits; 4-bit digits take at most twice the
 // passes with 1/16 of the look-back entries per pass, and their global digit
 // counts come from the same byte histograms.
-template <typename K, int KPT, int DB>
+template <typename K, int KPT, int DB, int THREADS = kSortThreads>
 static cudaError_t sort_passes(K* keys, uint32_t* values, uint32_t n, const uint32_t* n_dev, int key_bits,
                                const SortLayout& L, unsigned char* scratch, cudaStream_t s) {
-    constexpr uint32_t TILE = kSortThreads * KPT;
+    constexpr uint32_t TILE = THREADS * KPT;
     constexpr uint32_t RADIX = 1u << DB;
+    constexpr bool TAGGED = THREADS == kTinyThreads;
     const int passes = (key_bits + DB - 1) / DB;
     uint32_t* tickets = reinterpret_cast<uint32_t*>(scratch + L.off_ticket);
     uint32_t* hist = reinterpret_cast<uint32_t*>(scratch + L.off_hist);
@@ -636,7 +727,7 @@ static cudaError_t sort_passes(K* keys, uint32_t* values, uint32_t n, const uint
     K* alt_keys = reinterpret_cast<K*>(scratch + L.off_keys);
     uint32_t* alt_vals = reinterpret_cast<uint32_t*>(scratch + L.off_vals);
     const uint32_t tiles = (n + TILE - 1) / TILE;
-    const size_t smem = onesweep_smem<K, KPT, DB>();
+    const size_t smem = onesweep_smem<K, KPT, DB, THREADS>();
     // Prefetch distance in tiles: half the CTAs resident at once (measured
     // 3/8 to 5/8 of them equally good at 2^24-2^26 pairs; a whole wave
     // ahead was 6 % slower, two waves slower than no prefetch).
@@ -648,10 +739,11 @@ static cudaError_t sort_passes(K* keys, uint32_t* values, uint32_t n, const uint
     uint32_t* dst_v = alt_vals;
     for (int p = 0; p < passes; ++p) {
         const int byte = DB == 8 ? p : p / 2;
-        e = launch_dependent(k_onesweep<K, KPT, DB>, tiles, kSortThreads, smem, s, (const K*)src_k,
+        e = launch_dependent(k_onesweep<K, KPT, DB, THREADS>, tiles, THREADS, smem, s, (const K*)src_k,
                              (const uint32_t*)src_v, dst_k, dst_v, n, n_dev, (int)(DB * p), pass_mask(key_bits, p, DB),
-                             (const uint32_t*)(hist + byte * kRadix), lookback + (size_t)p * L.tiles * RADIX,
-                             tickets + p, (int)(DB == 8 ? 0 : (p & 1)), lead);
+                             (const uint32_t*)(hist + byte * kRadix), TAGGED ? lookback : lookback + (size_t)p * L.tiles * RADIX,
+                             tickets + p, (int)(DB == 8 ? 0 : (p & 1)), lead,
+                             TAGGED ? (uint32_t)(p + 1) << kLbTagShift : 0u);
         count_launch();
         if (e != cudaSuccess || (e = cudaGetLastError()) != cudaSuccess) return e;
         std::swap(src_k, dst_k);
@@ -666,12 +758,27 @@ static cudaError_t sort_passes(K* keys, uint32_t* values, uint32_t n, const uint
     return cudaSuccess;
 }
 
+// The clear, the histograms and the passes of a sort of tiny tiles.
+template <typename K, int KPT>
+static cudaError_t sort_tiny(K* keys, uint32_t* values, uint32_t n, const uint32_t* n_dev, int key_bits,
+                             const SortLayout& L, unsigned char* scratch, cudaStream_t s) {
+    const size_t tile = (size_t)kTinyThreads * KPT;
+    const size_t used = L.off_lookback + ((size_t)n + tile - 1) / tile * kRadix * 4;
+    cudaError_t e = launch_clear_hist<K>(keys, n, n_dev, L.passes, key_bits, scratch, used,
+                                         reinterpret_cast<uint32_t*>(scratch + L.off_hist), s);
+    if (e != cudaSuccess) return e;
+    return sort_passes<K, KPT, 8, kTinyThreads>(keys, values, n, n_dev, key_bits, L, scratch, s);
+}
+
 template <typename K>
 static cudaError_t sort_impl(K* keys, uint32_t* values, uint32_t n, const uint32_t* n_dev, int key_bits,
                              unsigned char* scratch, cudaStream_t s) {
     SortLayout L = sort_layout(n, key_bits);
     cudaError_t e;
     if ((e = sort_prepare()) != cudaSuccess) return e;
+    const int tiny = tiny_kpt(n, L);
+    if (tiny == kKptTiny) return sort_tiny<K, kKptTiny>(keys, values, n, n_dev, key_bits, L, scratch, s);
+    if (tiny == kKptTinyLarge) return sort_tiny<K, kKptTinyLarge>(keys, values, n, n_dev, key_bits, L, scratch, s);
     // Tickets, histograms and look-back states start at zero.
     if ((e = cudaMemsetAsync(scratch, 0, L.off_keys, s)) != cudaSuccess) return e;
     uint32_t* hist = reinterpret_cast<uint32_t*>(scratch + L.off_hist);
@@ -719,8 +826,8 @@ cudaError_t sort_selftest_timeout(cudaStream_t s) {
     e = cudaMemsetAsync(buf, 0, words * sizeof(uint32_t), s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(ticket, &one, sizeof(one), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
-        k_onesweep<uint32_t, KPT, 8><<<1, kSortThreads, onesweep_smem<uint32_t, KPT, 8>(), s>>>(
-            keys, vals, keys_out, vals_out, N, nullptr, 0, 0xFFu, hist, lookback, ticket, 0, 0u);
+        k_onesweep<uint32_t, KPT, 8, kSortThreads><<<1, kSortThreads, onesweep_smem<uint32_t, KPT, 8>(), s>>>(
+            keys, vals, keys_out, vals_out, N, nullptr, 0, 0xFFu, hist, lookback, ticket, 0, 0u, 0u);
         count_launch();
         e = cudaGetLastError();
     }
