@@ -144,7 +144,7 @@ struct wfpt_renderer {
     };
     std::vector<ShadowSlot> slots;
     DevBuf aux2;
-    cudaEvent_t ev_fork = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_shade = nullptr;
     int pending_slots = 0;  // slots the next shadow pass (or the frame's end) waits for
     int last_slots = 0;     // slots used by the last frame
     RayBufferDev primary, shadow, queue[2];
@@ -279,6 +279,7 @@ struct wfpt_renderer {
             sl.scratch.release();
         }
         if (ev_fork) cudaEventDestroy(ev_fork);
+        if (ev_shade) cudaEventDestroy(ev_shade);
         for (auto* b : {&i2p, &p2i, &seeds, &decreases, &aux, &sort_scratch, &path_scratch, &counters, &work, &aux2})
             b->release();
         primary.release();
@@ -409,7 +410,7 @@ struct wfpt_renderer {
         if (sequential_shadow && (e = shadow.ensure(shadow_cap, true)) != cudaSuccess) return e;
         size_t sort_n = std::max(n, sequential_shadow ? shadow_cap : (size_t)0);
         if ((e = sort_scratch.ensure(wfpt::sort_scratch_bytes((uint32_t)sort_n, 64))) != cudaSuccess) return e;
-        if ((e = path_scratch.ensure(wfpt::raygen_path_scratch_bytes((uint32_t)n))) != cudaSuccess) return e;
+        if ((e = path_scratch.ensure(kMaxDepth * wfpt::raygen_path_scratch_bytes((uint32_t)n))) != cudaSuccess) return e;
         if ((e = counters.ensure((size_t)kMaxSamples * kCountersPerPass * 4)) != cudaSuccess) return e;
         if (cfg.accumulate_fp64 && (e = accum64.ensure(n * 32)) != cudaSuccess) return e;
         if (!work.p) {
@@ -418,7 +419,8 @@ struct wfpt_renderer {
         }
         if (cfg.shadow_overlap) {
             if ((e = aux2.ensure(n * 16)) != cudaSuccess) return e;
-            if (!ev_fork && (e = cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming)) != cudaSuccess) return e;
+            for (cudaEvent_t* ev : {&ev_fork, &ev_shade})
+                if (!*ev && (e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming)) != cudaSuccess) return e;
             const int want = plan_slots(n, S, shadow_cap);
             if ((int)slots.size() < want) slots.resize(want);
             for (int k = 0; k < want; ++k) {
@@ -509,24 +511,28 @@ struct wfpt_renderer {
     // whose slot->pixel map is `in_s2i`; n_in is the capacity, n_in_dev the
     // device-side count (null when the host count is exact).  Batches of
     // batch_diff input rays, as the reference cuts them.
+    // shade() launches, on s, the reconstructSmooth that writes in_pixels.
     //  - Overlapped (cfg.shadow_overlap, not timed): batch b is generated,
     //    traced and reconstructed on the stream of slot b % nslots, forked
-    //    from s; s waits for the last batch generated on every slot before it
-    //    goes on (raygenShadow reads the seeds that the next raygenPath
-    //    rewrites), and join_shadow() makes the next shadow pass wait for
-    //    all of them, which keeps the order of the additions into
-    //    out_pixels.  A slot's batches run in order on its stream, so a
-    //    slot's buffers are reused only after its previous batch is done.
+    //    from s before shade(), which shadow rays do not need; the
+    //    reconstructions wait for it and, by join_shadow(), for the previous
+    //    shadow pass, which keeps the order of the additions into
+    //    out_pixels.  s waits for the last batch generated on every slot
+    //    before it goes on (raygenShadow reads the seeds that the next
+    //    raygenPath rewrites).  A slot's batches run in order on its stream,
+    //    so a slot's buffers are reused only after its previous batch is done.
     //  - Sequential: every batch on s, in the reference's order.
-    cudaError_t shadow_pass(const wfpt_ray* in_rays, const wfpt_hit* in_res, const int32_t* in_s2i, uint32_t n_in,
+    template <typename Shade>
+    cudaError_t shadow_pass(Shade&& shade, const wfpt_ray* in_rays, const wfpt_hit* in_res, const int32_t* in_s2i, uint32_t n_in,
                             const uint32_t* n_in_dev, float* in_pixels, float* out_pixels,
                             uint32_t* batch_counters, cudaStream_t s, int kind, int slot_log) {
         const int S = cfg.num_shadow_samples;
         const uint32_t batch_diff = (uint32_t)(kMaxBatch / S);
         cudaError_t e;
-        if ((e = join_shadow(s)) != cudaSuccess) return e;
         if (cfg.shadow_overlap && !timing_on && nslots >= 1 && (int)slots.size() >= nslots) {
             if ((e = cudaEventRecord(ev_fork, s)) != cudaSuccess) return e;
+            if ((e = shade()) != cudaSuccess || (e = join_shadow(s)) != cudaSuccess) return e;
+            if ((e = cudaEventRecord(ev_shade, s)) != cudaSuccess) return e;
             const uint32_t nb = (n_in + batch_diff - 1) / batch_diff;
             const int used = (int)std::min<uint32_t>((uint32_t)nslots, std::max(nb, 1u));
             for (int k = 0; k < used; ++k)
@@ -535,22 +541,18 @@ struct wfpt_renderer {
                 ShadowSlot& sl = slots[b % used];
                 const cudaStream_t ss = sl.stream;
                 const uint32_t bb = b * batch_diff, bs = std::min(batch_diff, n_in - bb);
-                const uint32_t* n_sh_dev = nullptr;
-                if (n_in_dev) {
-                    uint32_t* bc = batch_counters + (b % used);
-                    if ((e = wfpt::launch_batch_count(n_in_dev, bb, bs, S, bc, ss)) != cudaSuccess) return e;
-                    n_sh_dev = bc;
-                }
+                uint32_t* n_sh_dev = n_in_dev ? batch_counters + (b % used) : nullptr;
                 sl.rb.swapped = false;
                 if ((e = wfpt::launch_raygen_shadow(seeds.as<uint32_t>(), in_rays, in_res, sl.rb.rays_cur(),
                                                     sl.rb.s2i_cur(), sl.rb.i2s_cur(), light, cfg.shadow_radius,
-                                                    (int)bb, (int)bs, n_in_dev, S, ss)) != cudaSuccess)
+                                                    (int)bb, (int)bs, n_in_dev, S, ss, n_sh_dev)) != cudaSuccess)
                     return e;
                 if ((e = cudaEventRecord(sl.ev_rg, ss)) != cudaSuccess) return e;
                 if ((e = trace_rays(sl.rb, bs * (uint32_t)S, n_sh_dev, cfg.sort_shadow_rays != 0,
                                     cfg.reorder_shadow_rays != 0, false, ss, sl.work.as<uint32_t>(), sl.scratch,
                                     kind)) != cudaSuccess)
                     return e;
+                if (b < (uint32_t)used && (e = cudaStreamWaitEvent(ss, ev_shade, 0)) != cudaSuccess) return e;
                 if ((e = wfpt::launch_reconstruct_shadow(sl.rb.results.as<wfpt_hit>(), in_s2i, sl.rb.i2s_cur(),
                                                          in_pixels, out_pixels, (int)bb, (int)bs, n_in_dev, S, 0,
                                                          ss)) != cudaSuccess)
@@ -564,20 +566,17 @@ struct wfpt_renderer {
             last_slots = std::max(last_slots, used);
             return cudaSuccess;
         }
+        if ((e = shade()) != cudaSuccess || (e = join_shadow(s)) != cudaSuccess) return e;
+        uint32_t* n_sh_dev = n_in_dev ? batch_counters : nullptr;
         uint32_t bb = 0;
         do {
             uint32_t be = std::min(bb + batch_diff, n_in);
             uint32_t bs = be - bb;
-            const uint32_t* n_sh_dev = nullptr;
-            if (n_in_dev) {
-                if ((e = wfpt::launch_batch_count(n_in_dev, bb, bs, S, batch_counters, s)) != cudaSuccess) return e;
-                n_sh_dev = batch_counters;
-            }
             shadow.swapped = false;
             if ((e = timed(s, T_SHADOW, C_NONE, -1, [&]() {
                      return wfpt::launch_raygen_shadow(seeds.as<uint32_t>(), in_rays, in_res, shadow.rays_cur(),
                                                        shadow.s2i_cur(), shadow.i2s_cur(), light, cfg.shadow_radius,
-                                                       (int)bb, (int)bs, n_in_dev, S, s);
+                                                       (int)bb, (int)bs, n_in_dev, S, s, n_sh_dev);
                  })) != cudaSuccess)
                 return e;
             if ((e = trace_rays(shadow, bs * (uint32_t)S, n_sh_dev, cfg.sort_shadow_rays != 0,
@@ -594,31 +593,28 @@ struct wfpt_renderer {
         return cudaSuccess;
     }
 
-    // Renderer::primaryPass (Renderer.cpp:124-131).
+    // Renderer::primaryPass (Renderer.cpp:124-131): the camera rays and their
+    // shading.
     // hit_counter (nullable): receives the number of primary hits (the
     // shadow pass's input count, countRayHits) from reconstructSmooth.
     // fresh: target is this pass's colour buffer, taken as cleared (its
     // pixels are written, not accumulated); otherwise reconstructSmooth adds
     // into it (the frame buffer of the primary-rays mode, over the samples).
-    cudaError_t primary_pass(const float* s2w, const float* eye, float zfar, int pass, float* target, cudaStream_t s,
-                             const wfpt::FrameParams* fp, uint32_t* hit_counter, bool fresh) {
+    cudaError_t primary_trace(const float* s2w, const float* eye, float zfar, int pass, cudaStream_t s,
+                              const wfpt::FrameParams* fp) {
         uint32_t n = (uint32_t)width * height;
-        cudaError_t e;
         int sample_index = pass + cfg.num_primary_samples * (frame_index - 1);
-        if ((e = timed(s, T_PRIMARY, C_NONE, -1, [&]() {
-                 cudaError_t r = wfpt::launch_raygen_primary(s2w, i2p.as<int32_t>(), primary.rays_cur(), eye,
-                                                             sample_index, width, height, zfar, s, fp, pass,
-                                                             cfg.num_primary_samples);
-                 if (r != cudaSuccess) return r;
-                 return wfpt::launch_trace(*wfpt::scene_device(scene), primary_kind(), primary.rays_cur(),
-                                           primary.results.as<wfpt_hit>(), nullptr, n, nullptr, 1, s,
-                                           work.as<uint32_t>(), gpu_shared);
-             })) != cudaSuccess)
-            return e;
-        const float one = 1.0f;
-        uint32_t one_bits;
-        std::memcpy(&one_bits, &one, 4);
-        if ((e = wfpt::launch_fill_u32(decreases.p, one_bits, (size_t)n * 4, s)) != cudaSuccess) return e;
+        return timed(s, T_PRIMARY, C_NONE, -1, [&]() {
+            cudaError_t r = wfpt::launch_raygen_primary(s2w, i2p.as<int32_t>(), primary.rays_cur(), eye, sample_index,
+                                                        width, height, zfar, s, fp, pass, cfg.num_primary_samples);
+            if (r != cudaSuccess) return r;
+            return wfpt::launch_trace(*wfpt::scene_device(scene), primary_kind(), primary.rays_cur(),
+                                      primary.results.as<wfpt_hit>(), nullptr, n, nullptr, 1, s, work.as<uint32_t>(),
+                                      gpu_shared);
+        });
+    }
+    cudaError_t primary_shade(float* target, cudaStream_t s, uint32_t* hit_counter, bool fresh) {
+        uint32_t n = (uint32_t)width * height;
         return wfpt::launch_reconstruct_smooth(primary.rays_cur(), primary.results.as<wfpt_hit>(), i2p.as<int32_t>(),
                                                target, decreases.as<float>(), geoms, light, bg, n, nullptr,
                                                cfg.num_primary_samples, s, hit_counter, fresh);
@@ -637,16 +633,21 @@ struct wfpt_renderer {
         spans.clear();
         last_slots = 0;
         primary.swapped = queue[0].swapped = queue[1].swapped = shadow.swapped = false;
-        if ((e = cudaMemsetAsync(frame_pixels, 0, (size_t)n * 16, s)) != cudaSuccess) return e;
-        if ((e = cudaMemsetAsync(counters.p, 0, (size_t)cfg.num_primary_samples * kCountersPerPass * 4, s)) !=
-            cudaSuccess)
-            return e;
         int rt = cfg.ray_type;
-        if (rt == WFPT_PATH_RAYS || rt == WFPT_SHADOW_RAYS)
-            if ((e = wfpt::launch_init_seeds(seeds.as<uint32_t>(), n, frame_index, s, fp)) != cudaSuccess) return e;
+        const size_t path_bytes = wfpt::raygen_path_scratch_bytes(n);  // one bounce's
         for (int pass = 0; pass < cfg.num_primary_samples; ++pass) {
+            const bool first = pass == 0;
+            if ((e = wfpt::launch_begin_pass(first && rt != WFPT_PRIMARY_RAYS ? seeds.as<uint32_t>() : nullptr,
+                                             first ? frame_pixels : nullptr, n, frame_index, fp,
+                                             decreases.as<float>(), counters.as<uint32_t>(),
+                                             first ? (uint32_t)(cfg.num_primary_samples * kCountersPerPass) : 0u,
+                                             path_scratch.as<uint32_t>(),
+                                             rt == WFPT_PATH_RAYS ? (uint32_t)(cfg.recursion_depth * path_bytes / 4) : 0u,
+                                             s)) != cudaSuccess)
+                return e;
             if (rt == WFPT_PRIMARY_RAYS) {
-                if ((e = primary_pass(s2w, eye, zfar, pass, frame_pixels, s, fp, nullptr, false)) != cudaSuccess)
+                if ((e = primary_trace(s2w, eye, zfar, pass, s, fp)) != cudaSuccess ||
+                    (e = primary_shade(frame_pixels, s, nullptr, false)) != cudaSuccess)
                     return e;
                 continue;
             }
@@ -659,10 +660,9 @@ struct wfpt_renderer {
             // The colour buffers are not cleared (Renderer.cpp clears them per
             // pass): every pixel the shadow pass reads back was written by
             // this pass's reconstructSmooth in fresh mode.
-            if ((e = primary_pass(s2w, eye, zfar, pass, auxb[ai], s, fp, cnt(pass, kCntHits + 0), true)) !=
-                cudaSuccess)
-                return e;
-            if ((e = shadow_pass(primary.rays_cur(), primary.results.as<wfpt_hit>(), i2p.as<int32_t>(), n, nullptr,
+            if ((e = primary_trace(s2w, eye, zfar, pass, s, fp)) != cudaSuccess) return e;
+            auto shade = [&]() { return primary_shade(auxb[ai], s, cnt(pass, kCntHits + 0), true); };
+            if ((e = shadow_pass(shade, primary.rays_cur(), primary.results.as<wfpt_hit>(), i2p.as<int32_t>(), n, nullptr,
                                  auxb[ai], frame_pixels, cnt(pass, kCntBatch), s, primary_kind(), 0)) != cudaSuccess)
                 return e;
             if (rt != WFPT_PATH_RAYS) continue;
@@ -708,20 +708,22 @@ struct wfpt_renderer {
                 if ((e = timed(s, T_PATH, C_NONE, -1, [&]() {
                          return wfpt::launch_raygen_path(seeds.as<uint32_t>(), geoms, in_rays, out.rays_cur(), in_s2i,
                                                          out.s2i_cur(), in_res, decreases.as<float>(), out_cnt, n,
-                                                         in_cnt, cfg.albedo, path_scratch.p, s,
-                                                         fused_keys ? &mo : nullptr);
+                                                         in_cnt, cfg.albedo,
+                                                         path_scratch.as<unsigned char>() + bounce * path_bytes, s,
+                                                         fused_keys ? &mo : nullptr, true);
                      })) != cudaSuccess)
                     return e;
                 if ((e = trace_rays(out, n, out_cnt, sort_b, sort_b && cfg.reorder_path_rays != 0, true, s,
                                     work.as<uint32_t>(), sort_scratch, cfg.bvh_kind, T_PATH, 100 + bounce,
                                     fused_keys)) != cudaSuccess)
                     return e;
-                if ((e = wfpt::launch_reconstruct_smooth(out.rays_cur(), out.results.as<wfpt_hit>(), out.s2i_cur(),
-                                                         auxb[ai], decreases.as<float>(), geoms, light, bg, n,
-                                                         out_cnt, cfg.num_primary_samples, s,
-                                                         cnt(pass, kCntHits + bounce + 1), true)) != cudaSuccess)
-                    return e;
-                if ((e = shadow_pass(out.rays_cur(), out.results.as<wfpt_hit>(), out.s2i_cur(), n, out_cnt,
+                auto shade_bounce = [&]() {
+                    return wfpt::launch_reconstruct_smooth(out.rays_cur(), out.results.as<wfpt_hit>(), out.s2i_cur(),
+                                                           auxb[ai], decreases.as<float>(), geoms, light, bg, n,
+                                                           out_cnt, cfg.num_primary_samples, s,
+                                                           cnt(pass, kCntHits + bounce + 1), true);
+                };
+                if ((e = shadow_pass(shade_bounce, out.rays_cur(), out.results.as<wfpt_hit>(), out.s2i_cur(), n, out_cnt,
                                      auxb[ai], frame_pixels, cnt(pass, kCntBatch), s, cfg.bvh_kind, bounce + 1)) !=
                     cudaSuccess)
                     return e;

@@ -55,6 +55,24 @@ __global__ void k_init_seeds(uint32_t* __restrict__ seeds, uint32_t n, uint32_t 
     if (i < n) seeds[i] = tea(i, frame, 16);
 }
 
+// What a renderer's pass starts from, in one launch (six before: at 256x256
+// each is a node of 2-3 us on the frame's critical path): the seeds, the frame
+// buffer and the counters (a frame's first pass; null later), the path weights,
+// and the tile states of every bounce's path generation.
+__global__ void k_begin_pass(uint32_t* __restrict__ seeds, float4* __restrict__ pixels, uint32_t n, uint32_t frame,
+                             const FrameParams* __restrict__ fp, float4* __restrict__ decreases,
+                             uint32_t* __restrict__ counters, uint32_t num_counters, uint32_t* __restrict__ states,
+                             uint32_t num_states) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, threads = gridDim.x * blockDim.x;
+    for (uint32_t k = i; k < num_counters; k += threads) counters[k] = 0u;
+    for (uint32_t k = i; k < num_states; k += threads) states[k] = 0u;
+    if (i >= n) return;
+    if (fp) frame = (uint32_t)fp->frame_index;
+    if (seeds) seeds[i] = tea(i, frame, 16);
+    if (pixels) pixels[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    decreases[i] = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+}
+
 // ------------------------------------------------------------- primary
 // raygenPrimary.comp:11-22 (radical inverse in float, same operation order).
 __device__ __forceinline__ float halton(int i, int base) {
@@ -162,12 +180,14 @@ __global__ void k_raygen_shadow(const uint32_t* __restrict__ seeds,
                                 const int4* __restrict__ in_results, float4* __restrict__ out_rays,
                                 int32_t* __restrict__ out_s2i, int32_t* __restrict__ out_i2s,
                                 float lx, float ly, float lz, float radius, int batch_begin,
-                                int batch_size, const uint32_t* __restrict__ n_in_dev, int S, bool wide) {
+                                int batch_size, const uint32_t* __restrict__ n_in_dev, int S, bool wide,
+                                uint32_t* __restrict__ out_count) {
     int size = batch_size;
     if (n_in_dev != nullptr) {
         int avail = (int)*n_in_dev - batch_begin;
         if (avail < size) size = avail;
     }
+    if (out_count != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *out_count = (uint32_t)S * (uint32_t)max(size, 0);
     for (uint32_t task = blockIdx.x * blockDim.x + threadIdx.x; (int64_t)task < size;
          task = next_task<LOOP>(task)) {
         uint32_t seed = seeds[task];
@@ -322,7 +342,7 @@ __device__ uint32_t tile_prefix(uint32_t* tile_state, uint32_t tile, uint32_t co
 }
 
 // raygenPath.comp:95-167.  scratch[0] = tile ticket, scratch[1..] = tile
-// states; both zeroed by the host before the launch.  MK >= 0: also writes
+// states; both zeroed before the launch.  MK >= 0: also writes
 // the Morton key of kind MK of every output ray and its index (keys[dst],
 // key_idx[dst] = dst), which the Morton kernel would otherwise compute
 // from the written rays.
@@ -612,13 +632,6 @@ __global__ void k_interpolate_colors_fp64(float4* __restrict__ frame_pixels, flo
 }
 
 // Device-side size of one shadow batch: S * clamp(n_in - begin, 0, size).
-__global__ void k_batch_count(const uint32_t* __restrict__ n_in_dev, uint32_t begin, uint32_t size, uint32_t S,
-                              uint32_t* __restrict__ out) {
-    uint32_t n_in = *n_in_dev;
-    uint32_t avail = n_in > begin ? n_in - begin : 0u;
-    *out = S * (avail < size ? avail : size);
-}
-
 __global__ void k_fill_u32(uint32_t* __restrict__ dst, uint32_t v, size_t n) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -650,6 +663,17 @@ cudaError_t launch_init_seeds(uint32_t* seeds, uint32_t n, int frame, cudaStream
     return cudaGetLastError();
 }
 
+cudaError_t launch_begin_pass(uint32_t* seeds, float* pixels, uint32_t n, int frame, const FrameParams* fp,
+                              float* decreases, uint32_t* counters, uint32_t num_counters, uint32_t* states,
+                              uint32_t num_states, cudaStream_t s) {
+    if (n == 0) return cudaSuccess;
+    k_begin_pass<<<grid_for(n), kBlock, 0, s>>>(seeds, reinterpret_cast<float4*>(pixels), n, (uint32_t)frame, fp,
+                                                reinterpret_cast<float4*>(decreases), counters, num_counters, states,
+                                                num_states);
+    count_launch();
+    return cudaGetLastError();
+}
+
 cudaError_t launch_raygen_primary(const float* m, const int32_t* i2p, wfpt_ray* rays, const float* o,
                                   int sample_index, int w, int h, float max_dist, cudaStream_t s,
                                   const FrameParams* fp, int pass, int spp) {
@@ -668,13 +692,13 @@ cudaError_t launch_raygen_primary(const float* m, const int32_t* i2p, wfpt_ray* 
 cudaError_t launch_raygen_shadow(const uint32_t* seeds, const wfpt_ray* in_rays, const wfpt_hit* in_res,
                                  wfpt_ray* out_rays, int32_t* s2i, int32_t* i2s, const float* light,
                                  float radius, int bb, int bs, const uint32_t* n_in_dev, int S,
-                                 cudaStream_t s) {
+                                 cudaStream_t s, uint32_t* out_count) {
     if (bs <= 0) return cudaSuccess;
     auto k = capped((uint64_t)bs, n_in_dev) ? k_raygen_shadow<true> : k_raygen_shadow<false>;
     k<<<grid_for((uint64_t)bs, n_in_dev), kBlock, 0, s>>>(
         seeds, reinterpret_cast<const float4*>(in_rays), reinterpret_cast<const int4*>(in_res),
         reinterpret_cast<float4*>(out_rays), s2i, i2s, light[0], light[1], light[2], radius, bb, bs,
-        n_in_dev, S, wide_rays(out_rays));
+        n_in_dev, S, wide_rays(out_rays), out_count);
     count_launch();
     return cudaGetLastError();
 }
@@ -688,10 +712,12 @@ cudaError_t launch_raygen_path(uint32_t* seeds, const wfpt_geometry* geoms, cons
                                wfpt_ray* out_rays, const int32_t* in_i2p, int32_t* out_i2p,
                                const wfpt_hit* in_res, float* decreases, uint32_t* out_count,
                                uint32_t n, const uint32_t* n_dev, float albedo, void* scratch,
-                               cudaStream_t s, const MortonOut* mo) {
+                               cudaStream_t s, const MortonOut* mo, bool cleared) {
     size_t tiles = ((size_t)n + kBlock - 1) / kBlock;
-    cudaError_t e = cudaMemsetAsync(scratch, 0, (1 + tiles) * sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
+    if (!cleared) {
+        cudaError_t e = cudaMemsetAsync(scratch, 0, (1 + tiles) * sizeof(uint32_t), s);
+        if (e != cudaSuccess) return e;
+    }
     unsigned grid = tiles == 0 ? 1u : grid_for(n, n_dev);
     const Box6 box = mo ? mo->box : Box6{};
     auto k = k_raygen_path<-1>;
@@ -903,13 +929,6 @@ cudaError_t launch_interpolate_colors_fp64(float* frame_pixels, float* pixels, d
                                                              reinterpret_cast<float4*>(pixels),
                                                              reinterpret_cast<double4_32a*>(accum), n, frame_index, key,
                                                              white, fp);
-    count_launch();
-    return cudaGetLastError();
-}
-
-cudaError_t launch_batch_count(const uint32_t* n_in_dev, uint32_t begin, uint32_t size, int S, uint32_t* out,
-                               cudaStream_t s) {
-    k_batch_count<<<1, 1, 0, s>>>(n_in_dev, begin, size, (uint32_t)S, out);
     count_launch();
     return cudaGetLastError();
 }

@@ -53,18 +53,24 @@ cudaError_t launch_init_seeds(uint32_t* seeds, uint32_t n, int frame, cudaStream
 cudaError_t launch_raygen_primary(const float* m, const int32_t* i2p, wfpt_ray* rays, const float* o,
                                   int sample_index, int w, int h, float max_dist, cudaStream_t s,
                                   const FrameParams* fp = nullptr, int pass = 0, int spp = 1);
+// States (also counters, seeds, pixels: nullable) that a renderer's pass needs cleared.
+cudaError_t launch_begin_pass(uint32_t* seeds, float* pixels, uint32_t n, int frame, const FrameParams* fp,
+                              float* decreases, uint32_t* counters, uint32_t num_counters, uint32_t* states,
+                              uint32_t num_states, cudaStream_t s);
+// out_count (nullable): receives the number of rays written.
 cudaError_t launch_raygen_shadow(const uint32_t* seeds, const wfpt_ray* in_rays, const wfpt_hit* in_res,
                                  wfpt_ray* out_rays, int32_t* s2i, int32_t* i2s, const float* light,
                                  float radius, int bb, int bs, const uint32_t* n_in_dev, int S,
-                                 cudaStream_t s);
+                                 cudaStream_t s, uint32_t* out_count = nullptr);
 size_t raygen_path_scratch_bytes(uint32_t max_n);
 // mo (nullable): also the Morton keys of the output rays (what
-// launch_morton over out_rays and *out_count would write).
+// launch_morton over out_rays and *out_count would write).  cleared: the
+// scratch has been zeroed already.
 cudaError_t launch_raygen_path(uint32_t* seeds, const wfpt_geometry* geoms, const wfpt_ray* in_rays,
                                wfpt_ray* out_rays, const int32_t* in_i2p, int32_t* out_i2p,
                                const wfpt_hit* in_res, float* decreases, uint32_t* out_count,
                                uint32_t n, const uint32_t* n_dev, float albedo, void* scratch,
-                               cudaStream_t s, const MortonOut* mo = nullptr);
+                               cudaStream_t s, const MortonOut* mo = nullptr, bool cleared = false);
 // launch_raygen_path over the library's static scratch (n at most
 // WFPT_RAYGEN_PATH_STATIC_MAX_RAYS); calls on one device must not overlap.
 cudaError_t launch_raygen_path_static(uint32_t* seeds, const wfpt_geometry* geoms, const wfpt_ray* in_rays,
@@ -96,8 +102,6 @@ cudaError_t host_malloc(void** p, size_t bytes);
 uint64_t alloc_count();
 cudaError_t sort_prepare();
 cudaError_t launch_fill_u32(void* dst, uint32_t v, size_t n, cudaStream_t s);
-cudaError_t launch_batch_count(const uint32_t* n_in_dev, uint32_t begin, uint32_t size, int S, uint32_t* out,
-                               cudaStream_t s);
 
 // keys.cu
 cudaError_t launch_morton(const wfpt_ray* rays, uint32_t n, const uint32_t* n_dev, const float* smin,
