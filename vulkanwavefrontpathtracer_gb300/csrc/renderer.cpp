@@ -511,16 +511,20 @@ struct wfpt_renderer {
     // whose slot->pixel map is `in_s2i`; n_in is the capacity, n_in_dev the
     // device-side count (null when the host count is exact).  Batches of
     // batch_diff input rays, as the reference cuts them.
-    // shade() launches, on s, the reconstructSmooth that writes in_pixels.
+    // shade(false) launches, on s, the reconstructSmooth that writes in_pixels;
+    // shade(true) may launch it together with the next raygenPath, which
+    // rewrites the seeds that raygenShadow reads.
     //  - Overlapped (cfg.shadow_overlap, not timed): batch b is generated,
     //    traced and reconstructed on the stream of slot b % nslots, forked
-    //    from s before shade(), which shadow rays do not need; the
+    //    from s before the shading, which shadow rays do not need; the
     //    reconstructions wait for it and, by join_shadow(), for the previous
     //    shadow pass, which keeps the order of the additions into
-    //    out_pixels.  s waits for the last batch generated on every slot
-    //    before it goes on (raygenShadow reads the seeds that the next
-    //    raygenPath rewrites).  A slot's batches run in order on its stream,
-    //    so a slot's buffers are reused only after its previous batch is done.
+    //    out_pixels.  With a slot for every batch, s waits for the generation
+    //    of all batches and then shades (true); with fewer it shades (false)
+    //    at once, as a slot's next batch waits behind a reconstruction, and
+    //    waits for the generations afterwards.  A slot's batches run in order
+    //    on its stream, so a slot's buffers are reused only after its previous
+    //    batch is done.
     //  - Sequential: every batch on s, in the reference's order.
     template <typename Shade>
     cudaError_t shadow_pass(Shade&& shade, const wfpt_ray* in_rays, const wfpt_hit* in_res, const int32_t* in_s2i, uint32_t n_in,
@@ -531,42 +535,58 @@ struct wfpt_renderer {
         cudaError_t e;
         if (cfg.shadow_overlap && !timing_on && nslots >= 1 && (int)slots.size() >= nslots) {
             if ((e = cudaEventRecord(ev_fork, s)) != cudaSuccess) return e;
-            if ((e = shade()) != cudaSuccess || (e = join_shadow(s)) != cudaSuccess) return e;
-            if ((e = cudaEventRecord(ev_shade, s)) != cudaSuccess) return e;
             const uint32_t nb = (n_in + batch_diff - 1) / batch_diff;
             const int used = (int)std::min<uint32_t>((uint32_t)nslots, std::max(nb, 1u));
             for (int k = 0; k < used; ++k)
                 if ((e = cudaStreamWaitEvent(slots[k].stream, ev_fork, 0)) != cudaSuccess) return e;
-            for (uint32_t b = 0; b < nb; ++b) {
+            auto generate = [&](uint32_t b) {
                 ShadowSlot& sl = slots[b % used];
-                const cudaStream_t ss = sl.stream;
                 const uint32_t bb = b * batch_diff, bs = std::min(batch_diff, n_in - bb);
-                uint32_t* n_sh_dev = n_in_dev ? batch_counters + (b % used) : nullptr;
                 sl.rb.swapped = false;
-                if ((e = wfpt::launch_raygen_shadow(seeds.as<uint32_t>(), in_rays, in_res, sl.rb.rays_cur(),
-                                                    sl.rb.s2i_cur(), sl.rb.i2s_cur(), light, cfg.shadow_radius,
-                                                    (int)bb, (int)bs, n_in_dev, S, ss, n_sh_dev)) != cudaSuccess)
-                    return e;
-                if ((e = cudaEventRecord(sl.ev_rg, ss)) != cudaSuccess) return e;
-                if ((e = trace_rays(sl.rb, bs * (uint32_t)S, n_sh_dev, cfg.sort_shadow_rays != 0,
-                                    cfg.reorder_shadow_rays != 0, false, ss, sl.work.as<uint32_t>(), sl.scratch,
-                                    kind)) != cudaSuccess)
-                    return e;
-                if (b < (uint32_t)used && (e = cudaStreamWaitEvent(ss, ev_shade, 0)) != cudaSuccess) return e;
-                if ((e = wfpt::launch_reconstruct_shadow(sl.rb.results.as<wfpt_hit>(), in_s2i, sl.rb.i2s_cur(),
-                                                         in_pixels, out_pixels, (int)bb, (int)bs, n_in_dev, S, 0,
-                                                         ss)) != cudaSuccess)
-                    return e;
+                cudaError_t r = wfpt::launch_raygen_shadow(
+                    seeds.as<uint32_t>(), in_rays, in_res, sl.rb.rays_cur(), sl.rb.s2i_cur(), sl.rb.i2s_cur(), light,
+                    cfg.shadow_radius, (int)bb, (int)bs, n_in_dev, S, sl.stream,
+                    n_in_dev ? batch_counters + (b % used) : nullptr);
+                return r != cudaSuccess ? r : cudaEventRecord(sl.ev_rg, sl.stream);
+            };
+            auto trace_and_add = [&](uint32_t b) {
+                ShadowSlot& sl = slots[b % used];
+                const uint32_t bb = b * batch_diff, bs = std::min(batch_diff, n_in - bb);
+                cudaError_t r = trace_rays(sl.rb, bs * (uint32_t)S, n_in_dev ? batch_counters + (b % used) : nullptr,
+                                           cfg.sort_shadow_rays != 0, cfg.reorder_shadow_rays != 0, false, sl.stream,
+                                           sl.work.as<uint32_t>(), sl.scratch, kind);
+                if (r == cudaSuccess && b < (uint32_t)used) r = cudaStreamWaitEvent(sl.stream, ev_shade, 0);
+                if (r != cudaSuccess) return r;
+                return wfpt::launch_reconstruct_shadow(sl.rb.results.as<wfpt_hit>(), in_s2i, sl.rb.i2s_cur(),
+                                                       in_pixels, out_pixels, (int)bb, (int)bs, n_in_dev, S, 0,
+                                                       sl.stream);
+            };
+            auto generated = [&]() {  // s goes on after the generation of every batch issued so far
+                cudaError_t r = cudaSuccess;
+                for (int k = 0; k < used && r == cudaSuccess; ++k) r = cudaStreamWaitEvent(s, slots[k].ev_rg, 0);
+                return r;
+            };
+            if (nb <= (uint32_t)used) {
+                for (uint32_t b = 0; b < nb; ++b)
+                    if ((e = generate(b)) != cudaSuccess) return e;
+                if ((e = join_shadow(s)) != cudaSuccess || (e = generated()) != cudaSuccess) return e;
+                if ((e = shade(true)) != cudaSuccess || (e = cudaEventRecord(ev_shade, s)) != cudaSuccess) return e;
+                for (uint32_t b = 0; b < nb; ++b)
+                    if ((e = trace_and_add(b)) != cudaSuccess) return e;
+            } else {
+                if ((e = shade(false)) != cudaSuccess || (e = join_shadow(s)) != cudaSuccess) return e;
+                if ((e = cudaEventRecord(ev_shade, s)) != cudaSuccess) return e;
+                for (uint32_t b = 0; b < nb; ++b)
+                    if ((e = generate(b)) != cudaSuccess || (e = trace_and_add(b)) != cudaSuccess) return e;
+                if ((e = generated()) != cudaSuccess) return e;
             }
-            for (int k = 0; k < used; ++k) {
+            for (int k = 0; k < used; ++k)
                 if ((e = cudaEventRecord(slots[k].ev_done, slots[k].stream)) != cudaSuccess) return e;
-                if ((e = cudaStreamWaitEvent(s, slots[k].ev_rg, 0)) != cudaSuccess) return e;
-            }
             pending_slots = used;
             last_slots = std::max(last_slots, used);
             return cudaSuccess;
         }
-        if ((e = shade()) != cudaSuccess || (e = join_shadow(s)) != cudaSuccess) return e;
+        if ((e = shade(false)) != cudaSuccess || (e = join_shadow(s)) != cudaSuccess) return e;
         uint32_t* n_sh_dev = n_in_dev ? batch_counters : nullptr;
         uint32_t bb = 0;
         do {
@@ -593,13 +613,7 @@ struct wfpt_renderer {
         return cudaSuccess;
     }
 
-    // Renderer::primaryPass (Renderer.cpp:124-131): the camera rays and their
-    // shading.
-    // hit_counter (nullable): receives the number of primary hits (the
-    // shadow pass's input count, countRayHits) from reconstructSmooth.
-    // fresh: target is this pass's colour buffer, taken as cleared (its
-    // pixels are written, not accumulated); otherwise reconstructSmooth adds
-    // into it (the frame buffer of the primary-rays mode, over the samples).
+    // The camera rays of Renderer::primaryPass (Renderer.cpp:124-131).
     cudaError_t primary_trace(const float* s2w, const float* eye, float zfar, int pass, cudaStream_t s,
                               const wfpt::FrameParams* fp) {
         uint32_t n = (uint32_t)width * height;
@@ -613,13 +627,6 @@ struct wfpt_renderer {
                                       gpu_shared);
         });
     }
-    cudaError_t primary_shade(float* target, cudaStream_t s, uint32_t* hit_counter, bool fresh) {
-        uint32_t n = (uint32_t)width * height;
-        return wfpt::launch_reconstruct_smooth(primary.rays_cur(), primary.results.as<wfpt_hit>(), i2p.as<int32_t>(),
-                                               target, decreases.as<float>(), geoms, light, bg, n, nullptr,
-                                               cfg.num_primary_samples, s, hit_counter, fresh);
-    }
-
     // One frame.  fp (nullable): device-side frame parameters that replace
     // s2w/eye/zfar/frame_index, so that the same launches can be captured
     // once into a graph and replayed every frame.  (The reference also
@@ -646,8 +653,12 @@ struct wfpt_renderer {
                                              s)) != cudaSuccess)
                 return e;
             if (rt == WFPT_PRIMARY_RAYS) {
+                // The shading adds into the frame buffer over the samples.
                 if ((e = primary_trace(s2w, eye, zfar, pass, s, fp)) != cudaSuccess ||
-                    (e = primary_shade(frame_pixels, s, nullptr, false)) != cudaSuccess)
+                    (e = wfpt::launch_reconstruct_smooth(primary.rays_cur(), primary.results.as<wfpt_hit>(),
+                                                         i2p.as<int32_t>(), frame_pixels, decreases.as<float>(), geoms,
+                                                         light, bg, n, nullptr, cfg.num_primary_samples, s, nullptr,
+                                                         false)) != cudaSuccess)
                     return e;
                 continue;
             }
@@ -661,40 +672,24 @@ struct wfpt_renderer {
             // pass): every pixel the shadow pass reads back was written by
             // this pass's reconstructSmooth in fresh mode.
             if ((e = primary_trace(s2w, eye, zfar, pass, s, fp)) != cudaSuccess) return e;
-            auto shade = [&]() { return primary_shade(auxb[ai], s, cnt(pass, kCntHits + 0), true); };
-            if ((e = shadow_pass(shade, primary.rays_cur(), primary.results.as<wfpt_hit>(), i2p.as<int32_t>(), n, nullptr,
-                                 auxb[ai], frame_pixels, cnt(pass, kCntBatch), s, primary_kind(), 0)) != cudaSuccess)
-                return e;
-            if (rt != WFPT_PATH_RAYS) continue;
+            // Level 0: the camera rays; level b + 1: the rays of bounce b.
             int qsel = 0;  // PathQueue::swapBuffers
-            for (int bounce = 0; bounce < cfg.recursion_depth; ++bounce) {
-                ai ^= 1;
+            const wfpt_ray* in_rays = primary.rays_cur();
+            const wfpt_hit* in_res = primary.results.as<wfpt_hit>();
+            const int32_t* in_s2i = i2p.as<int32_t>();
+            const uint32_t* in_cnt = nullptr;
+            int kind = primary_kind();
+            for (int level = 0;; ++level) {
+                const bool more = rt == WFPT_PATH_RAYS && level < cfg.recursion_depth;
                 RayBufferDev& out = queue[qsel ? 0 : 1];
-                const wfpt_ray* in_rays;
-                const wfpt_hit* in_res;
-                const int32_t* in_s2i;
-                const uint32_t* in_cnt;
-                if (bounce == 0) {
-                    in_rays = primary.rays_cur();
-                    in_res = primary.results.as<wfpt_hit>();
-                    in_s2i = i2p.as<int32_t>();
-                    in_cnt = nullptr;
-                } else {
-                    RayBufferDev& in = queue[qsel ? 1 : 0];
-                    in_rays = in.rays_cur();
-                    in_res = in.results.as<wfpt_hit>();
-                    in_s2i = in.s2i_cur();
-                    in_cnt = cnt(pass, kCntPath + bounce - 1);
-                }
-                out.swapped = false;
-                uint32_t* out_cnt = cnt(pass, kCntPath + bounce);
-                const bool sort_b = cfg.sort_path_rays != 0 && ((cfg.path_sort_skip >> bounce) & 1) == 0;
+                uint32_t* out_cnt = more ? cnt(pass, kCntPath + level) : nullptr;
+                const bool sort_b = cfg.sort_path_rays != 0 && ((cfg.path_sort_skip >> level) & 1) == 0;
                 // A sorted bounce gets its Morton keys from the path-ray
                 // generation (the same keys the Morton kernel would compute
                 // from the written rays); a timed frame keeps the Morton
                 // kernel, whose time the sort log reports.
                 wfpt::MortonOut mo{};
-                const bool fused_keys = sort_b && !timing_on;
+                const bool fused_keys = more && sort_b && !timing_on;
                 if (fused_keys) {
                     mo.kind = cfg.morton_kind;
                     mo.keys = out.keys.p;
@@ -705,28 +700,44 @@ struct wfpt_renderer {
                     }
                 }
                 // Renderer::pathPass -> tracePathRays (Renderer.cpp:156-162, 277-297).
-                if ((e = timed(s, T_PATH, C_NONE, -1, [&]() {
-                         return wfpt::launch_raygen_path(seeds.as<uint32_t>(), geoms, in_rays, out.rays_cur(), in_s2i,
-                                                         out.s2i_cur(), in_res, decreases.as<float>(), out_cnt, n,
-                                                         in_cnt, cfg.albedo,
-                                                         path_scratch.as<unsigned char>() + bounce * path_bytes, s,
-                                                         fused_keys ? &mo : nullptr, true);
-                     })) != cudaSuccess)
+                bool generated = false;
+                auto path = [&](const wfpt::ShadeOut* so) {
+                    generated = true;
+                    out.swapped = false;
+                    return timed(s, T_PATH, C_NONE, -1, [&]() {
+                        return wfpt::launch_raygen_path(
+                            seeds.as<uint32_t>(), geoms, in_rays, out.rays_cur(), in_s2i, out.s2i_cur(), in_res,
+                            decreases.as<float>(), out_cnt, n, in_cnt, cfg.albedo,
+                            path_scratch.as<unsigned char>() + level * path_bytes, s, fused_keys ? &mo : nullptr, true,
+                            so);
+                    });
+                };
+                auto shade = [&](bool with_path) {
+                    uint32_t* hits = cnt(pass, kCntHits + level);
+                    if (with_path && more) {
+                        wfpt::ShadeOut so{auxb[ai], {light[0], light[1], light[2]}, {bg[0], bg[1], bg[2]},
+                                          cfg.num_primary_samples, hits};
+                        return path(&so);
+                    }
+                    return wfpt::launch_reconstruct_smooth(in_rays, in_res, in_s2i, auxb[ai], decreases.as<float>(),
+                                                           geoms, light, bg, n, in_cnt, cfg.num_primary_samples, s,
+                                                           hits, true);
+                };
+                if ((e = shadow_pass(shade, in_rays, in_res, in_s2i, n, in_cnt, auxb[ai], frame_pixels,
+                                     cnt(pass, kCntBatch), s, kind, level)) != cudaSuccess)
                     return e;
+                if (!more) break;
+                if (!generated && (e = path(nullptr)) != cudaSuccess) return e;
                 if ((e = trace_rays(out, n, out_cnt, sort_b, sort_b && cfg.reorder_path_rays != 0, true, s,
-                                    work.as<uint32_t>(), sort_scratch, cfg.bvh_kind, T_PATH, 100 + bounce,
+                                    work.as<uint32_t>(), sort_scratch, cfg.bvh_kind, T_PATH, 100 + level,
                                     fused_keys)) != cudaSuccess)
                     return e;
-                auto shade_bounce = [&]() {
-                    return wfpt::launch_reconstruct_smooth(out.rays_cur(), out.results.as<wfpt_hit>(), out.s2i_cur(),
-                                                           auxb[ai], decreases.as<float>(), geoms, light, bg, n,
-                                                           out_cnt, cfg.num_primary_samples, s,
-                                                           cnt(pass, kCntHits + bounce + 1), true);
-                };
-                if ((e = shadow_pass(shade_bounce, out.rays_cur(), out.results.as<wfpt_hit>(), out.s2i_cur(), n, out_cnt,
-                                     auxb[ai], frame_pixels, cnt(pass, kCntBatch), s, cfg.bvh_kind, bounce + 1)) !=
-                    cudaSuccess)
-                    return e;
+                in_rays = out.rays_cur();
+                in_res = out.results.as<wfpt_hit>();
+                in_s2i = out.s2i_cur();
+                in_cnt = out_cnt;
+                kind = cfg.bvh_kind;
+                ai ^= 1;
                 qsel ^= 1;  // PathQueue::swap
             }
         }

@@ -341,6 +341,12 @@ __device__ uint32_t tile_prefix(uint32_t* tile_state, uint32_t tile, uint32_t co
     return s_prefix;
 }
 
+// reconstructSmooth's addition to a fresh pixel.
+__device__ __forceinline__ void store_shaded(const ShadeOut& o, int pixel, f3 c) {
+    const f3 color = add(mk(0.0f, 0.0f, 0.0f), divs(c, (float)o.spp));
+    reinterpret_cast<float4*>(o.pixels)[pixel] = make_float4(color.x, color.y, color.z, 1.0f);
+}
+
 // raygenPath.comp:95-167.  scratch[0] = tile ticket, scratch[1..] = tile
 // states; both zeroed before the launch.  MK >= 0: also writes
 // the Morton key of kind MK of every output ray and its index (keys[dst],
@@ -351,15 +357,19 @@ __device__ uint32_t tile_prefix(uint32_t* tile_state, uint32_t tile, uint32_t co
 // spilled) and 256-bit loads of the ray and the vertices, 97 -> 87 us at 2.07M
 // courtyard rays, 342 -> 302 at 8.3M; at 46 registers and five blocks 93 and
 // 320.
-template <int MK>
-__global__ void __launch_bounds__(kBlock, 8) k_raygen_path(uint32_t* __restrict__ seeds, const wfpt_geometry* __restrict__ geoms,
+// SHADE: also what reconstructSmooth does with the same rays, so that the ray,
+// the hit and the gather of its vertices are read once: 121 us a bounce of
+// 2.07M courtyard rays instead of 72 + 89 (four to eight blocks per SM equal).
+template <int MK, bool SHADE>
+__global__ void __launch_bounds__(kBlock, SHADE ? 6 : 8) k_raygen_path(
+                              uint32_t* __restrict__ seeds, const wfpt_geometry* __restrict__ geoms,
                               const float4* __restrict__ in_rays, float4* __restrict__ out_rays,
                               const int32_t* __restrict__ in_i2p, int32_t* __restrict__ out_i2p,
                               const int4* __restrict__ in_results, float4* __restrict__ decreases,
                               uint32_t* __restrict__ out_count, uint32_t n,
                               const uint32_t* __restrict__ n_dev, float albedo,
                               uint32_t* __restrict__ scratch, void* __restrict__ keys,
-                              uint32_t* __restrict__ key_idx, Box6 box, bool wide) {
+                              uint32_t* __restrict__ key_idx, Box6 box, bool wide, ShadeOut shade) {
     __shared__ uint32_t s_tile;
     __shared__ uint32_t s_warp[kBlock / 32];
     uint32_t count = load_count(n, n_dev);
@@ -382,16 +392,25 @@ __global__ void __launch_bounds__(kBlock, 8) k_raygen_path(uint32_t* __restrict_
             pixel = in_i2p[task];
             uint32_t seed = seeds[task];
             int4 res = in_results[task];
+            if (SHADE) {
+                dc = decreases[pixel];
+                if (res.x < 0)
+                    store_shaded(shade, pixel, mul(mk(dc.x, dc.y, dc.z), mk(shade.bg[0], shade.bg[1], shade.bg[2])));
+            }
             if (res.x >= 0) {
                 float4 r0, r1;
                 load_ray(in_rays, task, r0, r1, wide);
                 f3 dir = mk(r1.x, r1.y, r1.z);
                 f3 nrm = unpack_normal<true>(geoms, res.y, res.x, (uint32_t)res.w);
                 f3 ff = faceforward(nrm, dir, nrm);
-                float ra = randf(seed);
-                float rb = randf(seed);
                 float t = __int_as_float(res.z);
                 f3 hit = add(mk(r0.x, r0.y, r0.z), mul(dir, t));
+                if (SHADE) {
+                    const f3 L = normalize(sub(mk(shade.light[0], shade.light[1], shade.light[2]), hit));
+                    store_shaded(shade, pixel, mul(mk(dc.x, dc.y, dc.z), fmaxf(dot(ff, L), 0.1f)));
+                }
+                float ra = randf(seed);
+                float rb = randf(seed);
                 const float EPS = 1.0e-4f;
                 f3 nd = cosine_random_vector(ra, rb, ff);
                 f3 org = add(hit, mul(nd, EPS));
@@ -402,7 +421,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_raygen_path(uint32_t* __restrict_
                 // Read the pixel's path throughput now (each pixel has one ray
                 // per pass): the load overlaps the look-back below instead of
                 // following it (12 % faster at the frame's 2.07M rays).
-                dc = decreases[pixel];
+                if (!SHADE) dc = decreases[pixel];
             }
         }
         // Block-level ordered ranks.
@@ -437,7 +456,10 @@ __global__ void __launch_bounds__(kBlock, 8) k_raygen_path(uint32_t* __restrict_
             dc.w = __fmul_rn(dc.w, 1.0f);
             decreases[pixel] = dc;
         }
-        if (tile == ntiles - 1 && threadIdx.x == 0) *out_count = base + total;
+        if (tile == ntiles - 1 && threadIdx.x == 0) {
+            *out_count = base + total;
+            if (SHADE) *shade.hit_count = base + total;  // a path ray per hit
+        }
         if (once) return;
         __syncthreads();  // s_tile, s_warp and the tile prefix are reused
     }
@@ -708,11 +730,21 @@ size_t raygen_path_scratch_bytes(uint32_t max_n) {
     return (1 + tiles + 1) * sizeof(uint32_t);
 }
 
+template <bool SHADE>
+static auto path_kernel(int morton_kind) {
+    switch (morton_kind) {
+        case WFPT_MORTON_AILA32: return k_raygen_path<WFPT_MORTON_AILA32, SHADE>;
+        case WFPT_MORTON_6D48: return k_raygen_path<WFPT_MORTON_6D48, SHADE>;
+        case WFPT_MORTON_6D64: return k_raygen_path<WFPT_MORTON_6D64, SHADE>;
+        default: return k_raygen_path<-1, SHADE>;
+    }
+}
+
 cudaError_t launch_raygen_path(uint32_t* seeds, const wfpt_geometry* geoms, const wfpt_ray* in_rays,
                                wfpt_ray* out_rays, const int32_t* in_i2p, int32_t* out_i2p,
                                const wfpt_hit* in_res, float* decreases, uint32_t* out_count,
                                uint32_t n, const uint32_t* n_dev, float albedo, void* scratch,
-                               cudaStream_t s, const MortonOut* mo, bool cleared) {
+                               cudaStream_t s, const MortonOut* mo, bool cleared, const ShadeOut* shade) {
     size_t tiles = ((size_t)n + kBlock - 1) / kBlock;
     if (!cleared) {
         cudaError_t e = cudaMemsetAsync(scratch, 0, (1 + tiles) * sizeof(uint32_t), s);
@@ -720,18 +752,14 @@ cudaError_t launch_raygen_path(uint32_t* seeds, const wfpt_geometry* geoms, cons
     }
     unsigned grid = tiles == 0 ? 1u : grid_for(n, n_dev);
     const Box6 box = mo ? mo->box : Box6{};
-    auto k = k_raygen_path<-1>;
-    if (mo != nullptr) {
-        k = mo->kind == WFPT_MORTON_AILA32 ? k_raygen_path<WFPT_MORTON_AILA32>
-            : mo->kind == WFPT_MORTON_6D48 ? k_raygen_path<WFPT_MORTON_6D48>
-                                           : k_raygen_path<WFPT_MORTON_6D64>;
-    }
+    auto k = path_kernel<false>(mo ? mo->kind : -1);
+    if (shade != nullptr) k = path_kernel<true>(mo ? mo->kind : -1);
     k<<<grid, kBlock, 0, s>>>(seeds, geoms, reinterpret_cast<const float4*>(in_rays),
                               reinterpret_cast<float4*>(out_rays), in_i2p, out_i2p,
                               reinterpret_cast<const int4*>(in_res), reinterpret_cast<float4*>(decreases),
                               out_count, n, n_dev, albedo, reinterpret_cast<uint32_t*>(scratch),
                               mo ? mo->keys : nullptr, mo ? mo->indices : nullptr, box,
-                              wide_rays(in_rays) && wide_rays(out_rays));
+                              wide_rays(in_rays) && wide_rays(out_rays), shade ? *shade : ShadeOut{});
     count_launch();
     return cudaGetLastError();
 }
@@ -764,9 +792,9 @@ cudaError_t raygen_path_selftest_timeout(cudaStream_t s) {
     if (e == cudaSuccess) e = cudaMemsetAsync(results, 0xFF, N * sizeof(int4), s);  // every ray a miss
     if (e == cudaSuccess) e = cudaMemcpyAsync(scratch, &one, sizeof(one), cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) {
-        k_raygen_path<-1><<<1, kBlock, 0, s>>>(seeds, nullptr, in_rays, out_rays, in_i2p, out_i2p, results,
+        k_raygen_path<-1, false><<<1, kBlock, 0, s>>>(seeds, nullptr, in_rays, out_rays, in_i2p, out_i2p, results,
                                                decreases, count, N, nullptr, 0.8f, scratch, nullptr, nullptr,
-                                               Box6{}, wide_rays(out_rays));
+                                               Box6{}, wide_rays(out_rays), ShadeOut{});
         count_launch();
         e = cudaGetLastError();
     }
@@ -867,11 +895,11 @@ cudaError_t launch_raygen_path_static(uint32_t* seeds, const wfpt_geometry* geom
     e = cudaMemsetAsync(scratch, 0, (1 + tiles) * sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
     unsigned grid = tiles == 0 ? 1u : grid_for(n, n_dev);
-    k_raygen_path<-1><<<grid, kBlock, 0, s>>>(
+    k_raygen_path<-1, false><<<grid, kBlock, 0, s>>>(
         seeds, geoms, reinterpret_cast<const float4*>(in_rays), reinterpret_cast<float4*>(out_rays), in_i2p,
         out_i2p, reinterpret_cast<const int4*>(in_res), reinterpret_cast<float4*>(decreases), out_count, n,
         n_dev, albedo, scratch, nullptr, nullptr, Box6{},
-        wide_rays(in_rays) && wide_rays(out_rays));
+        wide_rays(in_rays) && wide_rays(out_rays), ShadeOut{});
     count_launch();
     return cudaGetLastError();
 }

@@ -35,6 +35,15 @@ struct MortonOut {
     Box6 box;
 };
 
+// Shading written by the path-ray generation for its input rays: what
+// launch_reconstruct_smooth writes into fresh pixels, and the hit count.
+struct ShadeOut {
+    float* pixels;
+    float light[3], bg[3];
+    int spp;
+    uint32_t* hit_count;
+};
+
 // Number of kernels this library has launched (all threads, all devices).
 void count_launch(uint32_t k = 1);
 uint64_t launch_count();
@@ -65,12 +74,14 @@ cudaError_t launch_raygen_shadow(const uint32_t* seeds, const wfpt_ray* in_rays,
 size_t raygen_path_scratch_bytes(uint32_t max_n);
 // mo (nullable): also the Morton keys of the output rays (what
 // launch_morton over out_rays and *out_count would write).  cleared: the
-// scratch has been zeroed already.
+// scratch has been zeroed already.  shade (nullable): also what
+// launch_reconstruct_smooth (fresh) does with the input rays.
 cudaError_t launch_raygen_path(uint32_t* seeds, const wfpt_geometry* geoms, const wfpt_ray* in_rays,
                                wfpt_ray* out_rays, const int32_t* in_i2p, int32_t* out_i2p,
                                const wfpt_hit* in_res, float* decreases, uint32_t* out_count,
                                uint32_t n, const uint32_t* n_dev, float albedo, void* scratch,
-                               cudaStream_t s, const MortonOut* mo = nullptr, bool cleared = false);
+                               cudaStream_t s, const MortonOut* mo = nullptr, bool cleared = false,
+                               const ShadeOut* shade = nullptr);
 // launch_raygen_path over the library's static scratch (n at most
 // WFPT_RAYGEN_PATH_STATIC_MAX_RAYS); calls on one device must not overlap.
 cudaError_t launch_raygen_path_static(uint32_t* seeds, const wfpt_geometry* geoms, const wfpt_ray* in_rays,
