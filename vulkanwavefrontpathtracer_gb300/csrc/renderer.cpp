@@ -460,14 +460,22 @@ struct wfpt_renderer {
     // :281-286 do (the sorted trace then overwrites those results).
     // keys_ready: rb.keys / rb.idx already hold the rays' Morton keys (written
     // by the path-ray generation), so the sort starts without the Morton kernel.
-    cudaError_t trace_rays(RayBufferDev& rb, uint32_t n, const uint32_t* n_dev, bool sort, bool reorder, bool closest,
+    // kOccluded: rb.results gets a word per ray (launch_occluded).
+    enum Query { kAnyHit, kClosestHit, kOccluded };
+    cudaError_t trace_rays(RayBufferDev& rb, uint32_t n, const uint32_t* n_dev, bool sort, bool reorder, Query query,
                            cudaStream_t s, uint32_t* wk, DevBuf& scratch, int kind, int total = T_NONE,
                            int log = -1, bool keys_ready = false) {
         const wfpt::SceneDevice& sc = *wfpt::scene_device(scene);
         cudaError_t e;
+        auto trace = [&](const uint32_t* index) {
+            if (query == kOccluded)
+                return wfpt::launch_occluded(sc, kind, rb.rays_cur(), rb.results.as<int32_t>(), index, n, n_dev, s, wk,
+                                             gpu_shared);
+            return wfpt::launch_trace(sc, kind, rb.rays_cur(), rb.results.as<wfpt_hit>(), index, n, n_dev,
+                                      query == kClosestHit ? 1 : 0, s, wk, gpu_shared);
+        };
         auto plain = [&]() {
-            return wfpt::launch_trace(sc, kind, rb.rays_cur(), rb.results.as<wfpt_hit>(), nullptr, n, n_dev,
-                                      closest ? 1 : 0, s, wk, gpu_shared);
+            return trace(nullptr);
         };
         if (!sort) return timed(s, total, C_NONE, -1, plain);
         if (timing_on && log >= 0 && (e = timed(s, T_NONE, C_TRACE, log, plain)) != cudaSuccess) return e;
@@ -491,9 +499,7 @@ struct wfpt_renderer {
             rb.swap();
         }
         return timed(s, total, C_TRACE_SORT, log, [&]() {
-            return wfpt::launch_trace(sc, kind, rb.rays_cur(), rb.results.as<wfpt_hit>(),
-                                      reorder ? nullptr : rb.idx.as<uint32_t>(), n, n_dev, closest ? 1 : 0, s, wk,
-                                      gpu_shared);
+            return trace(reorder ? nullptr : rb.idx.as<uint32_t>());
         });
     }
 
@@ -531,6 +537,8 @@ struct wfpt_renderer {
                             const uint32_t* n_in_dev, float* in_pixels, float* out_pixels,
                             uint32_t* batch_counters, cudaStream_t s, int kind, int slot_log) {
         const int S = cfg.num_shadow_samples;
+        const Query query = wfpt::occluded_ready(*wfpt::scene_device(scene), kind) ? kOccluded : kAnyHit;
+        const int hit_stride = query == kOccluded ? 1 : 4;  // words of a result
         const uint32_t batch_diff = (uint32_t)(kMaxBatch / S);
         cudaError_t e;
         if (cfg.shadow_overlap && !timing_on && nslots >= 1 && (int)slots.size() >= nslots) {
@@ -553,11 +561,11 @@ struct wfpt_renderer {
                 ShadowSlot& sl = slots[b % used];
                 const uint32_t bb = b * batch_diff, bs = std::min(batch_diff, n_in - bb);
                 cudaError_t r = trace_rays(sl.rb, bs * (uint32_t)S, n_in_dev ? batch_counters + (b % used) : nullptr,
-                                           cfg.sort_shadow_rays != 0, cfg.reorder_shadow_rays != 0, false, sl.stream,
+                                           cfg.sort_shadow_rays != 0, cfg.reorder_shadow_rays != 0, query, sl.stream,
                                            sl.work.as<uint32_t>(), sl.scratch, kind);
                 if (r == cudaSuccess && b < (uint32_t)used) r = cudaStreamWaitEvent(sl.stream, ev_shade, 0);
                 if (r != cudaSuccess) return r;
-                return wfpt::launch_reconstruct_shadow(sl.rb.results.as<wfpt_hit>(), in_s2i, sl.rb.i2s_cur(),
+                return wfpt::launch_reconstruct_shadow(sl.rb.results.as<int32_t>(), hit_stride, in_s2i, sl.rb.i2s_cur(),
                                                        in_pixels, out_pixels, (int)bb, (int)bs, n_in_dev, S, 0,
                                                        sl.stream);
             };
@@ -600,10 +608,10 @@ struct wfpt_renderer {
                  })) != cudaSuccess)
                 return e;
             if ((e = trace_rays(shadow, bs * (uint32_t)S, n_sh_dev, cfg.sort_shadow_rays != 0,
-                                cfg.reorder_shadow_rays != 0, false, s, work.as<uint32_t>(), sort_scratch, kind,
+                                cfg.reorder_shadow_rays != 0, query, s, work.as<uint32_t>(), sort_scratch, kind,
                                 T_SHADOW, slot_log)) != cudaSuccess)
                 return e;
-            if ((e = wfpt::launch_reconstruct_shadow(shadow.results.as<wfpt_hit>(), in_s2i, shadow.i2s_cur(),
+            if ((e = wfpt::launch_reconstruct_shadow(shadow.results.as<int32_t>(), hit_stride, in_s2i, shadow.i2s_cur(),
                                                      in_pixels, out_pixels, (int)bb, (int)bs, n_in_dev, S, 0, s)) !=
                 cudaSuccess)
                 return e;
@@ -728,7 +736,7 @@ struct wfpt_renderer {
                     return e;
                 if (!more) break;
                 if (!generated && (e = path(nullptr)) != cudaSuccess) return e;
-                if ((e = trace_rays(out, n, out_cnt, sort_b, sort_b && cfg.reorder_path_rays != 0, true, s,
+                if ((e = trace_rays(out, n, out_cnt, sort_b, sort_b && cfg.reorder_path_rays != 0, kClosestHit, s,
                                     work.as<uint32_t>(), sort_scratch, cfg.bvh_kind, T_PATH, 100 + level,
                                     fused_keys)) != cudaSuccess)
                     return e;

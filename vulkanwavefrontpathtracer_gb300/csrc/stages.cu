@@ -523,9 +523,10 @@ __global__ void k_reconstruct_smooth(const float4* __restrict__ rays, const int4
 }
 
 // ---------------------------------------------------- reconstructShadow
-// reconstructShadow.comp:39-59.
+// reconstructShadow.comp:39-59.  hits: the first words of the results, `stride`
+// words apart.
 template <bool LOOP>
-__global__ void k_reconstruct_shadow(const int4* __restrict__ results, const int32_t* __restrict__ i2p,
+__global__ void k_reconstruct_shadow(const int32_t* __restrict__ hits, int stride, const int32_t* __restrict__ i2p,
                                      const int32_t* __restrict__ i2s,
                                      const float4* __restrict__ in_pixels, float4* __restrict__ out_pixels,
                                      int batch_begin, int batch_size,
@@ -542,7 +543,7 @@ __global__ void k_reconstruct_shadow(const int4* __restrict__ results, const int
         float shadow = 0.0f;
         for (int i = 0; i < S; ++i) {
             int slot = i2s[(int)task * S + i];
-            if (results[slot].x == -1) shadow = __fadd_rn(shadow, 1.0f);
+            if (hits[(size_t)slot * stride] == -1) shadow = __fadd_rn(shadow, 1.0f);
         }
         shadow = __fdiv_rn(shadow, (float)S);
         float4 c = make_float4(__fmul_rn(ip.x, shadow), __fmul_rn(ip.y, shadow), __fmul_rn(ip.z, shadow), 1.0f);
@@ -919,13 +920,13 @@ cudaError_t launch_reconstruct_smooth(const wfpt_ray* rays, const wfpt_hit* res,
     return cudaGetLastError();
 }
 
-cudaError_t launch_reconstruct_shadow(const wfpt_hit* res, const int32_t* i2p, const int32_t* i2s,
+cudaError_t launch_reconstruct_shadow(const int32_t* hits, int stride, const int32_t* i2p, const int32_t* i2s,
                                       const float* in_pixels, float* out_pixels, int bb, int bs,
                                       const uint32_t* n_in_dev, int S, int replace, cudaStream_t s) {
     if (bs <= 0) return cudaSuccess;
     auto k = capped((uint64_t)bs, n_in_dev) ? k_reconstruct_shadow<true> : k_reconstruct_shadow<false>;
     k<<<grid_for((uint64_t)bs, n_in_dev), kBlock, 0, s>>>(
-        reinterpret_cast<const int4*>(res), i2p, i2s, reinterpret_cast<const float4*>(in_pixels),
+        hits, stride, i2p, i2s, reinterpret_cast<const float4*>(in_pixels),
         reinterpret_cast<float4*>(out_pixels), bb, bs, n_in_dev, S, replace);
     count_launch();
     return cudaGetLastError();

@@ -93,7 +93,8 @@ cudaError_t launch_reconstruct_smooth(const wfpt_ray* rays, const wfpt_hit* res,
                                       const float* light, const float* bg, uint32_t n,
                                       const uint32_t* n_dev, int spp, cudaStream_t s,
                                       uint32_t* hit_count = nullptr, bool fresh = false);
-cudaError_t launch_reconstruct_shadow(const wfpt_hit* res, const int32_t* i2p, const int32_t* i2s,
+// hits: a word per shadow ray, -1 for a miss, `stride` words apart.
+cudaError_t launch_reconstruct_shadow(const int32_t* hits, int stride, const int32_t* i2p, const int32_t* i2s,
                                       const float* in_pixels, float* out_pixels, int bb, int bs,
                                       const uint32_t* n_in_dev, int S, int replace, cudaStream_t s);
 cudaError_t launch_count_hits(const wfpt_hit* res, uint32_t n, const uint32_t* n_dev, uint32_t* count,
