@@ -371,6 +371,10 @@ __device__ __forceinline__ uint32_t byte_of(uint32_t w, int b) { return (w >> (8
 __device__ __forceinline__ float q2f(uint32_t w, int b) {
     return __uint_as_float(__byte_perm(w, 0x47000000u, 0x7604u | ((uint32_t)b << 4)));
 }
+// The same for bytes 0 and 2 by a two-way dot product with 256, off the ALU.
+__device__ __forceinline__ float q2f_dot(uint32_t w, int b) {
+    return __uint_as_float((b & 2) ? __dp2a_hi(256u, w, 0x47000000u) : __dp2a_lo(256u, w, 0x47000000u));
+}
 
 // Two FP32 fused multiply-adds in one instruction (sm_100 and later), each
 // rounded as one alone: a child's near and far plane of an axis.
@@ -402,6 +406,11 @@ __device__ __forceinline__ void unpair2(uint64_t v, float& lo, float& hi) {
 // bounce-1 rays), any hit 1221 -> 1141 us.  With the ALU relieved, the paired
 // multiply-adds pay too (24 issue slots a node): 949 -> 920 and 1141 -> 1108
 // us.  City: 468 -> 444 and 361 -> 339 us.
+// DOT: every other byte of an axis by a dot product, for the kernels with
+// registers to spare: 65K courtyard rays 105 -> 101 us closest, 84 -> 80 us any
+// hit, 57K soup rays 98 -> 95 us.  Under the 64-register cap of the large
+// wavefronts' kernels it spills and costs 8 %.
+template <bool DOT = false>
 __device__ __forceinline__ uint32_t intersect_node8(const float4* __restrict__ nd, const RayT& r, float tcur,
                                                     uint32_t& child_base, uint32_t& imask, uint32_t& leaf) {
     float4 n0 = __ldg(nd + 0);
@@ -454,7 +463,9 @@ __device__ __forceinline__ uint32_t intersect_node8(const float4* __restrict__ n
         float tnx, tny, tnz, tfx, tfy, tfz;
         unpair2(fma2(pair2(q2f(nx[w], b), q2f(fx[w], b)), A[0], B[0]), tnx, tfx);
         unpair2(fma2(pair2(q2f(ny[w], b), q2f(fy[w], b)), A[1], B[1]), tny, tfy);
-        unpair2(fma2(pair2(q2f(nz[w], b), q2f(fz[w], b)), A[2], B[2]), tnz, tfz);
+        const bool dot = DOT && (b & 1) == 0;
+        const float qn = dot ? q2f_dot(nz[w], b) : q2f(nz[w], b), qf = dot ? q2f_dot(fz[w], b) : q2f(fz[w], b);
+        unpair2(fma2(pair2(qn, qf), A[2], B[2]), tnz, tfz);
         float tn = fmaxf(max3f(tnx, tny, tnz), r.tmin);
         float tf = fminf(min3f(tfx, tfy, tfz), tcur);
         if (tn <= tf * kBoxSlack) hit[w] |= 0x10u << (8 * b);
@@ -836,7 +847,7 @@ __global__ void __launch_bounds__(kBlock, PER_SM) k_trace_bvh8_coop(
                 }
                 uint32_t child_base, imask, lf;
                 if (COUNT) ++c_nodes;
-                const uint32_t inner = intersect_node8(nodes + 5 * (size_t)node, r, tcur, child_base, imask, lf);
+                const uint32_t inner = intersect_node8<PER_SM == 3>(nodes + 5 * (size_t)node, r, tcur, child_base, imask, lf);
                 ng = make_uint2(child_base, inner | imask);
                 if (leaf == 0u) {
                     leaf = lf;
@@ -1062,7 +1073,7 @@ __global__ void __launch_bounds__(kBlock, PER_SM) k_occluded_bvh8(
                     }
                 }
                 uint32_t child_base, imask, lf;
-                const uint32_t inner = intersect_node8(nodes + 5 * (size_t)node, r, tmax, child_base, imask, lf);
+                const uint32_t inner = intersect_node8<PER_SM == 3>(nodes + 5 * (size_t)node, r, tmax, child_base, imask, lf);
                 ng = make_uint2(child_base, inner | imask);
                 if (leaf == 0u) {
                     leaf = lf;
