@@ -980,27 +980,33 @@ __global__ void __launch_bounds__(kBlock, PER_SM) k_trace_bvh8_coop(
     }
 }
 
-// Occlusion only: the any-hit traversal above without the hit's record.  A
-// shadow pass reads no more of a hit than that there is one, so any accepted
-// triangle will do: no keys and atomics, no order among the triangles in hand,
-// no barycentrics, no waiting, and one word per ray (0, or -1 if nothing is in
-// the way) instead of sixteen bytes.  All pairs of an iteration are tested at
-// its end, so they need no ring.  The nine shadow passes of a 1080p courtyard
-// frame (two rays per hit) 10.11 -> 9.02 ms, reading them back 0.51 -> 0.45 ms.
-// The nearest child first is best here too (1040 us against 1081 in slot order
-// and 1098 farthest first; the city 314, 311 and 309).
+// Any-hit traversal: that of k_trace_bvh8_coop for rays that are tested after
+// every iteration (its batch 1, the default).  Then a lane has nothing to wait
+// for, and the pairs need no ring: 2.07M courtyard bounce-1 hits (two rays
+// each) 1108 -> 1091 us, the city's 1.6M 339 -> 330, 6.4M 1245 -> 1211.
+//
+// !RECORD: for occlusion alone.  A shadow pass reads no more of a hit than that
+// there is one, so any accepted triangle will do: no keys and atomics, no order
+// among the triangles in hand, no barycentrics, and one word per ray (0, or -1
+// if nothing is in the way) instead of sixteen bytes.  The nine shadow passes
+// of a 1080p courtyard frame (two rays per hit) 10.11 -> 9.02 ms, reading them
+// back 0.51 -> 0.45 ms.  The nearest child first is best here too (1040 us
+// against 1081 in slot order and 1098 farthest first; the city 314, 311, 309).
 // Small wavefronts (PER_SM 3) go on past four leaves: 256x256 frame 914 -> 893
 // us; large ones that way 0.6 % slower.
 constexpr uint32_t kFewOccluded = 16;  // 20: 0-1 % slower, 24: 1-3 %, 12: 0-1 %
-template <int PER_SM>
-__global__ void __launch_bounds__(kBlock, PER_SM) k_occluded_bvh8(
+template <bool RECORD, int PER_SM>
+__global__ void __launch_bounds__(kBlock, PER_SM) k_any_bvh8(
     const float4* __restrict__ nodes, const float4* __restrict__ tris, const float4* __restrict__ rays,
-    int32_t* __restrict__ occluded, const uint32_t* __restrict__ ray_index, uint32_t n,
+    void* __restrict__ results, const uint32_t* __restrict__ ray_index, uint32_t n,
     const uint32_t* __restrict__ n_dev, uint32_t* __restrict__ work, uint32_t refill, uint32_t steps) {
     __shared__ RayS s_ray[kBlock];
     __shared__ float s_tmax[kBlock];
-    __shared__ uint32_t s_hit[kBlock];
-    constexpr uint32_t MORE = PER_SM == 3 ? 4u : kMoreLeaves;
+    __shared__ uint32_t s_hit[RECORD ? 1 : kBlock];
+    __shared__ unsigned long long s_best[RECORD ? kBlock : 1];
+    __shared__ uint4 s_rec[RECORD ? kBlock : 1];        // best hit: primId, geomId, packed barycentrics, t
+    __shared__ uint32_t s_second[RECORD ? kBlock : 1];  // where the pairs of the lane's second group start
+    constexpr uint32_t MORE = !RECORD && PER_SM == 3 ? 4u : kMoreLeaves;
     __shared__ uint32_t s_task[kBlock / 32][32 * (3 * MORE + 24)];
     const uint32_t count = load_count(n, n_dev);
     const uint32_t lane = threadIdx.x & 31;
@@ -1022,7 +1028,14 @@ __global__ void __launch_bounds__(kBlock, PER_SM) k_occluded_bvh8(
         const uint32_t busy_mask = __ballot_sync(0xffffffffu, state == kTracing);
         if (want_mask != 0u && (__popc(want_mask) >= refill || busy_mask == 0u)) {
             if (state >= kFree) {
-                occluded[ri] = state == kBlocked ? 0 : -1;
+                if (!RECORD) {
+                    static_cast<int32_t*>(results)[ri] = state == kBlocked ? 0 : -1;
+                } else if (state == kBlocked) {
+                    const uint4 h = s_rec[threadIdx.x];
+                    static_cast<int4*>(results)[ri] = make_int4((int)h.x, (int)h.y, (int)h.w, (int)h.z);
+                } else {
+                    write_miss(static_cast<int4*>(results), ri);
+                }
                 state = kIdle;
             }
             const uint32_t leader = __ffs(want_mask) - 1u;
@@ -1036,14 +1049,20 @@ __global__ void __launch_bounds__(kBlock, PER_SM) k_occluded_bvh8(
                     const float4 r0 = rays[2 * (size_t)idx + 0];
                     const float4 r1 = rays[2 * (size_t)idx + 1];
                     if (!(r1.w >= r0.w)) {  // empty interval: nothing in the way, lane stays idle
-                        occluded[idx] = -1;
+                        if (RECORD)
+                            write_miss(static_cast<int4*>(results), idx);
+                        else
+                            static_cast<int32_t*>(results)[idx] = -1;
                     } else {
                         ri = idx;
                         state = kTracing;
                         r = setup_ray(r0, r1);
                         s_ray[threadIdx.x] = ray_shared(r);
                         s_tmax[threadIdx.x] = r1.w;
-                        s_hit[threadIdx.x] = 0u;
+                        if (RECORD)
+                            s_best[threadIdx.x] = ~0ull;
+                        else
+                            s_hit[threadIdx.x] = 0u;
                         tmax = r1.w;
                         sp = 0;
                         ng = make_uint2(0u, 0x80000000u);
@@ -1056,7 +1075,7 @@ __global__ void __launch_bounds__(kBlock, PER_SM) k_occluded_bvh8(
         if (__ballot_sync(0xffffffffu, state != kIdle || !exhausted) == 0u) break;
 
         uint32_t leaf = 0, leaf2 = 0, from = 0, from2 = 0;
-        const uint32_t few = __any_sync(0xffffffffu, exhausted) ? 1u : kFewOccluded;
+        const uint32_t few = __any_sync(0xffffffffu, exhausted) ? 1u : RECORD ? kFewLanes : kFewOccluded;
         for (uint32_t st = 0; st < steps; ++st) {
             const bool go = state == kTracing && ng.y > 0x00FFFFFFu && leaf2 == 0u && __popc(leaf) <= MORE;
             if (st >= 1u && (uint32_t)__popc(__ballot_sync(0xffffffffu, go)) < few) break;
@@ -1090,7 +1109,8 @@ __global__ void __launch_bounds__(kBlock, PER_SM) k_occluded_bvh8(
         uint4 meta = make_uint4(0u, 0u, 0u, 0u), meta2 = meta;
         if (leaf != 0u) meta = __ldg(reinterpret_cast<const uint4*>(nodes + 5 * (size_t)from + 1));
         if (leaf2 != 0u) meta2 = __ldg(reinterpret_cast<const uint4*>(nodes + 5 * (size_t)from2 + 1));
-        const uint32_t cnt = leaf_count(leaf, meta.z, meta.w) + leaf_count(leaf2, meta2.z, meta2.w);
+        const uint32_t cnt1 = leaf_count(leaf, meta.z, meta.w);
+        const uint32_t cnt = cnt1 + leaf_count(leaf2, meta2.z, meta2.w);
         uint32_t incl = cnt;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
@@ -1101,6 +1121,7 @@ __global__ void __launch_bounds__(kBlock, PER_SM) k_occluded_bvh8(
         if (total != 0u) {
             uint32_t pos = incl - cnt;
             const uint32_t owner = lane << kRecBits;
+            if (RECORD) s_second[threadIdx.x] = pos + cnt1;
             while (leaf != 0u) {
                 const uint32_t bit = (uint32_t)__ffs(leaf) - 1u;
                 leaf &= leaf - 1u;
@@ -1116,21 +1137,47 @@ __global__ void __launch_bounds__(kBlock, PER_SM) k_occluded_bvh8(
                 }
             }
             __syncwarp();
-            for (uint32_t j = lane; j < total; j += 32u) {
-                const uint32_t w = task[j];
-                const uint32_t o = wbase + (w >> kRecBits);
-                const uint32_t rec = w & ((1u << kRecBits) - 1u);
-                const RayS rs = s_ray[o];
-                const Uvw q = tri_uvw(rs, __ldg(&tris[3 * rec + 0]), __ldg(&tris[3 * rec + 1]), __ldg(&tris[3 * rec + 2]));
-                if (q.edge_ok && q.det != 0.0f) {
-                    const float t = __fdiv_rn(q.T, q.det);
-                    if (t >= rs.tmin && t <= s_tmax[o]) s_hit[o] = 1u;
+            for (uint32_t j0 = 0; j0 < total; j0 += 32u) {
+                const uint32_t j = j0 + lane;
+                uint32_t o = 0;
+                bool cand = false;
+                unsigned long long hk = 0;
+                uint4 h = make_uint4(0u, 0u, 0u, 0u);
+                if (j < total) {
+                    const uint32_t w = task[j];
+                    o = wbase + (w >> kRecBits);
+                    const uint32_t rec = w & ((1u << kRecBits) - 1u);
+                    const RayS rs = s_ray[o];
+                    const float4 a4 = __ldg(&tris[3 * rec + 0]), b4 = __ldg(&tris[3 * rec + 1]);
+                    const float4 c4 = __ldg(&tris[3 * rec + 2]);
+                    const Uvw q = tri_uvw(rs, a4, b4, c4);
+                    if (q.edge_ok && q.det != 0.0f) {
+                        const float t = __fdiv_rn(q.T, q.det);
+                        if (t >= rs.tmin && t <= s_tmax[o]) {
+                            if (!RECORD) {
+                                s_hit[o] = 1u;
+                            } else {
+                                hk = any_key(t, __float_as_uint(c4.w), j >= s_second[o]);
+                                if (hk < s_best[o]) {  // a stale read can only be larger
+                                    atomicMin(&s_best[o], hk);
+                                    cand = true;
+                                    const float u = __fdiv_rn(q.V, q.det), v = __fdiv_rn(q.W, q.det);
+                                    h = make_uint4(__float_as_uint(a4.w), __float_as_uint(b4.w), pack_unorm2x16(u, v),
+                                                   __float_as_uint(t));
+                                }
+                            }
+                        }
+                    }
+                }
+                if (RECORD) {  // the best of the round records its fields (keys are unique)
+                    __syncwarp();
+                    if (cand && s_best[o] == hk) s_rec[o] = h;
                 }
             }
             __syncwarp();
         }
         if (state == kTracing) {
-            if (s_hit[threadIdx.x] != 0u)
+            if (RECORD ? s_best[threadIdx.x] != ~0ull : s_hit[threadIdx.x] != 0u)
                 state = kBlocked;
             else if (ng.y <= 0x00FFFFFFu)
                 state = kFree;
@@ -1151,9 +1198,9 @@ __global__ void __launch_bounds__(kBlock, PER_SM) k_occluded_bvh8(
 // traces on different streams do not share a counter.
 static std::atomic<uint32_t> g_slot{0};
 // Resident blocks per SM: [closest] for the per-lane kernel, [2 + closest]
-// for the cooperative one, [4 + closest] for its small-wavefront form; [6] and
-// [7] for the occlusion kernel and its small-wavefront form.
-static int g_blocks_per_sm[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+// for the cooperative one, [4 + closest] for its small-wavefront form; [6 + 2
+// record] for the any-hit kernel, [7 + 2 record] for its small-wavefront form.
+static int g_blocks_per_sm[10] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0};
 static int g_num_sms = 0;
 static uint32_t g_refill = 6;  // 4 to 8 within 1 % on bounce-1 rays, 6 the best sum
 
@@ -1208,10 +1255,11 @@ cudaError_t trace_prepare() {
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_blocks_per_sm[0], k_trace_bvh8<false, false>, kBlock, 0);
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_blocks_per_sm[1], k_trace_bvh8<true, false>, kBlock, 0);
-    const void* coop[6] = {(const void*)k_trace_bvh8_coop<false, false, 4>, (const void*)k_trace_bvh8_coop<true, false, 4>,
+    const void* coop[8] = {(const void*)k_trace_bvh8_coop<false, false, 4>, (const void*)k_trace_bvh8_coop<true, false, 4>,
                            (const void*)k_trace_bvh8_coop<false, false, 3>, (const void*)k_trace_bvh8_coop<true, false, 3>,
-                           (const void*)k_occluded_bvh8<4>, (const void*)k_occluded_bvh8<3>};
-    for (int k = 0; k < 6 && e == cudaSuccess; ++k)
+                           (const void*)k_any_bvh8<false, 4>, (const void*)k_any_bvh8<false, 3>,
+                           (const void*)k_any_bvh8<true, 4>, (const void*)k_any_bvh8<true, 3>};
+    for (int k = 0; k < 8 && e == cudaSuccess; ++k)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&g_blocks_per_sm[2 + k], coop[k], kBlock, 0);
     if (e == cudaSuccess) g_num_sms = sms;
     return e;
@@ -1253,7 +1301,13 @@ cudaError_t launch_trace(const SceneDevice& sc, int kind, const wfpt_ray* rays, 
         const uint32_t lanes = pgrid * kBlock;
         if (grid < pgrid) pgrid = grid;
         uint32_t* work = own_work ? own_work : sc.work + 16 * (g_slot.fetch_add(1) % kWorkSlots);
-        if (coop) {
+        if (coop && !closest && !g_count && kernel_batch(false) <= 1u) {
+            const unsigned resident = std::max(1u, (unsigned)(g_num_sms * g_blocks_per_sm[small ? 9 : 8]));
+            auto k8 = small ? k_any_bvh8<true, 3> : k_any_bvh8<true, 4>;
+            k8<<<std::min((n + kBlock - 1) / kBlock, resident), kBlock, 0, s>>>(
+                sc.bvh8_nodes, sc.bvh8_tris, rr, out, ray_index, n, n_dev, work, g_refill,
+                kernel_steps(false, n, resident * kBlock));
+        } else if (coop) {
             auto k8 = closest ? (g_count ? k_trace_bvh8_coop<true, true, 4> : k_trace_bvh8_coop<true, false, 4>)
                               : (g_count ? k_trace_bvh8_coop<false, true, 4> : k_trace_bvh8_coop<false, false, 4>);
             if (small) {
@@ -1308,7 +1362,7 @@ cudaError_t launch_occluded(const SceneDevice& sc, int kind, const wfpt_ray* ray
         }
         const bool small = n < kCoopLargeMin && !shared;
         const unsigned resident = std::max(1u, (unsigned)(g_num_sms * g_blocks_per_sm[small ? 7 : 6]));
-        auto k8 = small ? k_occluded_bvh8<3> : k_occluded_bvh8<4>;
+        auto k8 = small ? k_any_bvh8<false, 3> : k_any_bvh8<false, 4>;
         k8<<<std::min(grid, resident), kBlock, 0, s>>>(sc.bvh8_nodes, sc.bvh8_tris, rr, occluded, ray_index, n, n_dev,
                                                        work, g_refill, kernel_steps(false, n, resident * kBlock));
     } else {
