@@ -442,9 +442,9 @@ wfpt_status wfpt_reconstruct_shadow(const wfpt_hit* shadow_results, const int32_
     WFPT_REQUIRE(num_samples >= 1 && num_samples <= 1024, "num_samples must be in [1, 1024]");
     WFPT_REQUIRE(batch_size == 0 || (shadow_results && index_to_pixel && index_to_slot && in_pixels && out_pixels),
                  "null buffer");
-    return from_cuda(wfpt::launch_reconstruct_shadow(reinterpret_cast<const int32_t*>(shadow_results), 4, index_to_pixel, index_to_slot, in_pixels,
-                                                     out_pixels, batch_begin, batch_size, n_in_dev, num_samples,
-                                                     replace, S(stream)));
+    return from_cuda(wfpt::launch_reconstruct_shadow(reinterpret_cast<const int32_t*>(shadow_results), 4,
+                                                     index_to_pixel, index_to_slot, in_pixels, out_pixels, batch_begin,
+                                                     batch_size, n_in_dev, num_samples, replace, S(stream)));
 }
 
 wfpt_status wfpt_count_hits(const wfpt_hit* results, uint32_t n, const uint32_t* n_dev, uint32_t* count_dev,

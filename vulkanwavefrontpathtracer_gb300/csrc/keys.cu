@@ -59,7 +59,8 @@ __device__ __forceinline__ void store_record(uint4* p, uint4 v, uint64_t pol) {
                  : "memory");
 }
 
-// reorderRays.comp:37-45.
+// reorderRays.comp:37-45.  out_i2s (nullable, here and below): a renderer's path
+// rays are never looked up by index (2.07M rays 39 -> 31 us without).
 template <bool STREAM>
 __global__ void k_reorder(const uint32_t* __restrict__ idx, const uint4* __restrict__ in_rays,
                           uint4* __restrict__ out_rays, const int32_t* __restrict__ in_s2i,
@@ -85,7 +86,7 @@ __global__ void k_reorder(const uint32_t* __restrict__ idx, const uint4* __restr
     } else {
         out_s2i[i] = index;
     }
-    out_i2s[index] = (int32_t)i;
+    if (out_i2s != nullptr) out_i2s[index] = (int32_t)i;
 }
 
 // The same gather for records of C x 16 bytes (ray records with a payload,
@@ -251,11 +252,11 @@ static cudaError_t launch_maps(const uint32_t* idx, const int32_t* in_s2i, int32
         const uint32_t lo = r * step;
         gather<<<grid, kBlock, 0, s>>>(idx, in_s2i, out_s2i, n, n_dev, lo, r + 1 == ranges ? 0xFFFFFFFFu - lo : step);
     }
-    for (uint32_t r = 0; r < ranges; ++r) {
+    for (uint32_t r = 0; r < ranges && out_i2s != nullptr; ++r) {
         const uint32_t lo = r * step;
         scatter<<<grid, kBlock, 0, s>>>(out_s2i, out_i2s, n, n_dev, lo, r + 1 == ranges ? 0xFFFFFFFFu - lo : step);
     }
-    count_launch(2 * ranges);
+    count_launch(out_i2s != nullptr ? 2 * ranges : ranges);
     return cudaGetLastError();
 }
 

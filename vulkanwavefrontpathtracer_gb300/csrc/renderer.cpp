@@ -493,7 +493,8 @@ struct wfpt_renderer {
         if (reorder) {
             if ((e = timed(s, total, C_REORDER, log, [&]() {
                      return wfpt::launch_reorder(rb.idx.as<uint32_t>(), rb.rays_cur(), rb.rays_out(), rb.s2i_cur(),
-                                                 rb.s2i_out(), rb.i2s_out(), n, n_dev, s);
+                                                 rb.s2i_out(), query == kClosestHit ? nullptr : rb.i2s_out(), n, n_dev,
+                                                 s);
                  })) != cudaSuccess)
                 return e;
             rb.swap();
@@ -538,6 +539,9 @@ struct wfpt_renderer {
                             uint32_t* batch_counters, cudaStream_t s, int kind, int slot_log) {
         const int S = cfg.num_shadow_samples;
         const Query query = wfpt::occluded_ready(*wfpt::scene_device(scene), kind) ? kOccluded : kAnyHit;
+        // Shadow rays that are not reordered need no maps (2.07M hits: generation
+        // 41 -> 35 us, reconstruction 51 -> 47 us).
+        const bool maps = cfg.sort_shadow_rays != 0 && cfg.reorder_shadow_rays != 0;
         const int hit_stride = query == kOccluded ? 1 : 4;  // words of a result
         const uint32_t batch_diff = (uint32_t)(kMaxBatch / S);
         cudaError_t e;
@@ -552,8 +556,8 @@ struct wfpt_renderer {
                 const uint32_t bb = b * batch_diff, bs = std::min(batch_diff, n_in - bb);
                 sl.rb.swapped = false;
                 cudaError_t r = wfpt::launch_raygen_shadow(
-                    seeds.as<uint32_t>(), in_rays, in_res, sl.rb.rays_cur(), sl.rb.s2i_cur(), sl.rb.i2s_cur(), light,
-                    cfg.shadow_radius, (int)bb, (int)bs, n_in_dev, S, sl.stream,
+                    seeds.as<uint32_t>(), in_rays, in_res, sl.rb.rays_cur(), maps ? sl.rb.s2i_cur() : nullptr,
+                    maps ? sl.rb.i2s_cur() : nullptr, light, cfg.shadow_radius, (int)bb, (int)bs, n_in_dev, S, sl.stream,
                     n_in_dev ? batch_counters + (b % used) : nullptr);
                 return r != cudaSuccess ? r : cudaEventRecord(sl.ev_rg, sl.stream);
             };
@@ -565,7 +569,8 @@ struct wfpt_renderer {
                                            sl.work.as<uint32_t>(), sl.scratch, kind);
                 if (r == cudaSuccess && b < (uint32_t)used) r = cudaStreamWaitEvent(sl.stream, ev_shade, 0);
                 if (r != cudaSuccess) return r;
-                return wfpt::launch_reconstruct_shadow(sl.rb.results.as<int32_t>(), hit_stride, in_s2i, sl.rb.i2s_cur(),
+                return wfpt::launch_reconstruct_shadow(sl.rb.results.as<int32_t>(), hit_stride, in_s2i,
+                                                       maps ? sl.rb.i2s_cur() : nullptr,
                                                        in_pixels, out_pixels, (int)bb, (int)bs, n_in_dev, S, 0,
                                                        sl.stream);
             };
@@ -603,7 +608,8 @@ struct wfpt_renderer {
             shadow.swapped = false;
             if ((e = timed(s, T_SHADOW, C_NONE, -1, [&]() {
                      return wfpt::launch_raygen_shadow(seeds.as<uint32_t>(), in_rays, in_res, shadow.rays_cur(),
-                                                       shadow.s2i_cur(), shadow.i2s_cur(), light, cfg.shadow_radius,
+                                                       maps ? shadow.s2i_cur() : nullptr,
+                                                       maps ? shadow.i2s_cur() : nullptr, light, cfg.shadow_radius,
                                                        (int)bb, (int)bs, n_in_dev, S, s, n_sh_dev);
                  })) != cudaSuccess)
                 return e;
@@ -611,7 +617,8 @@ struct wfpt_renderer {
                                 cfg.reorder_shadow_rays != 0, query, s, work.as<uint32_t>(), sort_scratch, kind,
                                 T_SHADOW, slot_log)) != cudaSuccess)
                 return e;
-            if ((e = wfpt::launch_reconstruct_shadow(shadow.results.as<int32_t>(), hit_stride, in_s2i, shadow.i2s_cur(),
+            if ((e = wfpt::launch_reconstruct_shadow(shadow.results.as<int32_t>(), hit_stride, in_s2i,
+                                                     maps ? shadow.i2s_cur() : nullptr,
                                                      in_pixels, out_pixels, (int)bb, (int)bs, n_in_dev, S, 0, s)) !=
                 cudaSuccess)
                 return e;

@@ -173,7 +173,9 @@ __device__ __forceinline__ uint32_t next_task(uint32_t task) {
 }
 
 // raygenShadow.comp:82-136.  Output rays of input task t occupy
-// [S*t, S*t+S) of the batch-local output buffer.
+// [S*t, S*t+S) of the batch-local output buffer.  The maps are nullable: a
+// renderer's shadow rays that stay in this order need none (8 bytes a ray
+// written here and 4 read again in reconstructShadow).
 template <bool LOOP>
 __global__ void k_raygen_shadow(const uint32_t* __restrict__ seeds,
                                 const float4* __restrict__ in_rays,
@@ -226,8 +228,8 @@ __global__ void k_raygen_shadow(const uint32_t* __restrict__ seeds,
             float tmax = tri == -1 ? -1.0f : length(dir);
             store_ray(out_rays, ray_index, make_float4(origin.x, origin.y, origin.z, EPS),
                       make_float4(nd.x, nd.y, nd.z, tmax), wide);
-            out_s2i[ray_index] = ray_index;
-            out_i2s[ray_index] = ray_index;
+            if (out_s2i != nullptr) out_s2i[ray_index] = ray_index;
+            if (out_i2s != nullptr) out_i2s[ray_index] = ray_index;
             ++ray_index;
         }
     }
@@ -524,7 +526,7 @@ __global__ void k_reconstruct_smooth(const float4* __restrict__ rays, const int4
 
 // ---------------------------------------------------- reconstructShadow
 // reconstructShadow.comp:39-59.  hits: the first words of the results, `stride`
-// words apart.
+// words apart.  i2s null: shadow rays in the order of their generation.
 template <bool LOOP>
 __global__ void k_reconstruct_shadow(const int32_t* __restrict__ hits, int stride, const int32_t* __restrict__ i2p,
                                      const int32_t* __restrict__ i2s,
@@ -542,7 +544,8 @@ __global__ void k_reconstruct_shadow(const int32_t* __restrict__ hits, int strid
         float4 ip = in_pixels[pixel];
         float shadow = 0.0f;
         for (int i = 0; i < S; ++i) {
-            int slot = i2s[(int)task * S + i];
+            const int ray = (int)task * S + i;
+            const int slot = i2s != nullptr ? i2s[ray] : ray;
             if (hits[(size_t)slot * stride] == -1) shadow = __fadd_rn(shadow, 1.0f);
         }
         shadow = __fdiv_rn(shadow, (float)S);
