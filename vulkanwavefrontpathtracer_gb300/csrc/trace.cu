@@ -197,6 +197,41 @@ __device__ __forceinline__ void box2(const RayT& r, float lox, float hix, float 
     hit = tn <= tf * kBoxSlack;
 }
 
+// An inner node: goes on to the nearer child hit (the other on the stack) or to
+// the top of the stack; false when that is empty.
+__device__ __forceinline__ void bvh2_step(const float4* __restrict__ nodes, const RayT& r, float tcur, int& node,
+                                          int* stack, int& sp, bool& done) {
+    float4 a, b, c, lf;
+    load32(nodes + 4 * (size_t)node, a, b);
+    load32(nodes + 4 * (size_t)node + 2, c, lf);
+    const int2 l = make_int2(__float_as_int(lf.x), __float_as_int(lf.y));
+    float t0, t1;
+    bool h0, h1;
+    box2(r, a.x, a.y, a.z, a.w, c.x, c.y, tcur, t0, h0);
+    box2(r, b.x, b.y, b.z, b.w, c.z, c.w, tcur, t1, h1);
+    if (h0 && h1) {
+        int nearc = l.x, farc = l.y;
+        if (t1 < t0) {
+            nearc = l.y;
+            farc = l.x;
+        }
+        if (sp < kStack2) {
+            stack[sp++] = farc;
+        } else {
+            raise_status(kErrBounds);
+        }
+        node = nearc;
+    } else if (h0) {
+        node = l.x;
+    } else if (h1) {
+        node = l.y;
+    } else if (sp == 0) {
+        done = true;
+    } else {
+        node = stack[--sp];
+    }
+}
+
 // One ray, traced by one thread.  OCCLUDED: results is an array of words, which
 // get 0 for a hit and -1 for a miss.
 template <bool CLOSEST, bool COUNT, bool OCCLUDED = false>
@@ -224,37 +259,8 @@ __device__ __forceinline__ void trace_bvh2_ray(const float4* __restrict__ nodes,
         // Inner nodes.
         while (node >= 0) {
             if (COUNT) ++c_nodes;
-            float4 a, b, c, lf;
-            load32(nodes + 4 * (size_t)node, a, b);
-            load32(nodes + 4 * (size_t)node + 2, c, lf);
-            const int2 l = make_int2(__float_as_int(lf.x), __float_as_int(lf.y));
-            float t0, t1;
-            bool h0, h1;
-            box2(r, a.x, a.y, a.z, a.w, c.x, c.y, h.t, t0, h0);
-            box2(r, b.x, b.y, b.z, b.w, c.z, c.w, h.t, t1, h1);
-            if (h0 && h1) {
-                int nearc = l.x, farc = l.y;
-                if (t1 < t0) {
-                    nearc = l.y;
-                    farc = l.x;
-                }
-                if (sp < kStack2) {
-                    stack[sp++] = farc;
-                } else {
-                    raise_status(kErrBounds);
-                }
-                node = nearc;
-            } else if (h0) {
-                node = l.x;
-            } else if (h1) {
-                node = l.y;
-            } else {
-                if (sp == 0) {
-                    done = true;
-                    break;
-                }
-                node = stack[--sp];
-            }
+            bvh2_step(nodes, r, h.t, node, stack, sp, done);
+            if (done) break;
         }
         if (done) break;
         // Leaves.
@@ -315,23 +321,30 @@ __global__ void __launch_bounds__(BLOCK, PER_SM) k_trace_bvh2(const float4* __re
     trace_bvh2_ray<CLOSEST, COUNT, OCCLUDED>(nodes, tris, rays, results, ray_index ? ray_index[i] : i);
 }
 
-// The same with resident warps that take 32 rays at a time, the first by
-// warp number, the next from work[0]; work[1] counts finished warps, and the
-// last resets both.  For wavefronts whose size only the device knows: a
-// bounce's count is often far below its capacity n, and the launch above pays
-// for every empty block (68 us at n = 8.3M, 133 us for its shadow rays; this
-// one 8 us).  And for very large ones: 6.4M city bounce-1 rays 1464 -> 1388 us
-// closest, 1333 -> 1265 us any hit, 8.3M camera rays 714 -> 702 us.  At full
-// counts in between it is 2-5 % faster on incoherent rays (courtyard closest
-// 1648 -> 1613 us) but 3-20 % slower on camera rays (2.07M: 632 -> 651 us, 262K:
-// 159 -> 192 us), whose sizes the host knows; asking for the next 32 rays
-// before tracing the current ones (which binds them to a warp that may be
-// slow) made those worse still (706 and 239 us).  Only for callers that bring
-// their own counters: the scene's are handed out in turn, and two replays of
-// one captured launch at a time would share a pair.
+// The same with resident warps whose lanes take new rays (work[0] hands them
+// out; work[1] counts finished warps, and the last resets both), for a
+// renderer's bounce and shadow rays.  Incoherent rays take very different
+// numbers of steps, and above a warp waits for its longest one with 6 to 9 lanes
+// busy.  Here idle lanes get new rays once there are kBvh2Refill of them, and the
+// node steps, asked about every fourth time, end when fewer than kBvh2Few lanes
+// take one, so that leaves are tested by many lanes at once: 2.07M courtyard
+// bounce-1 rays 1648 -> 1220 us, any hit 1567 -> 1399; the city's 1.6M 423 ->
+// 344 and 385 -> 304, 6.4M 1462 -> 1186 and 1331 -> 1057.  Rays that go together
+// lose by it (camera rays 632 -> 764 and 713 -> 813 us): those keep the kernel
+// above, and so do wavefronts smaller than the lanes of this one, which have
+// nothing to refill with (262K rays 296 -> 252 us, 228K 278 -> 236, 120K 173 ->
+// 189).  It also runs no empty blocks where a bounce's count is far below its
+// capacity (68 us at n = 8.3M, 133 us for its shadow rays).  Refill 8, 16, 24,
+// 28: 16.4, 15.2, 15.1, 15.9 ms for a 4K city frame that takes 15.1 ms; few 2, 4,
+// 10: 15.6, 15.1, 15.2; a vote per step 15.5, every second 15.3; four blocks per
+// SM 17.0; two or four leaves in a row 15.6.
+//
+// It needs counters of the caller's own: a scene's are handed out in turn, and
+// two replays of one captured launch at a time would share a pair.
 constexpr int kBvh2PerSm = 5;
 constexpr unsigned kBvh2Grid = 152 * kBvh2PerSm;
-constexpr uint32_t kBvh2PersistentMin = 1u << 22;  // with a host-side count
+constexpr uint32_t kBvh2RefillMin = 152 * kBvh2PerSm * kBlock;
+constexpr int kBvh2Refill = 20, kBvh2Steps = 32, kBvh2Few = 6;
 template <bool CLOSEST, bool COUNT, bool OCCLUDED = false>
 __global__ void __launch_bounds__(kBlock, kBvh2PerSm) k_trace_bvh2_persistent(
     const float4* __restrict__ nodes, const float4* __restrict__ tris, const float4* __restrict__ rays,
@@ -339,19 +352,86 @@ __global__ void __launch_bounds__(kBlock, kBvh2PerSm) k_trace_bvh2_persistent(
     const uint32_t* __restrict__ n_dev, uint32_t* __restrict__ work) {
     const uint32_t count = load_count(n, n_dev);
     const uint32_t lane = threadIdx.x & 31;
-    const uint32_t warps = gridDim.x * (kBlock / 32);
-    const uint32_t chunks = (count + 31u) / 32u;
-    uint32_t chunk = (blockIdx.x * kBlock + threadIdx.x) >> 5;
-    while (chunk < chunks) {
-        const uint32_t i = chunk * 32u + lane;
-        if (i < count)
-            trace_bvh2_ray<CLOSEST, COUNT, OCCLUDED>(nodes, tris, rays, results, ray_index ? ray_index[i] : i);
-        uint32_t next = 0;
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    RayT r;
+    HitS h{0.0f, 0xFFFFFFFFu, 0u};
+    bool active = false, found = false, exhausted = false;
+    uint32_t ri = 0, c_nodes = 0, c_tris = 0, c_rays = 0;
+    int stack[kStack2];
+    int sp = 0, node = 0;
+    for (;;) {
+        const bool want = !active && !exhausted;
+        const uint32_t want_mask = __ballot_sync(0xffffffffu, want);
+        const uint32_t busy_mask = __ballot_sync(0xffffffffu, active);
+        if (want_mask != 0u && (__popc(want_mask) >= kBvh2Refill || busy_mask == 0u)) {
+            const uint32_t leader = __ffs(want_mask) - 1u;
+            uint32_t base = 0;
+            if (lane == leader) base = atomicAdd(&work[0], __popc(want_mask));
+            base = __shfl_sync(0xffffffffu, base, leader);
+            if (want) {
+                const uint32_t i = base + __popc(want_mask & lt_mask);
+                if (i < count) {
+                    ri = ray_index ? ray_index[i] : i;
+                    const float4 r0 = rays[2 * (size_t)ri + 0];
+                    const float4 r1 = rays[2 * (size_t)ri + 1];
+                    if (!(r1.w >= r0.w)) {  // empty interval: miss, lane stays idle
+                        if (OCCLUDED)
+                            reinterpret_cast<int32_t*>(results)[ri] = -1;
+                        else
+                            write_miss(results, ri);
+                    } else {
+                        r = setup_ray(r0, r1);
+                        h = HitS{r1.w, 0xFFFFFFFFu, 0u};
+                        active = true;
+                        found = false;
+                        sp = 0;
+                        node = 0;
+                    }
+                } else {
+                    exhausted = true;
+                }
+            }
+        }
+        if (__ballot_sync(0xffffffffu, active || !exhausted) == 0u) break;
+        // Inner nodes, until few lanes are at one.
+        bool done = false;
+        for (int st = 0; st < kBvh2Steps; ++st) {
+            const bool go = active && !done && node >= 0;
+            if ((st & 3) == 3 && __popc(__ballot_sync(0xffffffffu, go)) < kBvh2Few) break;
+            if (go) {
+                if (COUNT) ++c_nodes;
+                bvh2_step(nodes, r, h.t, node, stack, sp, done);
+            }
+        }
+        // A leaf of each lane that has come to one.
+        if (active && !done && node < 0) {
+            const uint32_t code = ~(uint32_t)node;
+            const uint32_t first = code >> 3, cnt = (code & 7u) + 1u;
+            for (uint32_t k = 0; k < cnt; ++k) {
+                if (COUNT) ++c_tris;
+                if (intersect_tri(r, tris, first + k, h)) {
+                    found = true;
+                    if (!CLOSEST) break;
+                }
+            }
+            if ((!CLOSEST && found) || sp == 0)
+                done = true;
+            else
+                node = stack[--sp];
+        }
+        if (active && done) {
+            if (OCCLUDED)
+                reinterpret_cast<int32_t*>(results)[ri] = found ? 0 : -1;
+            else
+                write_hit(results, ri, r, tris, h, found);
+            active = false;
+            if (COUNT) ++c_rays;
+        }
         __syncwarp();
-        if (lane == 0) next = atomicAdd(&work[0], 1u);
-        chunk = warps + __shfl_sync(0xffffffffu, next, 0);
     }
+    if (COUNT) add_counts(c_nodes, c_tris, c_rays, 0u);
     if (lane == 0) {
+        const uint32_t warps = gridDim.x * (kBlock / 32);
         __threadfence();
         if (atomicAdd(&work[1], 1u) == warps - 1u) {
             work[0] = 0u;
@@ -1323,7 +1403,7 @@ cudaError_t launch_trace(const SceneDevice& sc, int kind, const wfpt_ray* rays, 
                                         g_postpone);
         }
     } else {
-        if (own_work != nullptr && n >= (n_dev != nullptr ? kBvh2SmallMin : kBvh2PersistentMin)) {
+        if (own_work != nullptr && n_dev != nullptr && n >= kBvh2RefillMin) {
             auto k2 = closest ? (g_count ? k_trace_bvh2_persistent<true, true> : k_trace_bvh2_persistent<true, false>)
                               : (g_count ? k_trace_bvh2_persistent<false, true> : k_trace_bvh2_persistent<false, false>);
             k2<<<std::min(grid, kBvh2Grid), kBlock, 0, s>>>(sc.bvh2_nodes, sc.bvh2_tris, rr, out, ray_index, n, n_dev,
@@ -1368,7 +1448,7 @@ cudaError_t launch_occluded(const SceneDevice& sc, int kind, const wfpt_ray* ray
     } else {
         int4* out = reinterpret_cast<int4*>(occluded);
         constexpr int B = kBvh2SmallBlock, P = kBvh2SmallPerSm;
-        if (n >= (n_dev != nullptr ? kBvh2SmallMin : kBvh2PersistentMin))
+        if (n >= kBvh2RefillMin)
             k_trace_bvh2_persistent<false, false, true><<<std::min(grid, kBvh2Grid), kBlock, 0, s>>>(
                 sc.bvh2_nodes, sc.bvh2_tris, rr, out, ray_index, n, n_dev, work);
         else if (n >= kBvh2SmallMin)
