@@ -71,17 +71,15 @@ WORKLOAD_NAME = ("courtyard: 268,304 triangles, 1920x1080, 1 spp, path rays, 8 b
 METRIC = "Mrays/s per bounce, chosen vs plain form; radix sort+reorder HBM GB/s vs peak"
 # DRAM bytes (read + write) per ray of the full-size bounce-1 BVH8 traversal
 # launches (2,073,600 sorted closest-hit path rays, 4,147,200 any-hit shadow
-# rays), median of 12 launches each from one ncu capture of
-# `bench.py --micro-only` (dram__bytes_read.sum + dram__bytes_write.sum,
-# cold caches): closest 87.6 MB + 10.2 MB, any-hit 152.9 MB + 40.6 MB.
-TRACE_DRAM_BYTES_PER_RAY = {"any": 46.64, "closest": 47.20}
-# Warp instructions per ray of the courtyard's bounce-1 BVH8 traversal
-# (sm__inst_executed.sum / rays of one launch each, `bench.py --trace-profile`
-# under ncu at 960x540: 288,619,160 for 518,400 sorted closest-hit path rays,
-# 337,241,928 for 1,036,800 any-hit shadow rays).  With the live launch time
+# rays), from an ncu capture of `bench.py --micro-only` (dram__bytes_read.sum +
+# dram__bytes_write.sum, cold caches): closest 86.7 MB + 10.1 MB, any hit
+# 152.4 MB + 40.3 MB.
+TRACE_DRAM_BYTES_PER_RAY = {"any": 46.47, "closest": 46.68}
+# Warp instructions per ray of the same launches (sm__inst_executed.sum / rays:
+# 872,800,000 closest hit, 1,031,600,000 any hit).  With the live launch time
 # they give the issue rate; the issue peak is 152 SMs x 4 schedulers x one
 # warp instruction per clock at the sampled SM clock.
-TRACE_WARP_INST_PER_RAY = {"any": 325.27, "closest": 556.75}
+TRACE_WARP_INST_PER_RAY = {"any": 248.75, "closest": 420.91}
 NUM_SMS = 152
 
 
@@ -423,10 +421,10 @@ def run_ours(args):
             return {"bound": "issue", "achieved": round(ach_g, 1), "peak": round(peak_g, 1),
                     "unit": "G warp instructions/s", "frac": round(ach_g / peak_g, 3),
                     "warp_inst_per_ray": TRACE_WARP_INST_PER_RAY[kind], "sm_mhz": mhz,
-                    "source": "warp instructions per ray from one ncu launch of the same traversal at 960x540 "
+                    "source": "warp instructions per ray from an ncu capture of the same launches "
                               "(sm__inst_executed.sum); launch time measured here"}
 
-        roof = trace_roof(micro["trace_shadow"], "k_trace_bvh8_coop<any-hit> (bounce-1 shadow rays, 2 per path ray)",
+        roof = trace_roof(micro["trace_shadow"], "k_any_bvh8 (bounce-1 shadow rays, 2 per path ray)",
                           "any")
         roof["issue_roofline"] = issue_roof(micro["trace_shadow"], "any")
         closest_roof = trace_roof(micro["trace_chosen"],
@@ -1059,8 +1057,8 @@ def reorder_row(api, dev, stream, n=1 << 24, reps=5):
     ms = timed(lambda: api.reorder_records(perm, wide, wide_out, s2i, os2i, oi2s))
     res["rec48"] = {"ms": round(ms, 4), "gbs": round(112.0 * n / (ms * 1e-3) / 1e9, 1),
                     "frac": round(112.0 * n / (ms * 1e-3) / 1e9 / hbm, 3), "alg_bytes_per_ray": 112}
-    res["note"] = ("random 32/48-byte record gathers and 4-byte slot-map accesses: about 3.7x the algorithmic "
-                   "bytes reach DRAM (sector and burst granularity), the kernel's ceiling beyond L2")
+    res["note"] = ("random 32/48-byte record gathers, bound by DRAM's access granularity, then the slot maps in "
+                   "ranges that stay in L2")
     del rays, wide, wide_out, perm, s2i, os2i, oi2s
     torch.cuda.empty_cache()
     return res

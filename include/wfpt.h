@@ -137,11 +137,13 @@ uint64_t wfpt_kernel_launch_count(void);
  *                          iteration takes up to twice this many node steps
  *                          per lane, each lane until a second node has
  *                          handed it triangles (1..8, default 2)
- *   "trace.bvh8.any_batch" the same for any-hit rays (default 1)
+ *   "trace.bvh8.any_batch" the same for any-hit rays (default 1; a frame's
+ *                          shadow rays are tested after every iteration)
  *   "trace.bvh8.any_steps" the same for any-hit rays, two node steps more
  *                          (default 3: up to eight)
  *   "sort.tiles"           radix sort tile size: 0 = by problem size
- *                          (default), 1 = small tiles, 2 = large tiles,
+ *                          (default; tiny tiles up to 393,216 pairs), 1 =
+ *                          small tiles, 2 = large tiles,
  *                          3 = extra-large tiles (32-bit keys; 64-bit keys
  *                          take the large ones)
  *   "sort.digit_bits"      radix digit width per pass: 8 (default) or 4
@@ -233,8 +235,9 @@ size_t wfpt_sort_scratch_bytes(uint32_t max_n, int key_bits);
  * uint64_t; only the low key_bits bits are sorted on (ceil(key_bits/8)
  * passes).  The result is left in keys/values, like the reference.  Values
  * are uint32.  Ordering equals a stable sort by key.  The call enqueues a
- * memset of the scratch, a histogram kernel and one kernel per pass; the
- * pass kernels are launched with programmatic stream serialisation after
+ * memset of the scratch (up to 393,216 pairs a kernel that clears it), a
+ * histogram kernel and one kernel per pass; the pass kernels (and the
+ * histogram after the clearing kernel) are launched with programmatic stream serialisation after
  * the library's own previous kernel (they start as it drains and wait for
  * it before reading), so a stream capture records programmatic edges
  * between them.  Work the caller enqueues after the sort starts only when
