@@ -1,6 +1,7 @@
 // C ABI of libwfpt: argument checks, CUDA error mapping and the scene
 // object.  Every stage entry point validates its arguments on the host and
 // forwards to one launcher; nothing here falls back to host computation.
+#include <atomic>
 #include <chrono>
 #include <cstdio>
 #include <cstring>
@@ -40,7 +41,10 @@ void set_error(const char* msg) { g_last_error = msg; }
 
 using wfpt::from_cuda;
 
+static std::atomic<uint64_t> g_scene_id{0};
+
 struct wfpt_scene {
+    const uint64_t id = ++g_scene_id;  // unlike an address, never used again
     wfpt::HostBvh2 bvh2;  // plain-form BVH kept on the host for export
     wfpt::HostBvh8 bvh8;
     wfpt::SceneDevice dev;
@@ -53,6 +57,7 @@ struct wfpt_scene {
 
 namespace wfpt {
 const SceneDevice* scene_device(const wfpt_scene* s) { return &s->dev; }
+uint64_t scene_id(const wfpt_scene* s) { return s->id; }
 bool scene_has(const wfpt_scene* s, int kind) {
     return !s->host_only && (kind == WFPT_BVH8_Q8 ? s->has8 : s->has2);
 }

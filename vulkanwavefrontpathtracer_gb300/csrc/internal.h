@@ -17,6 +17,9 @@ wfpt_status from_cuda(cudaError_t e);
 void set_error(const char* msg);
 
 const SceneDevice* scene_device(const wfpt_scene* s);
+// A number of this scene's own in the process (a later scene may get the
+// address of a destroyed one).
+uint64_t scene_id(const wfpt_scene* s);
 bool scene_has(const wfpt_scene* s, int kind);
 void scene_bounds(const wfpt_scene* s, float mn[3], float mx[3]);
 

@@ -195,7 +195,10 @@ struct wfpt_renderer {
     struct GraphKey {
         wfpt_renderer_config cfg;
         int w, h;
-        const void *pixels, *frame_pixels, *scene, *geoms;
+        const void *pixels, *frame_pixels, *geoms;
+        // The captured launches hold the scene's buffers: the scene itself, not
+        // its address, which a rebuilt scene often gets again.
+        uint64_t scene;
         float light[3], bg[3], smin[3], smax[3];
         int slots;
     } graph_key{};
@@ -209,7 +212,7 @@ struct wfpt_renderer {
         k.h = height;
         k.pixels = pixels;
         k.frame_pixels = frame_pixels;
-        k.scene = scene;
+        k.scene = wfpt::scene_id(scene);
         k.geoms = geoms;
         k.slots = nslots;
         for (int i = 0; i < 3; ++i) {
