@@ -61,3 +61,26 @@ def test_scene_rebuilt_between_frames(wf, dev):
         sc.close()
     assert not np.array_equal(frames[0], frames[5])
     assert api.device_status() == 0
+
+
+@pytest.mark.parametrize("bigger", [dict(num_shadow_samples=5), dict(timing=1), dict(sort_shadow_rays=1)])
+def test_buffers_grown_between_frames(wf, dev, bigger):
+    """A frame without the graph that needs larger buffers, then the captured frame again."""
+    import torch
+    api = wf.api
+    pos, nrm, idx = api.generate_scene(0, 42, 3000)
+    scene = api.Scene(pos, idx), api.Geometry(pos, nrm, idx, device=dev)
+    r = api.Renderer(config(wf))
+    r.set_scene(*scene, LIGHT, BG)
+    px = torch.zeros((2, 64 * 48, 4), dtype=torch.float32, device=dev)
+    first = render(wf, dev, r, 64, 48, px)
+    r.set_config(config(wf, use_graph=0, **bigger))
+    render(wf, dev, r, 640, 480)
+    r.set_config(config(wf))
+    # Whatever takes the place of the released buffers must not be written.
+    hold = [torch.full((1 << k,), 7, dtype=torch.int32, device=dev) for k in range(8, 22)]
+    assert np.array_equal(render(wf, dev, r, 64, 48, px), first)
+    assert np.array_equal(first, direct(wf, dev, scene, 64, 48))
+    assert all(bool((h == 7).all()) for h in hold)
+    r.close()
+    assert api.device_status() == 0

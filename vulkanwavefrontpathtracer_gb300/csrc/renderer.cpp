@@ -49,11 +49,16 @@ static std::atomic<int> g_shadow_slots{0};
 // touching the device.  -1 = off.
 static std::atomic<int> g_fail_alloc_after{-1};
 
+// Buffers that this thread's ensure() calls have released or allocated: a
+// captured frame graph holds the addresses from before.
+static thread_local uint64_t t_buffer_changes = 0;
+
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
     cudaError_t ensure(size_t b) {
         if (b <= bytes) return cudaSuccess;
+        ++t_buffer_changes;
         if (p) cudaFree(p);
         p = nullptr;
         bytes = 0;
@@ -902,7 +907,9 @@ wfpt_status wfpt_renderer_render(wfpt_renderer* r, const wfpt_camera* camera, in
         return WFPT_ERR_INVALID_ARGUMENT;
     }
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    const uint64_t buffers = t_buffer_changes;
     cudaError_t e = r->prepare(width, height);
+    if (t_buffer_changes != buffers) r->graph_valid = false;
     if (e != cudaSuccess) return wfpt::from_cuda(e);
     float s2w[16];
     if (!wfpt::camera_screen_to_world(camera->position, camera->rotation_deg, camera->fov_deg,
