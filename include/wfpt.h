@@ -165,6 +165,9 @@ uint64_t wfpt_kernel_launch_count(void);
  *                          overlapped shadow pass: 0 (default) = planned
  *                          from free device memory, 1..8 = that many
  *                          (capped by the batches a pass can need)
+ * The "trace." and "sort." knobs are read at each launch: a renderer captures
+ * its frame graph anew when one of them has changed; a batch keeps those of
+ * its creation.
  * Unknown keys and out-of-range values return WFPT_ERR_INVALID_ARGUMENT. */
 wfpt_status wfpt_tune_set(const char* key, int64_t value);
 wfpt_status wfpt_tune_get(const char* key, int64_t* value);

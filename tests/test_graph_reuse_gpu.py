@@ -84,3 +84,42 @@ def test_buffers_grown_between_frames(wf, dev, bigger):
     assert all(bool((h == 7).all()) for h in hold)
     r.close()
     assert api.device_status() == 0
+
+
+def test_knobs_changed_between_frames(wf, dev):
+    """A knob set after the capture reaches the next frame: counting counts the rays of a frame without
+    a graph, and stops."""
+    import torch
+    api = wf.api
+    pos, nrm, idx = api.generate_scene(0, 43, 3000)
+    scene = api.Scene(pos, idx), api.Geometry(pos, nrm, idx, device=dev)
+    r = api.Renderer(config(wf))
+    r.set_scene(*scene, LIGHT, BG)
+    px = torch.zeros((2, 80 * 60, 4), dtype=torch.float32, device=dev)
+
+    def counted(frame):
+        api.trace_counters(reset=True)
+        bits = frame()
+        return bits, api.trace_counters(reset=True)["rays"]
+
+    graph, rays = counted(lambda: render(wf, dev, r, 80, 60, px))
+    assert rays == 0
+    api.tune_set("trace.count", 1)
+    try:
+        ref, ref_rays = counted(lambda: direct(wf, dev, scene, 80, 60))
+        got, rays = counted(lambda: render(wf, dev, r, 80, 60, px))
+    finally:
+        api.tune_set("trace.count", 0)
+    assert ref_rays >= 80 * 60 and rays == ref_rays
+    assert np.array_equal(got, ref) and np.array_equal(got, graph)
+    assert counted(lambda: render(wf, dev, r, 80, 60, px))[1] == 0
+    launches = []
+    for tiles in (1, 0):
+        api.tune_set("sort.tiles", tiles)
+        assert np.array_equal(render(wf, dev, r, 80, 60, px), graph)
+        k0 = wf.api.lib().wfpt_kernel_launch_count()
+        assert np.array_equal(render(wf, dev, r, 80, 60, px), graph)
+        launches.append(wf.api.lib().wfpt_kernel_launch_count() - k0)
+    assert launches[0] != launches[1]  # the tiny tiles' scratch is cleared by a kernel, not by a memset
+    r.close()
+    assert api.device_status() == 0

@@ -206,6 +206,7 @@ struct wfpt_renderer {
         uint64_t scene;
         float light[3], bg[3], smin[3], smax[3];
         int slots;
+        int64_t knobs[10];  // the tuning knobs that its launches were made with
     } graph_key{};
     bool graph_valid = false;
 
@@ -220,6 +221,11 @@ struct wfpt_renderer {
         k.scene = wfpt::scene_id(scene);
         k.geoms = geoms;
         k.slots = nslots;
+        const int64_t knobs[10] = {wfpt::get_trace_refill(), wfpt::get_trace_postpone(), wfpt::get_trace_coop(),
+                                   wfpt::get_trace_batch(true), wfpt::get_trace_batch(false),
+                                   wfpt::get_trace_steps(true), wfpt::get_trace_steps(false), wfpt::get_trace_count(),
+                                   wfpt::get_sort_tiles(), wfpt::get_sort_digit_bits()};
+        std::memcpy(k.knobs, knobs, sizeof(knobs));
         for (int i = 0; i < 3; ++i) {
             k.light[i] = light[i];
             k.bg[i] = bg[i];
