@@ -78,7 +78,8 @@ __device__ __forceinline__ float box_area(float4 lo, float4 hi) {
 
 // ---------------------------------------------------------------- stage 1
 // Box of triangle g; false when one of its indices is out of range (read as
-// vertex 0, so the build can go on to the one read-back at its end).
+// vertex 0, so that the keys and the sort can follow without a read-back;
+// clustering and emission then return at once).
 __device__ __forceinline__ bool tri_box(const float* __restrict__ pos, uint32_t nv, const uint32_t* __restrict__ idx,
                                         uint32_t g, float lo[3], float hi[3]) {
     bool ok = true;
@@ -439,6 +440,7 @@ __global__ void __launch_bounds__(kBB, 4) k_ploc(uint32_t* cl_a, uint32_t* cl_b,
     const uint32_t cap = 2 * n - 1;
     const float delta = __fmul_rn(__uint_as_float(st->pmax), 0x1p-22f);
     uint32_t m = n, next_id = n, iter = 0, target = 0;
+    if (st->bad_index) return;  // refused by the host: the triangles may all be one
     while (m > 1) {
         const uint32_t ntiles = (m + T - 1) / T;
         const uint32_t nblocks = min(gridDim.x, ntiles);
@@ -593,6 +595,7 @@ __global__ void __launch_bounds__(kBB, 4) k_emit8(uint32_t* tasks_a, uint32_t* t
     const uint32_t node_cap = n - 1;
     const float inf = __int_as_float(0x7f800000);
     uint32_t ntasks = 1, level_base = 0, tri_base0 = 0, target = 0;
+    if (st->bad_index) return;
     for (uint32_t level = 0; ntasks > 0; ++level) {
         if (level > 64 || ntasks > node_cap || level_base + ntasks > node_cap) {  // cannot happen
             if (blockIdx.x == 0 && threadIdx.x == 0) st->stuck = 1;
