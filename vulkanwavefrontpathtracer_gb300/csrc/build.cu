@@ -48,6 +48,7 @@ namespace {
 constexpr int kBB = 256;      // threads per build block
 constexpr int kPlocRMax = 64;  // largest PLOC search radius (knob build.ploc.radius)
 constexpr uint32_t kNone = 0xFFFFFFFFu;
+constexpr uint32_t kSlowPass = 32;  // see k_ploc
 
 struct BuildStats {
     uint32_t bmin[3], bmax[3];  // order-preserving bits of the vertex box
@@ -405,14 +406,62 @@ __device__ __forceinline__ void write_node2(uint32_t index, uint32_t n, const ui
     __stcg(&meta[index], make_uint4(how[0], how[1], tris, arg[8]));
 }
 
+// The position of the R on either side of position i (box `at` in shared
+// memory) whose box merged with i's has the least surface area.  Ties go to
+// equal boxes first, and among these to the position with the least i xor j:
+// so a run of coincident triangles pairs up as (2 k, 2 k + 1).  Other ties go to
+// the smaller position, or (PAIR_TIES) also to the least i xor j.
+template <bool PAIR_TIES>
+__device__ __forceinline__ uint32_t nearest(const float4* s_lo, const float4* s_hi, int at, int R, int i, uint32_t m) {
+    const float4 alo = s_lo[at], ahi = s_hi[at];
+    uint32_t best = kNone, nn = kNone, last = kNone;  // last: the last position with the best area
+    const int d0 = max(-R, -i), d1 = min(R, (int)m - 1 - i);
+    for (int d = d0; d <= d1; ++d) {
+        if (d == 0) continue;
+        const float4 blo = s_lo[at + d], bhi = s_hi[at + d];
+        const float4 ulo = make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), 0.0f);
+        const float4 uhi = make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.0f);
+        const uint32_t key = __float_as_uint(box_area(ulo, uhi)), j = (uint32_t)(i + d);
+        if (key <= best) last = j;
+        if (key < best || (PAIR_TIES && key == best && ((uint32_t)i ^ j) < ((uint32_t)i ^ nn))) {
+            best = key;
+            nn = j;
+        }
+    }
+    // Several with the least area, and that no larger than this box: equal boxes?
+    // (One position may be the last and, by xor, the best of several.)
+    if ((PAIR_TIES || last != nn) && best == __float_as_uint(box_area(alo, ahi))) {
+        uint32_t tie = kNone;
+        for (int d = d0; d <= d1; ++d) {
+            const float4 blo = s_lo[at + d], bhi = s_hi[at + d];
+            const uint32_t x = (uint32_t)i ^ (uint32_t)(i + d);
+            if (d != 0 && x < tie && alo.x == blo.x && alo.y == blo.y && alo.z == blo.z && ahi.x == bhi.x &&
+                ahi.y == bhi.y && ahi.z == bhi.z) {
+                tie = x;
+                nn = (uint32_t)(i + d);
+            }
+        }
+    }
+    return nn;
+}
+
 // The whole clustering.  A block takes tiles of kBB - 2 R cluster positions
 // and holds the boxes of the tile and of 2 R positions on either side in
 // shared memory: enough to find the nearest neighbour (least merged surface
 // area, ties to the smaller position) of every position of the tile and of
 // the R on either side, hence the mutual pairs that start or end in the
-// tile.  For a fixed cluster that order is the order of (area, smaller
-// position, larger position) over pairs, so the pair that is least in that
-// order over all pairs is mutual and every pass merges at least one pair.
+// tile.  For a fixed cluster that order is an order of pairs (area; equal boxes
+// first; i xor j or the positions), so the pair that is least in it over all
+// pairs is mutual and every pass merges at least one pair.
+// No more than one, where all ties go to the smaller position: 600 coincident
+// triangles took 599 passes and gave a chain too deep for the emission and for
+// the traversal's stacks, and 80 of them in the courtyard's mesh a tree of depth
+// 100.  Equal boxes first: 10 passes, and depth 29.  A strip of 40,000 equal
+// triangles still took over 20,000 passes; so after a pass that merged less
+// than one in kSlowPass of its clusters the other ties go by i xor j too: 22
+// passes.  Triangle soups, the courtyard and the city merge 9 % and more at
+// every radius, a regular grid 6 % at radius 8: their trees are those of the
+// smaller position.
 // A pair's node is made by the block of its lower position, the first
 // threads of the block taking one pair each.  The pass ends at a barrier of
 // the blocks that had a tile; blocks without one are done for good, since
@@ -440,6 +489,7 @@ __global__ void __launch_bounds__(kBB, 4) k_ploc(uint32_t* cl_a, uint32_t* cl_b,
     const uint32_t cap = 2 * n - 1;
     const float delta = __fmul_rn(__uint_as_float(st->pmax), 0x1p-22f);
     uint32_t m = n, next_id = n, iter = 0, target = 0;
+    bool pair_ties = false;
     if (st->bad_index) return;  // refused by the host: the triangles may all be one
     while (m > 1) {
         const uint32_t ntiles = (m + T - 1) / T;
@@ -463,22 +513,7 @@ __global__ void __launch_bounds__(kBB, 4) k_ploc(uint32_t* cl_a, uint32_t* cl_b,
             __syncthreads();
             const int i = b0 - R + tid;
             uint32_t nn = kNone;
-            if (i >= 0 && i < (int)m) {
-                const float4 alo = s_lo[tid + R], ahi = s_hi[tid + R];
-                uint32_t best = kNone;
-                const int d0 = max(-R, -i), d1 = min(R, (int)m - 1 - i);
-                for (int d = d0; d <= d1; ++d) {
-                    if (d == 0) continue;
-                    const float4 blo = s_lo[tid + R + d], bhi = s_hi[tid + R + d];
-                    const float4 ulo = make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), 0.0f);
-                    const float4 uhi = make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.0f);
-                    const uint32_t key = __float_as_uint(box_area(ulo, uhi));
-                    if (key < best) {
-                        best = key;
-                        nn = (uint32_t)(i + d);
-                    }
-                }
-            }
+            if (i >= 0 && i < (int)m) nn = pair_ties ? nearest<true>(s_lo, s_hi, tid + R, R, i, m) : nearest<false>(s_lo, s_hi, tid + R, R, i, m);
             s_nn[tid] = nn;
             __syncthreads();
             bool keep = false, merge = false;
@@ -531,6 +566,7 @@ __global__ void __launch_bounds__(kBB, 4) k_ploc(uint32_t* cl_a, uint32_t* cl_b,
             if (left >= m) st->stuck = 1;
         }
         if (left >= m) return;
+        pair_ties = pair_ties || m - left < m / kSlowPass;
         m = left;
         // A lone block rewrites st->clusters in its next pass: not before
         // every thread has read it.
