@@ -82,7 +82,8 @@ def graded(n):
 
 
 # mesh, radius, passes at most, depth at most; the graded strip's passes go past the 128 that the
-# clustering's look-back states tell apart, with several tiles of clusters at the time
+# clustering's look-back states tell apart, with several tiles of clusters at the time, and past the
+# 256 of one launch
 MESHES = [("coincident", 40, 8, 6, 6), ("coincident", 241, 8, 8, 8), ("coincident", 400, 8, 9, 9),
           ("coincident", 600, 64, 10, 10), ("coincident", 100000, 8, 17, 17), ("coincident", 100000, 1, 17, 17),
           ("padded", 80, 8, 40, 30), ("padded", 5000, 8, 40, 30), ("equal", 63, 8, 40, 20),
@@ -108,15 +109,19 @@ def test_ties_do_not_make_chains(wf, dev, name, n, radius, passes, depth):
     old = wf.api.tune_get("build.ploc.radius")
     try:
         wf.api.tune_set("build.ploc.radius", radius)
+        launches = wf.api.lib().wfpt_kernel_launch_count()
         sc = build(wf, dev, pos, idx)
     finally:
         wf.api.tune_set("build.ploc.radius", old)
+    launches = wf.api.lib().wfpt_kernel_launch_count() - launches
     nodes, tris = sc.export_bvh2()
     v = tris.view(np.float32).reshape(-1, 12)[:, [0, 1, 2, 4, 5, 6, 8, 9, 10]].reshape(-1, 3, 3)
     kids, sizes, deep = ploc(v.min(1), v.max(1), radius)
     assert len(sizes) <= passes and deep <= depth
+    # Three kernels, the sort's ten (clear, histograms, eight passes), clustering and emission.
+    assert launches == 13 + 2 * -(-len(sizes) // 256)
     if (name, radius) == ("graded", 64):
-        assert len(sizes) > 128 and sizes[128] > 256 - 2 * radius
+        assert len(sizes) > 256 and sizes[128] > 256 - 2 * radius
     links = nodes.view(np.int32).reshape(-1, 16)[::-1, 12:14].astype(np.int64)
     assert np.array_equal(np.where(links < 0, (~links & 0xFFFFFFFF) >> 3, 2 * n - 2 - links), np.array(kids))
     ids = sc.export_bvh8()[1].view(np.uint32).reshape(-1, 12)[:, 11]

@@ -18,7 +18,8 @@
 //   4. the BVH8 by the host's SAH collapse, emitted top-down one level at a
 //      time in a second cooperative launch, eight lanes per node, with
 //      look-back allocation, so the layout is deterministic.
-// The host reads the device back once, at the end.  Every device wait is
+// The host reads the device back once, at the end (a mesh of more than
+// kPassesPerLaunch clustering passes: once per launch).  Every device wait is
 // bounded (kSpinLimit polls, then the timeout status); kernels check their
 // indices against the buffers they write.
 #include <algorithm>
@@ -49,15 +50,21 @@ constexpr int kBB = 256;      // threads per build block
 constexpr int kPlocRMax = 64;  // largest PLOC search radius (knob build.ploc.radius)
 constexpr uint32_t kNone = 0xFFFFFFFFu;
 constexpr uint32_t kSlowPass = 32;  // see k_ploc
+// Passes of one launch of k_ploc.  Meshes take some 20 to 100 in all; one that
+// merges a pair or two per pass (a strip whose triangles get steadily smaller:
+// passes grow with its length) goes on in further launches, so that no single
+// one runs for long.
+constexpr uint32_t kPassesPerLaunch = 256;
 
 struct BuildStats {
     uint32_t bmin[3], bmax[3];  // order-preserving bits of the vertex box
     uint32_t cmin[3], cmax[3];  // ... of the centroid box
     uint32_t pmax;              // bits of the largest |coordinate|
     uint32_t bad_index;
-    // Clustering: clusters and nodes after the last finished pass, passes,
-    // no pair merged (cannot happen), blocks that reached the pass barriers.
-    uint32_t clusters, next_id, iterations, stuck, ploc_barrier;
+    // Clustering: clusters and nodes after the last finished pass, passes, ties
+    // by pairs from now on, no pair merged (cannot happen), blocks that
+    // reached the pass barriers of the launch.
+    uint32_t clusters, next_id, iterations, pair_ties, stuck, ploc_barrier;
     // Emission: BVH8 nodes and triangles emitted; by level parity, the tasks
     // of the next level and the triangles so far; blocks that reached the
     // level barriers.
@@ -445,6 +452,11 @@ __device__ __forceinline__ uint32_t nearest(const float4* s_lo, const float4* s_
     return nn;
 }
 
+// Where a launch of k_ploc goes on (as in BuildStats).
+struct PlocStart {
+    uint32_t clusters, next_id, iterations, pair_ties;
+};
+
 // The whole clustering.  A block takes tiles of kBB - 2 R cluster positions
 // and holds the boxes of the tile and of 2 R positions on either side in
 // shared memory: enough to find the nearest neighbour (least merged surface
@@ -478,7 +490,7 @@ __device__ __forceinline__ uint32_t nearest(const float4* s_lo, const float4* s_
 __global__ void __launch_bounds__(kBB, 4) k_ploc(uint32_t* cl_a, uint32_t* cl_b, uint32_t n, int radius,
                                                  float4* boxes, float4* __restrict__ nodes2, float4* cost,
                                                  uint4* meta, int want8, float tri_cost, unsigned long long* state,
-                                                 BuildStats* st) {
+                                                 BuildStats* st, PlocStart from) {
     constexpr int kMost = kBB + 2 * kPlocRMax;
     __shared__ float4 s_lo[kMost], s_hi[kMost];
     __shared__ uint32_t s_id[kMost], s_nn[kBB], s_pair[kBB], s_warp[kBB / 32];
@@ -488,8 +500,8 @@ __global__ void __launch_bounds__(kBB, 4) k_ploc(uint32_t* cl_a, uint32_t* cl_b,
     const int tid = (int)threadIdx.x;
     const uint32_t cap = 2 * n - 1;
     const float delta = __fmul_rn(__uint_as_float(st->pmax), 0x1p-22f);
-    uint32_t m = n, next_id = n, iter = 0, target = 0;
-    bool pair_ties = false;
+    uint32_t m = from.clusters, next_id = from.next_id, iter = from.iterations, target = 0;
+    bool pair_ties = from.pair_ties != 0;
     if (st->bad_index) return;  // refused by the host: the triangles may all be one
     while (m > 1) {
         const uint32_t ntiles = (m + T - 1) / T;
@@ -561,12 +573,13 @@ __global__ void __launch_bounds__(kBB, 4) k_ploc(uint32_t* cl_a, uint32_t* cl_b,
         const uint32_t left = __ldcg(&st->clusters);
         next_id = __ldcg(&st->next_id);
         ++iter;
+        pair_ties = pair_ties || m - left < m / kSlowPass;
         if (blockIdx.x == 0 && tid == 0) {
             st->iterations = iter;
+            st->pair_ties = pair_ties;
             if (left >= m) st->stuck = 1;
         }
-        if (left >= m) return;
-        pair_ties = pair_ties || m - left < m / kSlowPass;
+        if (left >= m || iter - from.iterations == kPassesPerLaunch) return;
         m = left;
         // A lone block rewrites st->clusters in its next pass: not before
         // every thread has read it.
@@ -631,7 +644,7 @@ __global__ void __launch_bounds__(kBB, 4) k_emit8(uint32_t* tasks_a, uint32_t* t
     const uint32_t node_cap = n - 1;
     const float inf = __int_as_float(0x7f800000);
     uint32_t ntasks = 1, level_base = 0, tri_base0 = 0, target = 0;
-    if (st->bad_index) return;
+    if (st->bad_index || st->clusters != 1) return;
     for (uint32_t level = 0; ntasks > 0; ++level) {
         if (level > 64 || ntasks > node_cap || level_base + ntasks > node_cap) {  // cannot happen
             if (blockIdx.x == 0 && threadIdx.x == 0) st->stuck = 1;
@@ -971,16 +984,26 @@ cudaError_t build_scene_device(const float* positions_dev, uint32_t num_vertices
         // stage 3: clusters, BVH2, collapse tables
         const float tri_cost = (float)get_bvh8_tri_cost_pct() * 0.01f;
         const uint64_t tile = (uint64_t)(kBB - 2 * radius);
-        WFPT_TRY(launch_resident(k_ploc, ((uint64_t)n + tile - 1) / tile, s, ids_a, ids_b, n, radius, boxes,
-                                 reinterpret_cast<float4*>(nodes2), cost, meta, want8 ? 1 : 0, tri_cost, ploc_state,
-                                 st));
-        // stage 4: BVH8
-        if (want8)
-            WFPT_TRY(launch_resident(k_emit8, (uint64_t)emit_tiles, s, ids_a, ids_b, n, (const Bvh2Node*)nodes2,
-                                     (const uint4*)meta, (const float4*)recs2, reinterpret_cast<float4*>(tmp), recs8,
-                                     emit_state, st));
-        WFPT_TRY(cudaMemcpyAsync(&got, st, sizeof(got), cudaMemcpyDeviceToHost, s));
-        WFPT_TRY(cudaStreamSynchronize(s));
+        PlocStart from{n, n, 0, 0};
+        for (;;) {
+            WFPT_TRY(launch_resident(k_ploc, ((uint64_t)from.clusters + tile - 1) / tile, s, ids_a, ids_b, n, radius,
+                                     boxes, reinterpret_cast<float4*>(nodes2), cost, meta, want8 ? 1 : 0, tri_cost,
+                                     ploc_state, st, from));
+            // stage 4: BVH8
+            if (want8)
+                WFPT_TRY(launch_resident(k_emit8, (uint64_t)emit_tiles, s, ids_a, ids_b, n, (const Bvh2Node*)nodes2,
+                                         (const uint4*)meta, (const float4*)recs2, reinterpret_cast<float4*>(tmp),
+                                         recs8, emit_state, st));
+            WFPT_TRY(cudaMemcpyAsync(&got, st, sizeof(got), cudaMemcpyDeviceToHost, s));
+            WFPT_TRY(cudaStreamSynchronize(s));
+            // More passes to go (rare): anything else that left several
+            // clusters is an error, seen below.
+            if (got.bad_index || got.stuck || got.clusters <= 1 || got.clusters >= from.clusters ||
+                got.iterations != from.iterations + kPassesPerLaunch)
+                break;
+            from = PlocStart{got.clusters, got.next_id, got.iterations, got.pair_ties};
+            WFPT_TRY(cudaMemsetAsync(&st->ploc_barrier, 0, sizeof(st->ploc_barrier), s));
+        }
     }
     if (got.bad_index) {
         e = cudaErrorInvalidValue;
