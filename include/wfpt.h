@@ -438,7 +438,9 @@ wfpt_status wfpt_scene_create(const float* positions, uint32_t num_vertices,
  * host build (knobs "build.bvh8.*").  Hits equal those of a host-built scene
  * of the same mesh (the traversal result does not depend on the tree).
  * Runs on `stream` and returns when the scene is ready; out-of-range
- * triangle indices return WFPT_ERR_INVALID_ARGUMENT.  Exports of such a
+ * triangle indices return WFPT_ERR_INVALID_ARGUMENT, a mesh whose clustering
+ * gives a BVH8 of more than 65 levels (hundreds of triangles nested in one
+ * another) WFPT_ERR_UNSUPPORTED.  Exports of such a
  * scene copy its device buffers. */
 wfpt_status wfpt_scene_create_device(const float* positions_dev, uint32_t num_vertices,
                                      const uint32_t* indices_dev, uint32_t num_triangles,

@@ -140,3 +140,15 @@ def test_ties_do_not_make_chains(wf, dev, name, n, radius, passes, depth):
         wf.api.trace(sc, kind, rays, hits)
         assert torch.equal(hits, ref)
     assert wf.api.device_status() == 0
+
+
+def test_nested_triangles_are_refused_by_name(wf, dev):
+    """A thousand triangles nested in one another cluster into a chain, deeper than the BVH8's limit."""
+    scale = 100 * 1.05 ** -np.arange(1000.0)
+    pos = np.array([[-1, -1, 0], [1, -1, 0.1], [0, 1, 0.2]]) * scale[:, None, None]
+    pos, idx = pos.reshape(-1, 3).astype(np.float32), np.arange(3000).reshape(-1, 3)
+    with pytest.raises(wf.WfptError) as err:
+        build(wf, dev, pos, idx)
+    assert "nested too deep" in str(err.value) and "UNSUPPORTED" in str(err.value)
+    assert wf.api.Scene(pos, idx.astype(np.uint32)).info.num_triangles == 1000
+    assert wf.api.device_status() == 0

@@ -520,6 +520,10 @@ static wfpt_status create_device_built(const float* positions_dev, uint32_t num_
                                  (bvh_kinds_mask & (1 << WFPT_BVH8_Q8)) != 0, s, &b);
     cudaFree(gdev);
     if (e == cudaErrorInvalidValue) return invalid("triangle index out of range");
+    if (b.too_deep) {
+        g_last_error = "device BVH build: triangles nested too deep (more than 65 levels of the BVH8); build on the host";
+        return WFPT_ERR_UNSUPPORTED;
+    }
     if (e != cudaSuccess) {
         wfpt_status st = from_cuda(e);
         g_last_error = std::string("device BVH build failed: ") + g_last_error;

@@ -67,8 +67,8 @@ struct BuildStats {
     uint32_t clusters, next_id, iterations, pair_ties, stuck, ploc_barrier;
     // Emission: BVH8 nodes and triangles emitted; by level parity, the tasks
     // of the next level and the triangles so far; blocks that reached the
-    // level barriers.
-    uint32_t nodes8, tris8, tasks[2], tris[2], emit_barrier;
+    // level barriers; the tree is too deep.
+    uint32_t nodes8, tris8, tasks[2], tris[2], emit_barrier, too_deep;
 };
 
 __device__ __forceinline__ uint32_t ord(float f) {
@@ -631,6 +631,9 @@ __device__ __forceinline__ uint32_t how_of(const uint4& m, int s) {  // byte how
 // to count) and a prefix sum and a read-back per level, took 1.24 ms for 3M
 // triangles; this takes 0.52 ms.
 constexpr int kEmitTile = kBB / 8;
+// Levels below the root.  Meshes of millions of triangles have about ten;
+// a few hundred triangles nested in one another are a chain, and refused.
+constexpr uint32_t kMostLevels = 64;
 __global__ void __launch_bounds__(kBB, 4) k_emit8(uint32_t* tasks_a, uint32_t* tasks_b, uint32_t n,
                                                   const Bvh2Node* __restrict__ nodes, const uint4* __restrict__ meta,
                                                   const float4* __restrict__ recs2, float4* __restrict__ out,
@@ -646,7 +649,11 @@ __global__ void __launch_bounds__(kBB, 4) k_emit8(uint32_t* tasks_a, uint32_t* t
     uint32_t ntasks = 1, level_base = 0, tri_base0 = 0, target = 0;
     if (st->bad_index || st->clusters != 1) return;
     for (uint32_t level = 0; ntasks > 0; ++level) {
-        if (level > 64 || ntasks > node_cap || level_base + ntasks > node_cap) {  // cannot happen
+        if (level > kMostLevels) {
+            if (blockIdx.x == 0 && threadIdx.x == 0) st->too_deep = 1;
+            return;
+        }
+        if (ntasks > node_cap || level_base + ntasks > node_cap) {  // cannot happen
             if (blockIdx.x == 0 && threadIdx.x == 0) st->stuck = 1;
             return;
         }
@@ -1009,8 +1016,9 @@ cudaError_t build_scene_device(const float* positions_dev, uint32_t num_vertices
         e = cudaErrorInvalidValue;
         goto done;
     }
+    out->too_deep = got.too_deep != 0;
     WFPT_TRY(status_build(&status));
-    if (status || got.stuck || got.clusters != 1 || got.next_id != nall || (want8 && got.tris8 != n) ||
+    if (status || got.stuck || got.too_deep || got.clusters != 1 || got.next_id != nall || (want8 && got.tris8 != n) ||
         (want8 && (got.nodes8 == 0 || got.nodes8 > ninner))) {
         e = cudaErrorUnknown;
         goto done;

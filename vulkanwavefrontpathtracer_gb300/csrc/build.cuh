@@ -16,6 +16,7 @@ struct DeviceBuild {
     uint32_t bvh2_count = 0, bvh8_count = 0;
     float bounds_min[3] = {0, 0, 0}, bounds_max[3] = {0, 0, 0};
     uint32_t ploc_iterations = 0;
+    bool too_deep = false;  // the error is a BVH8 of too many levels
 };
 
 // Builds the BVH2 (PLOC over 63-bit Morton-sorted triangle centroids,
