@@ -252,7 +252,8 @@ wfpt_status wfpt_sort_pairs(void* keys, uint32_t* values, uint32_t n,
 /* reorderRays.comp:27-46 + Tracer::reorderRays (Tracer.cpp:80-98):
  * out_rays[i] = in_rays[idx[i]]; out_slot_to_index[i] =
  * in_slot_to_index[idx[i]]; out_index_to_slot[out_slot_to_index[i]] = i.
- * ray_index must be a permutation of [0, n); out_index_to_slot must have
+ * ray_index must be a permutation of [0, n) and may be out_slot_to_index
+ * (the map then takes its place); out_index_to_slot must have
  * room for every value in in_slot_to_index (pixel indices in a renderer,
  * which can exceed n in a compacted wavefront). */
 wfpt_status wfpt_reorder(const uint32_t* ray_index, const wfpt_ray* in_rays,

@@ -248,15 +248,18 @@ static cudaError_t launch_maps(const uint32_t* idx, const int32_t* in_s2i, int32
     const bool vec = ((reinterpret_cast<uintptr_t>(idx) | reinterpret_cast<uintptr_t>(out_s2i)) & 15u) == 0;
     auto gather = vec ? k_map_gather<true> : k_map_gather<false>;
     auto scatter = vec ? k_map_scatter<true> : k_map_scatter<false>;
-    for (uint32_t r = 0; r < ranges; ++r) {
+    // In place over the index array (a thread reads its entries before it writes
+    // them) it is one range: a second one would read the first one's output.
+    const uint32_t gathers = reinterpret_cast<const void*>(idx) == out_s2i ? 1u : ranges;
+    for (uint32_t r = 0; r < gathers; ++r) {
         const uint32_t lo = r * step;
-        gather<<<grid, kBlock, 0, s>>>(idx, in_s2i, out_s2i, n, n_dev, lo, r + 1 == ranges ? 0xFFFFFFFFu - lo : step);
+        gather<<<grid, kBlock, 0, s>>>(idx, in_s2i, out_s2i, n, n_dev, lo, r + 1 == gathers ? 0xFFFFFFFFu - lo : step);
     }
     for (uint32_t r = 0; r < ranges && out_i2s != nullptr; ++r) {
         const uint32_t lo = r * step;
         scatter<<<grid, kBlock, 0, s>>>(out_s2i, out_i2s, n, n_dev, lo, r + 1 == ranges ? 0xFFFFFFFFu - lo : step);
     }
-    count_launch(out_i2s != nullptr ? 2 * ranges : ranges);
+    count_launch(out_i2s != nullptr ? gathers + ranges : gathers);
     return cudaGetLastError();
 }
 
