@@ -1075,7 +1075,7 @@ __global__ void __launch_bounds__(kBlock, PER_SM) k_trace_bvh8_coop(
 // Small wavefronts (PER_SM 3) go on past four leaves: 256x256 frame 914 -> 893
 // us; large ones that way 0.6 % slower.
 constexpr uint32_t kFewOccluded = 16;  // 20: 0-1 % slower, 24: 1-3 %, 12: 0-1 %
-template <bool RECORD, int PER_SM>
+template <bool RECORD, int PER_SM, bool COUNT = false>
 __global__ void __launch_bounds__(kBlock, PER_SM) k_any_bvh8(
     const float4* __restrict__ nodes, const float4* __restrict__ tris, const float4* __restrict__ rays,
     void* __restrict__ results, const uint32_t* __restrict__ ray_index, uint32_t n,
@@ -1102,6 +1102,7 @@ __global__ void __launch_bounds__(kBlock, PER_SM) k_any_bvh8(
     RayT r;
     float tmax = 0.0f;
     uint2 ng = make_uint2(0u, 0u);
+    uint32_t c_nodes = 0, c_tris = 0, c_rays = 0, c_iters = 0;
     for (;;) {
         const bool want = state != kTracing && !exhausted;
         const uint32_t want_mask = __ballot_sync(0xffffffffu, want);
@@ -1153,6 +1154,7 @@ __global__ void __launch_bounds__(kBlock, PER_SM) k_any_bvh8(
             }
         }
         if (__ballot_sync(0xffffffffu, state != kIdle || !exhausted) == 0u) break;
+        if (COUNT && lane == 0) ++c_iters;
 
         uint32_t leaf = 0, leaf2 = 0, from = 0, from2 = 0;
         const uint32_t few = __any_sync(0xffffffffu, exhausted) ? 1u : RECORD ? kFewLanes : kFewOccluded;
@@ -1172,6 +1174,7 @@ __global__ void __launch_bounds__(kBlock, PER_SM) k_any_bvh8(
                     }
                 }
                 uint32_t child_base, imask, lf;
+                if (COUNT) ++c_nodes;
                 const uint32_t inner = intersect_node8<PER_SM == 3>(nodes + 5 * (size_t)node, r, tmax, child_base, imask, lf);
                 ng = make_uint2(child_base, inner | imask);
                 if (leaf == 0u) {
@@ -1191,6 +1194,7 @@ __global__ void __launch_bounds__(kBlock, PER_SM) k_any_bvh8(
         if (leaf2 != 0u) meta2 = __ldg(reinterpret_cast<const uint4*>(nodes + 5 * (size_t)from2 + 1));
         const uint32_t cnt1 = leaf_count(leaf, meta.z, meta.w);
         const uint32_t cnt = cnt1 + leaf_count(leaf2, meta2.z, meta2.w);
+        if (COUNT) c_tris += cnt;
         uint32_t incl = cnt;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
@@ -1261,8 +1265,10 @@ __global__ void __launch_bounds__(kBlock, PER_SM) k_any_bvh8(
                 state = kBlocked;
             else if (ng.y <= 0x00FFFFFFu)
                 state = kFree;
+            if (COUNT && state != kTracing) ++c_rays;
         }
     }
+    if (COUNT) add_counts(c_nodes, c_tris, c_rays, c_iters);
     if (lane == 0) {
         const uint32_t warps = gridDim.x * (blockDim.x / 32);
         __threadfence();
@@ -1381,6 +1387,8 @@ cudaError_t launch_trace(const SceneDevice& sc, int kind, const wfpt_ray* rays, 
         const uint32_t lanes = pgrid * kBlock;
         if (grid < pgrid) pgrid = grid;
         uint32_t* work = own_work ? own_work : sc.work + 16 * (g_slot.fetch_add(1) % kWorkSlots);
+        // Counted any-hit records come from the kernel with a ring at batch 1: the
+        // same node steps and tests as without.
         if (coop && !closest && !g_count && kernel_batch(false) <= 1u) {
             const unsigned resident = std::max(1u, (unsigned)(g_num_sms * g_blocks_per_sm[small ? 9 : 8]));
             auto k8 = small ? k_any_bvh8<true, 3> : k_any_bvh8<true, 4>;
@@ -1424,7 +1432,7 @@ cudaError_t launch_trace(const SceneDevice& sc, int kind, const wfpt_ray* rays, 
 }
 
 bool occluded_ready(const SceneDevice& sc, int kind) {
-    return !g_count && (kind != WFPT_BVH8_Q8 || (g_coop && sc.bvh8_num_tris < (1u << kRecBits)));
+    return kind != WFPT_BVH8_Q8 || (g_coop && sc.bvh8_num_tris < (1u << kRecBits));
 }
 
 cudaError_t launch_occluded(const SceneDevice& sc, int kind, const wfpt_ray* rays, int32_t* occluded,
@@ -1442,21 +1450,24 @@ cudaError_t launch_occluded(const SceneDevice& sc, int kind, const wfpt_ray* ray
         }
         const bool small = n < kCoopLargeMin && !shared;
         const unsigned resident = std::max(1u, (unsigned)(g_num_sms * g_blocks_per_sm[small ? 7 : 6]));
-        auto k8 = small ? k_any_bvh8<false, 3> : k_any_bvh8<false, 4>;
+        auto k8 = small ? (g_count ? k_any_bvh8<false, 3, true> : k_any_bvh8<false, 3>)
+                        : (g_count ? k_any_bvh8<false, 4, true> : k_any_bvh8<false, 4>);
         k8<<<std::min(grid, resident), kBlock, 0, s>>>(sc.bvh8_nodes, sc.bvh8_tris, rr, occluded, ray_index, n, n_dev,
                                                        work, g_refill, kernel_steps(false, n, resident * kBlock));
     } else {
         int4* out = reinterpret_cast<int4*>(occluded);
         constexpr int B = kBvh2SmallBlock, P = kBvh2SmallPerSm;
-        if (n >= kBvh2RefillMin)
-            k_trace_bvh2_persistent<false, false, true><<<std::min(grid, kBvh2Grid), kBlock, 0, s>>>(
-                sc.bvh2_nodes, sc.bvh2_tris, rr, out, ray_index, n, n_dev, work);
-        else if (n >= kBvh2SmallMin)
-            k_trace_bvh2<false, false, B, P, true><<<(n + B - 1) / B, B, 0, s>>>(sc.bvh2_nodes, sc.bvh2_tris, rr, out,
-                                                                                ray_index, n, n_dev);
-        else
-            k_trace_bvh2<false, false, kBlock, 1, true><<<grid, kBlock, 0, s>>>(sc.bvh2_nodes, sc.bvh2_tris, rr, out,
-                                                                               ray_index, n, n_dev);
+        if (n >= kBvh2RefillMin) {
+            auto k2 = g_count ? k_trace_bvh2_persistent<false, true, true> : k_trace_bvh2_persistent<false, false, true>;
+            k2<<<std::min(grid, kBvh2Grid), kBlock, 0, s>>>(sc.bvh2_nodes, sc.bvh2_tris, rr, out, ray_index, n, n_dev,
+                                                            work);
+        } else if (n >= kBvh2SmallMin) {
+            auto k2 = g_count ? k_trace_bvh2<false, true, B, P, true> : k_trace_bvh2<false, false, B, P, true>;
+            k2<<<(n + B - 1) / B, B, 0, s>>>(sc.bvh2_nodes, sc.bvh2_tris, rr, out, ray_index, n, n_dev);
+        } else {
+            auto k2 = g_count ? k_trace_bvh2<false, true, kBlock, 1, true> : k_trace_bvh2<false, false, kBlock, 1, true>;
+            k2<<<grid, kBlock, 0, s>>>(sc.bvh2_nodes, sc.bvh2_tris, rr, out, ray_index, n, n_dev);
+        }
     }
     count_launch();
     return cudaGetLastError();

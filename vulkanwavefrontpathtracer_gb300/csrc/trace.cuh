@@ -44,8 +44,8 @@ cudaError_t launch_trace(const SceneDevice& sc, int kind, const wfpt_ray* rays, 
                          cudaStream_t s, uint32_t* work = nullptr, bool shared = false);
 
 // Any-hit traversal that writes one word per ray: 0 if there is a hit, -1 if
-// not.  occluded_ready: false where it has no such form (per-lane BVH8 traversal,
-// counting), and launch_trace has to be used.  work as above, not null.
+// not.  occluded_ready: false where it has no such form (per-lane BVH8
+// traversal), and launch_trace has to be used.  work as above, not null.
 bool occluded_ready(const SceneDevice& sc, int kind);
 cudaError_t launch_occluded(const SceneDevice& sc, int kind, const wfpt_ray* rays, int32_t* occluded,
                             const uint32_t* ray_index, uint32_t n, const uint32_t* n_dev, cudaStream_t s,
