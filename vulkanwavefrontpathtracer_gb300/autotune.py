@@ -35,13 +35,16 @@ def _timeit(fn: Callable[[], None], reps: int = 5, warm: int = 2) -> float:
     return a.elapsed_time(b) / reps
 
 
-def tune_traversal(scene: api.Scene, closest_rays, any_rays, refills: Iterable[int] = (1, 2, 4, 8, 16, 32),
+def tune_traversal(scene: api.Scene, closest_rays, any_rays, refills: Iterable[int] = (1, 2, 4, 6, 8, 16, 32),
                    postpones: Iterable[int] = (0, 4, 8, 12), coops: Iterable[int] = (0, 1),
                    batches: Iterable[int] = (1, 8, 16, 24, 32), steps: Iterable[int] = (1, 2, 3),
                    reps: int = 5) -> Dict:
     """Grid search of refill x (cooperative tests: batch x node steps per
     iteration; per-lane tests: postpone) for BVH8 closest-hit and any-hit
-    traversal; returns the best settings and the full table (ms)."""
+    traversal; returns the best settings and the full table (ms).  Any-hit
+    rays are timed through `api.trace`, which writes records; a frame's shadow
+    rays go through the same loop without records, which takes the refill and
+    the steps found here and has no batch."""
     import torch
     dev = closest_rays.device
     res_c = torch.empty((closest_rays.shape[0], 4), dtype=torch.int32, device=dev)
@@ -95,7 +98,10 @@ KEY_CHOICES = ((L.MORTON_AILA32, 32), (L.MORTON_6D48, 48), (L.MORTON_6D64, 63))
 
 def tune_keys(scene: api.Scene, path_rays, bvh_kind: int = L.BVH8_Q8, reps: int = 5) -> Dict:
     """Times trace alone, and Morton + sort + (reorder | indirect) + trace for
-    each key layout; returns the fastest choice and the table (ms)."""
+    each key layout; returns the fastest choice and the table (ms).  The BVH2's
+    trace calls give every ray a thread; in a frame's bounces its lanes take new
+    rays as they finish, which helps unsorted rays more than these times show
+    (`tune_bvh_kinds` and `tune_bounce_sort` time whole frames)."""
     import torch
     dev = path_rays.device
     m = path_rays.shape[0]
@@ -126,12 +132,14 @@ def tune_keys(scene: api.Scene, path_rays, bvh_kind: int = L.BVH8_Q8, reps: int 
     return {"best": best, "table": table}
 
 
-def tune_sort(keys, key_bits: int, reps: int = 10) -> Dict:
-    """Radix digit width (4 or 8 bits) x tile variant (small, large,
-    extra-large; 64-bit keys have no extra-large tile, so 3 repeats 2) for
-    sorts of `keys` (a device tensor of int32 / int64 keys); returns the
-    fastest setting and the table (ms per sort, keys restored before
-    every sort)."""
+def tune_sort(keys, key_bits: int, reps: int = 10, margin: float = 0.02) -> Dict:
+    """Radix digit width (4 or 8 bits) x tile variant (0 by problem size,
+    small, large, extra-large; 64-bit keys have no extra-large tile) for sorts
+    of `keys` (a device tensor of int32 / int64 keys); returns the setting and
+    the table (ms per sort, keys restored before every sort).  The knobs hold
+    for sorts of every size, so the default (8 bits, by problem size, with its
+    tiny tiles for small sorts) stays unless another setting is faster by more
+    than `margin` of its time."""
     import torch
     n = keys.shape[0]
     work = keys.clone()
@@ -141,7 +149,7 @@ def tune_sort(keys, key_bits: int, reps: int = 10) -> Dict:
     old = (api.tune_get("sort.digit_bits"), api.tune_get("sort.tiles"))
     table = []
     try:
-        for db, tiles in itertools.product((8, 4), (1, 2) if key_bits > 32 else (1, 2, 3)):
+        for db, tiles in itertools.product((8, 4), (0, 1, 2) if key_bits > 32 else (0, 1, 2, 3)):
             api.tune_set("sort.digit_bits", db)
             api.tune_set("sort.tiles", tiles)
 
@@ -155,6 +163,8 @@ def tune_sort(keys, key_bits: int, reps: int = 10) -> Dict:
         api.tune_set("sort.digit_bits", old[0])
         api.tune_set("sort.tiles", old[1])
     best = min(table, key=lambda e: e["ms"])
+    if best["ms"] >= (1.0 - margin) * table[0]["ms"]:
+        best = table[0]
     return {"digit_bits": best["digit_bits"], "tiles": best["tiles"], "table": table}
 
 
