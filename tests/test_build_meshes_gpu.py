@@ -33,8 +33,8 @@ def area(lo, hi):
 
 def ploc(lo, hi, radius):
     """The clustering on the host: (children of the inner nodes in creation order, clusters before
-    each pass, depth).  Ties of the merged area go to equal boxes, the least i xor j first, then to the
-    smaller position (after a pass that merged less than 1 in 32 of its clusters the least i xor j)."""
+    each pass, depth).  Ties of the merged area go to the run of equal boxes, the least i xor j first, then
+    to the smaller position (after a pass that merged less than 1 in 32 of its clusters the least i xor j)."""
     n = lo.shape[0]
     ids = np.arange(n)
     depth = np.zeros(n, int)
@@ -42,11 +42,12 @@ def ploc(lo, hi, radius):
     while ids.size > 1:
         m = ids.size
         sizes.append(m)
+        run = np.concatenate([[0], np.cumsum(np.any((lo[1:] != lo[:-1]) | (hi[1:] != hi[:-1]), 1))])
         best, tie, nn = np.full(m, np.inf, np.float32), np.full(m, 2**40), np.full(m, -1)
         for d in [x for x in range(-radius, radius + 1) if x and abs(x) < m]:
             i = np.arange(max(0, -d), min(m, m - d))
             a = area(np.minimum(lo[i], lo[i + d]), np.maximum(hi[i], hi[i + d]))
-            same = np.all((lo[i] == lo[i + d]) & (hi[i] == hi[i + d]), 1)
+            same = run[i] == run[i + d]
             x = np.where(same, i ^ (i + d), 2**30 + (i ^ (i + d) if pair_ties else i + d))
             better = (a < best[i]) | ((a == best[i]) & (x < tie[i]))
             j = i[better]

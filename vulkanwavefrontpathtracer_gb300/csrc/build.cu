@@ -413,15 +413,21 @@ __device__ __forceinline__ void write_node2(uint32_t index, uint32_t n, const ui
     __stcg(&meta[index], make_uint4(how[0], how[1], tris, arg[8]));
 }
 
+__device__ __forceinline__ bool same_box(const float4* s_lo, const float4* s_hi, int a, int b) {
+    const float4 alo = s_lo[a], ahi = s_hi[a], blo = s_lo[b], bhi = s_hi[b];
+    return alo.x == blo.x && alo.y == blo.y && alo.z == blo.z && ahi.x == bhi.x && ahi.y == bhi.y && ahi.z == bhi.z;
+}
+
 // The position of the R on either side of position i (box `at` in shared
-// memory) whose box merged with i's has the least surface area.  Ties go to
-// equal boxes first, and among these to the position with the least i xor j:
-// so a run of coincident triangles pairs up as (2 k, 2 k + 1).  Other ties go to
-// the smaller position, or (PAIR_TIES) also to the least i xor j.
+// memory) whose box merged with i's has the least surface area.  Ties go to the
+// positions of i's own run of equal boxes first, and among these to the one with
+// the least i xor j: so coincident triangles, which follow one another in Morton
+// order, pair up as (2 k, 2 k + 1).  Other ties go to the smaller position, or
+// (PAIR_TIES) also to the least i xor j.
 template <bool PAIR_TIES>
 __device__ __forceinline__ uint32_t nearest(const float4* s_lo, const float4* s_hi, int at, int R, int i, uint32_t m) {
     const float4 alo = s_lo[at], ahi = s_hi[at];
-    uint32_t best = kNone, nn = kNone, last = kNone;  // last: the last position with the best area
+    uint32_t best = kNone, nn = kNone;
     const int d0 = max(-R, -i), d1 = min(R, (int)m - 1 - i);
     for (int d = d0; d <= d1; ++d) {
         if (d == 0) continue;
@@ -429,25 +435,22 @@ __device__ __forceinline__ uint32_t nearest(const float4* s_lo, const float4* s_
         const float4 ulo = make_float4(fminf(alo.x, blo.x), fminf(alo.y, blo.y), fminf(alo.z, blo.z), 0.0f);
         const float4 uhi = make_float4(fmaxf(ahi.x, bhi.x), fmaxf(ahi.y, bhi.y), fmaxf(ahi.z, bhi.z), 0.0f);
         const uint32_t key = __float_as_uint(box_area(ulo, uhi)), j = (uint32_t)(i + d);
-        if (key <= best) last = j;
         if (key < best || (PAIR_TIES && key == best && ((uint32_t)i ^ j) < ((uint32_t)i ^ nn))) {
             best = key;
             nn = j;
         }
     }
-    // Several with the least area, and that no larger than this box: equal boxes?
-    // (One position may be the last and, by xor, the best of several.)
-    if ((PAIR_TIES || last != nn) && best == __float_as_uint(box_area(alo, ahi))) {
+    // Only where the merged box is no larger than this one may it be an equal one's.
+    if (best == __float_as_uint(box_area(alo, ahi))) {
         uint32_t tie = kNone;
-        for (int d = d0; d <= d1; ++d) {
-            const float4 blo = s_lo[at + d], bhi = s_hi[at + d];
-            const uint32_t x = (uint32_t)i ^ (uint32_t)(i + d);
-            if (d != 0 && x < tie && alo.x == blo.x && alo.y == blo.y && alo.z == blo.z && ahi.x == bhi.x &&
-                ahi.y == bhi.y && ahi.z == bhi.z) {
-                tie = x;
-                nn = (uint32_t)(i + d);
+        for (int side = -1; side <= 1; side += 2)
+            for (int d = side; d0 <= d && d <= d1 && same_box(s_lo, s_hi, at, at + d); d += side) {
+                const uint32_t j = (uint32_t)(i + d), x = (uint32_t)i ^ j;
+                if (x < tie) {
+                    tie = x;
+                    nn = j;
+                }
             }
-        }
     }
     return nn;
 }
@@ -459,16 +462,15 @@ struct PlocStart {
 
 // The whole clustering.  A block takes tiles of kBB - 2 R cluster positions
 // and holds the boxes of the tile and of 2 R positions on either side in
-// shared memory: enough to find the nearest neighbour (least merged surface
-// area, ties to the smaller position) of every position of the tile and of
-// the R on either side, hence the mutual pairs that start or end in the
-// tile.  For a fixed cluster that order is an order of pairs (area; equal boxes
-// first; i xor j or the positions), so the pair that is least in it over all
-// pairs is mutual and every pass merges at least one pair.
+// shared memory: enough to find the nearest neighbour (see nearest) of every
+// position of the tile and of the R on either side, hence the mutual pairs that
+// start or end in the tile.  For a fixed cluster that order is an order of pairs
+// (area; runs of equal boxes first; i xor j or the positions), so the pair that
+// is least in it over all pairs is mutual and every pass merges at least one.
 // No more than one, where all ties go to the smaller position: 600 coincident
 // triangles took 599 passes and gave a chain too deep for the emission and for
 // the traversal's stacks, and 80 of them in the courtyard's mesh a tree of depth
-// 100.  Equal boxes first: 10 passes, and depth 29.  A strip of 40,000 equal
+// 100.  Runs of equal boxes first: 10 passes, and depth 29.  A strip of 40,000 equal
 // triangles still took over 20,000 passes; so after a pass that merged less
 // than one in kSlowPass of its clusters the other ties go by i xor j too: 22
 // passes.  Triangle soups, the courtyard and the city merge 9 % and more at
