@@ -464,7 +464,11 @@ wfpt_status wfpt_scene_export_bvh8(const wfpt_scene* scene, void* nodes,
  * stack traversal instead of rayQuery.  closest_hit = 0 terminates on the
  * first hit (gl_RayFlagsTerminateOnFirstHitEXT).  ray_index (nullable) is
  * the indirect index: thread i traces ray ray_index[i] and writes
- * results[ray_index[i]].  A ray with tmax < tmin misses. */
+ * results[ray_index[i]].  A ray with tmax < tmin misses.  BVH8 calls hand
+ * their rays out by one of 64 counters of the scene, taken in turn, so that
+ * up to 64 calls may overlap.  A captured call keeps its counter: replays of
+ * it must not run beside one another (copies of one graph), nor beside calls
+ * on the scene made 64 or more BVH8 calls after the capture. */
 wfpt_status wfpt_trace(const wfpt_scene* scene, int bvh_kind, const wfpt_ray* rays,
                        wfpt_hit* results, const uint32_t* ray_index, uint32_t n,
                        const uint32_t* n_dev, int closest_hit, void* stream);

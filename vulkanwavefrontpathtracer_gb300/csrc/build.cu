@@ -10,7 +10,7 @@
 //      cluster picks the neighbour among the 8 (knob) on either side (in
 //      Morton order) whose merged box has the least surface area, mutual pairs
 //      merge, the cluster list is compacted by a prefix sum, until one
-//      cluster is left.  All passes run in one cooperative launch, and the
+//      cluster is left.  The passes run in one cooperative launch, and the
 //      thread that merges a pair also writes the BVH2 node in the traversal
 //      format (children's boxes grown by 2^-22 P as in the host builder;
 //      single-triangle leaves) and the node's tables of the SAH collapse,
@@ -481,9 +481,9 @@ struct PlocStart {
 // the blocks that had a tile; blocks without one are done for good, since
 // the list only shrinks, and once one tile is left its block goes on alone.
 //
-// Bound by latency: 3M triangles take 52 passes, the 40 last of them with
+// Bound by latency: 3M triangles take 53 passes, the 40 last of them with
 // less than one tile per SM, each a chain of a few dependent L2 round trips
-// (28 % issue active, 1.1 TB/s).  0.88 ms, against 0.97 ms for the same passes
+// (28 % issue active, 1.1 TB/s).  0.79 ms, against 0.97 ms for the same passes
 // as separate kernels (neighbours, flags, a three-launch prefix sum, merge)
 // with as much again in launches and a host read-back per pass, plus 0.82 ms
 // for the BVH2 nodes and the collapse tables in kernels of their own.  Four
@@ -631,7 +631,7 @@ __device__ __forceinline__ uint32_t how_of(const uint4& m, int s) {  // byte how
 // The level's children are the next level's tasks; a barrier of all blocks
 // ends a level.  One thread per node, with the children collected twice (once
 // to count) and a prefix sum and a read-back per level, took 1.24 ms for 3M
-// triangles; this takes 0.52 ms.
+// triangles; this takes 0.47 ms.
 constexpr int kEmitTile = kBB / 8;
 // Levels below the root.  Meshes of millions of triangles have about ten;
 // a few hundred triangles nested in one another are a chain, and refused.

@@ -24,7 +24,8 @@ struct DeviceBuild {
 // (same policy knobs as the host collapse) from device-resident geometry:
 // positions_dev float[3*num_vertices], indices_dev uint32[3*num_triangles],
 // geom_first_dev uint32[num_geoms] (ascending, first 0).  Needs at least two
-// triangles.  Synchronises `s` between PLOC iterations and BVH8 levels.
+// triangles.  Synchronises `s` at the end (and after every 256 PLOC passes,
+// where a mesh takes more).
 // Returns cudaErrorInvalidValue when a triangle index is out of range.
 cudaError_t build_scene_device(const float* positions_dev, uint32_t num_vertices, const uint32_t* indices_dev,
                                uint32_t num_triangles, const uint32_t* geom_first_dev, uint32_t num_geoms,

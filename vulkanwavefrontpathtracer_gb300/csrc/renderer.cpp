@@ -9,9 +9,10 @@
 //    so a frame issues no host readback (the reference reads the path count
 //    and the hit count back after every pass, RayGen.cpp:178-183 and
 //    Renderer.cpp:85-88);
-//  - the per-pass hit count (countRayHits) is taken by the reconstructSmooth
-//    kernel that reads the same hit records just before the shadow pass,
-//    instead of a separate kernel on the frame's critical stream;
+//  - the per-pass hit count (countRayHits) is taken by the kernel that shades
+//    the same hit records, instead of a separate kernel on the frame's critical
+//    stream: the path generation where it shades too (its ray count), else
+//    reconstructSmooth (one atomic per block);
 //  - buffers are sized once per resolution (capacity = width*height rays per
 //    wavefront) and the frame can be captured into one CUDA graph;
 //  - ray statistics are read back once, after the frame.

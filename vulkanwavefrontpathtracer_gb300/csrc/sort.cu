@@ -368,7 +368,7 @@ __device__ __forceinline__ void onesweep_tile(const K* __restrict__ keys_in, con
     constexpr uint32_t TILE = THREADS * KPT;
     constexpr int WARPS = THREADS / 32;
     constexpr bool TAGGED = THREADS == kTinyThreads;
-        constexpr int kRadix = 1 << DB;
+    constexpr int kRadix = 1 << DB;
     K* s_keys = reinterpret_cast<K*>(smem);
     uint32_t* s_vals = reinterpret_cast<uint32_t*>(s_keys + TILE);
     uint32_t* s_hist = s_vals + TILE;  // [warp][digit]

@@ -657,7 +657,6 @@ __global__ void k_interpolate_colors_fp64(float4* __restrict__ frame_pixels, flo
     frame_pixels[i] = make_float4(t.x, t.y, t.z, 1.0f);
 }
 
-// Device-side size of one shadow batch: S * clamp(n_in - begin, 0, size).
 __global__ void k_fill_u32(uint32_t* __restrict__ dst, uint32_t v, size_t n) {
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     size_t stride = (size_t)gridDim.x * blockDim.x;
@@ -673,7 +672,8 @@ static inline unsigned grid_for(uint64_t n) { return (unsigned)((n + kBlock - 1)
 // a sixteenth of n = 8.3M rays left, path generation 35 -> 17 us, shadow
 // generation 29 -> 15 us, the reconstructions 23 -> 12 and 21 -> 9 us (host
 // time included, about 9 us a call).  At full counts the two forms are equal
-// (two waves of blocks keep every SM full); with the BVH2 traversal's
+// (two waves of blocks at eight per SM, 2.7 of the path generation with the
+// shading, which has six); with the BVH2 traversal's
 // persistent form a 4K city frame went from 20.4 to 18.5 ms.
 constexpr unsigned kStageGrid = 152 * 16;
 constexpr unsigned kStageCapped = 152 * 64;  // capacities of fewer blocks (2.5M rays) keep a block each
